@@ -26,6 +26,7 @@ enum : int {
     ERR_LOOKBACK_TIMEOUT = 1,  // a decoupled look-back wait gave up
     ERR_BAD_SEGMENT = 2,       // a segment offset table was not monotone
     ERR_LEARNED_OVERFLOW = 3,  // informational: learned sort used its fallback
+    ERR_MISPLACED = 4,         // a kernel computed a place outside its tile or segment and skipped the access
 };
 
 // How long a spin wait on another CTA may last before it records

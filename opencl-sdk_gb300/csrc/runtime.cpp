@@ -254,6 +254,10 @@ void device_context::finish()
                            "calls are invalid",
                            (int)cudaErrorLaunchTimeout);
     if (e == 2) throw std::invalid_argument("gbcompute: segment offsets are not monotone");
+    if (e == 4)
+        throw device_error("gbcompute: a sort kernel computed a place outside its tile; results of the last "
+                           "calls are invalid",
+                           (int)cudaErrorUnknown);
 }
 
 // ---- profiler -------------------------------------------------------------

@@ -13,22 +13,28 @@
 //   * tiny/small (<= WARP_CAP): one warp per segment, stable LSD radix sort in
 //     warp-private shared memory over the digit positions that vary inside the
 //     segment only;
-//   * medium (<= cta_cap): one CTA per segment, the same LSD in CTA shared
-//     memory;
-//   * large: a batched onesweep: the tiles of all large segments form one
-//     sequence, per-segment digit histograms come from one read of the keys,
-//     and the decoupled look-back of each digit pass stops at the first tile
-//     of its segment.
+//   * medium (<= cta_cap): one CTA per segment, the leading digits sorted and
+//     the rest repaired (tile_sort.cuh), in three classes by length;
+//   * large: the tiles of all large segments form one sequence, and
+//     per-segment digit histograms come from one read of the keys. A segment
+//     whose highest varying digit splits it into small enough buckets takes
+//     the MSD route: one pass on that digit, then one-CTA sorts of ranges of
+//     buckets. The others take a batched onesweep over every digit, whose
+//     decoupled look-back stops at the first tile of its segment.
 // The small/medium path and the large path are independent and run on two
 // streams that fork from and join back to the context's stream.
 #include <algorithm>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <string>
+#include <tuple>
 
 #include "device_common.cuh"
 #include "runtime.hpp"
 #include "segmented.hpp"
 #include "sort_internal.hpp"
+#include "tile_sort.cuh"
 
 namespace gbc {
 namespace seg {
@@ -46,12 +52,29 @@ constexpr int SMALL_WARPS = SMALL_THREADS / 32;
 template <typename K> struct Traits;
 template <> struct Traits<uint32_t> {
     static constexpr int PASSES = 4;
-    static constexpr int CTA_CAP = 8192;
 };
 template <> struct Traits<uint64_t> {
     static constexpr int PASSES = 8;
-    static constexpr int CTA_CAP = 6144;
 };
+
+// One-CTA sorts by length: up to 4,096, 8,192 and the type's largest capacity
+// (16,384 u32 keys; 10,240 u32 pairs or u64 keys, whose registers hold no
+// more; 8,192 u64 pairs, which leaves their last class empty).
+constexpr int CTA_CLASSES = 3;
+constexpr uint32_t CLASS0_CAP = 4096, CLASS1_CAP = 8192;
+template <typename K, bool HAS_V> constexpr uint32_t max_cta_cap()
+{
+    return sizeof(K) == 4 ? (HAS_V ? 10240u : 16384u) : (HAS_V ? 8192u : 10240u);
+}
+__device__ __forceinline__ int cta_class(uint32_t len)
+{
+    return len <= CLASS0_CAP ? 0 : len <= CLASS1_CAP ? 1 : 2;
+}
+
+// The MSD route joins neighbouring buckets of a segment whose first keys lie
+// in the same window of this many keys (a bucket of a few dozen keys is not
+// worth a CTA, and a range of neighbouring buckets is as good to sort).
+constexpr uint32_t SUB_WINDOW = 2048;
 
 __device__ __forceinline__ uint64_t pack_status(uint64_t flag, uint64_t seq, uint32_t v)
 {
@@ -60,12 +83,14 @@ __device__ __forceinline__ uint64_t pack_status(uint64_t flag, uint64_t seq, uin
 
 //! Per-call control block (zeroed before each call).
 struct SegControl {
-    uint32_t n_warp, n_cta, n_large;  // list lengths
-    uint32_t large_tiles;             // tiles of all large segments
-    uint32_t warp_next, cta_next;     // work queue heads
+    uint32_t n_warp, n_cta[CTA_CLASSES], n_large;  // list lengths
+    uint32_t large_tiles;                          // tiles of all large segments
+    uint32_t lsd_tiles;                            // tiles of those not on the MSD route
+    uint32_t warp_next, cta_next[CTA_CLASSES];     // work queue heads
     uint32_t tile_ctr[8];
-    uint32_t n_sub_warp, n_sub_cta;      // sub-bucket list lengths (MSD route)
-    uint32_t sub_warp_next, sub_cta_next;
+    uint32_t msd_tile_ctr;
+    uint32_t n_sub_warp, n_sub_cta[CTA_CLASSES];  // sub-bucket list lengths (MSD route)
+    uint32_t sub_warp_next, sub_cta_next[CTA_CLASSES];
     uint32_t barrier;                    // arrivals at the persistent batch's first grid barrier
     uint32_t large_barrier;              // ... and at those among its large-segment CTAs
 };
@@ -84,10 +109,12 @@ template <typename K> struct SegArgs {
     dev::KeyXform<K> xf;
     SegControl* ctl;
     uint32_t* warp_list;
-    uint32_t* cta_list;
+    uint32_t* cta_list;     // nseg entries per class
     uint32_t* large_list;
-    uint32_t* tile_begin;   // per large segment (n_large + 1)
+    uint32_t* tile_begin;   // per large segment: its first tile
     uint32_t* tile_seg;     // large tile -> index into large_list
+    uint32_t* lsd_begin;    // the same for the segments that take the LSD passes
+    uint32_t* lsd_seg;      // (tile_begin and tile_seg themselves without the MSD route)
     uint32_t* seg_hist;     // [large][PASSES][256]: bin start (absolute) per pass
     uint32_t max_large;
     uint32_t max_tiles;
@@ -99,95 +126,85 @@ template <typename K> struct SegArgs {
     // sub-buckets (begin, end pairs) are finished from alt into out by the
     // warp (<= WARP_CAP) and CTA (<= sub_cap) sorts.
     uint8_t* route;
-    uint32_t* sub_warp_list;
-    uint32_t* sub_cta_list;
+    uint32_t* sub_lists;  // 2 x max_sub (begin, end) pairs, see sub_entry
     uint32_t max_sub;
     uint32_t sub_cap;
 };
+
+// The (begin, end) pair at position i of a sub-bucket list: the warp class
+// (cls = -1) and class 0 share one array, classes 1 and 2 another, each pair
+// growing from both ends (there are at most max_sub sub-buckets in all).
+template <typename K> __device__ __forceinline__ uint2* sub_entry(const SegArgs<K>& a, int cls, uint32_t i)
+{
+    uint2* base = reinterpret_cast<uint2*>(a.sub_lists) + (cls >= 1 ? a.max_sub : 0u);
+    return cls == -1 || cls == 1 ? base + i : base + (a.max_sub - 1 - i);
+}
 
 constexpr uint8_t NO_ROUTE = 0xFF;
 
 // ---------------------------------------------------------------------------
 // Classification
 // ---------------------------------------------------------------------------
-template <typename K> __device__ __forceinline__ void seg_classify(const SegArgs<K>& a)
+template <typename K, int TILE> __device__ __forceinline__ void seg_classify(const SegArgs<K>& a)
 {
+    // whole warps take every step, so that a class's members in a warp share
+    // one addition to its counter
     const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.nseg; i += stride) {
-        const uint32_t b = a.off[i], e = a.off[i + 1];
-        if (e < b) {
-            dev::raise_error(a.err, dev::ERR_BAD_SEGMENT);
-            continue;
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < a.nseg; i0 += stride) {
+        const uint32_t i = i0 + lane;
+        uint32_t len = 0;
+        if (i < a.nseg) {
+            const uint32_t b = a.off[i], e = a.off[i + 1];
+            if (e < b) dev::raise_error(a.err, dev::ERR_BAD_SEGMENT);
+            else if (a.skip == nullptr || a.skip[i] == 0) len = e - b;
         }
-        const uint32_t len = e - b;
-        if (len == 0 || (a.skip != nullptr && a.skip[i] != 0)) continue;
-        if (len <= WARP_CAP) {
-            a.warp_list[atomicAdd(&a.ctl->n_warp, 1u)] = i;
-        } else if (len <= a.cta_cap) {
-            a.cta_list[atomicAdd(&a.ctl->n_cta, 1u)] = i;
-        } else {
+        // -1: nothing to do; 0: a warp's; 1 ..: the one-CTA classes
+        const int cls = len == 0 ? -1 : len <= WARP_CAP ? 0 : len <= a.cta_cap ? 1 + cta_class(len) : 1 + CTA_CLASSES;
+#pragma unroll
+        for (int c = 0; c <= CTA_CLASSES; ++c) {
+            const uint32_t members = __ballot_sync(FULL_MASK, cls == c);
+            if (members == 0) continue;
+            uint32_t at = 0;
+            if (lane == 0) at = atomicAdd(c == 0 ? &a.ctl->n_warp : &a.ctl->n_cta[c - 1], (uint32_t)__popc(members));
+            at = __shfl_sync(FULL_MASK, at, 0) + __popc(members & dev::lanemask_lt());
+            if (cls == c) (c == 0 ? a.warp_list : a.cta_list + (std::size_t)(c - 1) * a.nseg)[at] = i;
+        }
+        if (cls == 1 + CTA_CLASSES) {
             const uint32_t j = atomicAdd(&a.ctl->n_large, 1u);
-            if (j < a.max_large) a.large_list[j] = i;
-            else dev::raise_error(a.err, dev::ERR_BAD_SEGMENT);
+            if (j < a.max_large) {
+                a.large_list[j] = i;
+                // the segment's stretch of the tile sequence; the sequence's
+                // order among segments does not matter
+                a.tile_begin[j] = atomicAdd(&a.ctl->large_tiles, (len + TILE - 1) / TILE);
+            } else {
+                dev::raise_error(a.err, dev::ERR_BAD_SEGMENT);
+            }
         }
     }
 }
 
-template <typename K> __global__ void k_seg_classify(SegArgs<K> a) { seg_classify(a); }
+template <typename K, int TILE> __global__ void k_seg_classify(SegArgs<K> a) { seg_classify<K, TILE>(a); }
 
-// One CTA of NT threads: exclusive scan of the large segments' tile counts.
-template <typename K, int TILE, int NT> __device__ __forceinline__ void seg_plan_scan(const SegArgs<K>& a)
+// The tile -> segment map (a warp of the first `ctas` CTAs per large segment),
+// and zeros in the histogram rows of the large segments present.
+template <typename K, int TILE> __device__ __forceinline__ void seg_large_plan(const SegArgs<K>& a, uint32_t ctas)
 {
-    __shared__ uint32_t s_warp[NT / 32];
-    __shared__ uint32_t s_carry;
+    constexpr int P = Traits<K>::PASSES;
     const uint32_t nl = min(a.ctl->n_large, a.max_large);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) s_carry = 0;
-    __syncthreads();
-    for (uint32_t base = 0; base < nl; base += NT) {
-        const uint32_t j = base + threadIdx.x;
-        uint32_t cnt = 0;
-        if (j < nl) {
-            const uint32_t s = a.large_list[j];
-            cnt = (a.off[s + 1] - a.off[s] + TILE - 1) / TILE;
-        }
-        uint32_t x = dev::warp_inclusive_scan(cnt, [](uint32_t p, uint32_t q) { return p + q; });
-        if (lane == 31) s_warp[warp] = x;
-        __syncthreads();
-        uint32_t before = s_carry;
-        for (int w = 0; w < warp; ++w) before += s_warp[w];
-        if (j < nl) a.tile_begin[j] = before + x - cnt;
-        __syncthreads();
-        if (threadIdx.x == NT - 1) s_carry = before + x;
-        __syncthreads();
-    }
-    const uint32_t total = min(s_carry, a.max_tiles);
-    if (threadIdx.x == 0) {
-        a.tile_begin[nl] = total;
-        a.ctl->large_tiles = total;
-    }
-    __syncthreads();
-}
-
-// The tile -> segment map: the warps of the first `ctas` CTAs fill the tiles
-// of one large segment at a time.
-template <typename K> __device__ __forceinline__ void seg_plan_map(const SegArgs<K>& a, uint32_t ctas)
-{
-    const uint32_t nl = min(a.ctl->n_large, a.max_large);
-    const uint32_t total = a.ctl->large_tiles;
     const int lane = threadIdx.x & 31;
     const uint32_t warps = ctas * (blockDim.x / 32);
     for (uint32_t j = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); j < nl; j += warps) {
-        const uint32_t t0 = a.tile_begin[j], t1 = min(a.tile_begin[j + 1], total);
+        const uint32_t s = a.large_list[j];
+        const uint32_t t0 = a.tile_begin[j], t1 = min(t0 + (a.off[s + 1] - a.off[s] + TILE - 1) / TILE, a.max_tiles);
         for (uint32_t t = t0 + lane; t < t1; t += 32) a.tile_seg[t] = j;
     }
+    const std::size_t words = (std::size_t)nl * P * RADIX;
+    const std::size_t stride = (std::size_t)ctas * blockDim.x;
+    for (std::size_t i = (std::size_t)blockIdx.x * blockDim.x + threadIdx.x; i < words; i += stride) a.seg_hist[i] = 0;
 }
 
-template <typename K, int TILE> __global__ void __launch_bounds__(1024) k_seg_plan(SegArgs<K> a)
-{
-    seg_plan_scan<K, TILE, 1024>(a);
-    seg_plan_map(a, gridDim.x);
-}
+template <typename K, int TILE> __global__ void k_seg_large_plan(SegArgs<K> a) { seg_large_plan<K, TILE>(a, gridDim.x); }
 
 // ---------------------------------------------------------------------------
 // Shared-memory LSD sort of one segment by a group of GW warps (GW = 1: a
@@ -336,8 +353,9 @@ template <typename K, bool HAS_V, bool SUB> __device__ __forceinline__ void seg_
         if (w >= total) break;
         uint32_t b, len;
         if (SUB) {
-            b = a.sub_warp_list[2 * w];
-            len = a.sub_warp_list[2 * w + 1] - b;
+            const uint2 r = *sub_entry(a, -1, w);
+            b = r.x;
+            len = r.y - r.x;
         } else {
             const uint32_t s = a.warp_list[w];
             b = a.off[s];
@@ -366,11 +384,12 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_seg_small_warp(SegArgs<K> a)
     seg_small_warp<K, HAS_V, SUB>(a);
 }
 
-// THREADS: 256, or 512 where the shared memory allows (twice the warps in
-// flight on the SM for the same shared-memory tile).
-template <typename K, bool HAS_V, bool SUB, int THREADS = SMALL_THREADS>
-__device__ __forceinline__ void seg_small_cta(const SegArgs<K>& a)
+// The one-CTA sorts inside the persistent batch kernel: every class of up to
+// cta_cap (SUB: sub_cap) keys with the same shared-memory sort, which holds
+// any length in the shared memory that the kernel was launched with.
+template <typename K, bool HAS_V, bool SUB> __device__ __forceinline__ void seg_small_cta(const SegArgs<K>& a)
 {
+    constexpr int THREADS = SMALL_THREADS;
     constexpr int WARPS = THREADS / 32;
     static_assert(THREADS % 32 == 0 && THREADS >= RADIX && WARPS <= 32, "one thread per bin; scratch holds 32 warps");
     extern __shared__ __align__(16) unsigned char smem[];
@@ -386,20 +405,25 @@ __device__ __forceinline__ void seg_small_cta(const SegArgs<K>& a)
     __shared__ uint32_t scratch[64 + 8];
     __shared__ uint32_t s_work;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t total = SUB ? min(a.ctl->n_sub_cta, a.max_sub) : a.ctl->n_cta;
     const K* src_k = SUB ? a.alt_k : a.in_k;
     const uint32_t* src_v = SUB ? a.alt_v : a.in_v;
+    int cls = 0;
     for (;;) {
-        if (threadIdx.x == 0) s_work = atomicAdd(SUB ? &a.ctl->sub_cta_next : &a.ctl->cta_next, 1u);
+        if (threadIdx.x == 0) s_work = atomicAdd(SUB ? &a.ctl->sub_cta_next[cls] : &a.ctl->cta_next[cls], 1u);
         __syncthreads();
         const uint32_t w = s_work;
-        if (w >= total) break;
+        if (w >= (SUB ? min(a.ctl->n_sub_cta[cls], a.max_sub) : a.ctl->n_cta[cls])) {
+            if (++cls == CTA_CLASSES) break;
+            __syncthreads();  // every thread has read s_work
+            continue;
+        }
         uint32_t b, len;
         if (SUB) {
-            b = a.sub_cta_list[2 * w];
-            len = a.sub_cta_list[2 * w + 1] - b;
+            const uint2 r = *sub_entry(a, cls, w);
+            b = r.x;
+            len = r.y - r.x;
         } else {
-            const uint32_t s = a.cta_list[w];
+            const uint32_t s = a.cta_list[(std::size_t)cls * a.nseg + w];
             b = a.off[s];
             len = a.off[s + 1] - b;
         }
@@ -420,40 +444,85 @@ __device__ __forceinline__ void seg_small_cta(const SegArgs<K>& a)
     }
 }
 
-template <typename K, bool HAS_V, bool SUB, int THREADS>
-__global__ void __launch_bounds__(THREADS) k_seg_small_cta(SegArgs<K> a)
-{
-    seg_small_cta<K, HAS_V, SUB, THREADS>(a);
-}
-
-//! Shared memory of the one-CTA sort: two copies of keys (and values) and a
-//! packed rank per element, then a histogram and a peer-mask array per warp.
+//! Shared memory of that sort: two copies of keys (and values) and a packed
+//! rank per element, then a histogram and a peer-mask array per warp.
 template <typename K, bool HAS_V> constexpr std::size_t cta_sort_smem(uint32_t cap, int threads)
 {
     return (std::size_t)cap * (2 * sizeof(K) + (HAS_V ? 8 : 0) + 4) + 2 * (std::size_t)(threads / 32) * RADIX * 4;
 }
 
+// The one-CTA sorts of classes cls to last (tile_sort.cuh): persistent CTAs
+// take their segments (sub: the MSD route's sub-buckets) one at a time. Bound by
+// shared-memory accesses (about 27 wavefronts per 32 pairs and digit pass), so
+// what counts is the number of passes and the warps in flight: the sort of
+// every digit in two shared-memory copies, one CTA of 256 threads per SM at
+// the largest capacity, took 10.3 ms for 200,000 lognormal segments of u64
+// pairs (median 256), this one 4.1 ms, each beside its large-segment path.
+template <typename K, bool HAS_V, int THREADS, int ITEMS, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB) k_seg_tile(SegArgs<K> a, int cls, int last, bool sub)
+{
+    using S = tile::Sorter<K, HAS_V, THREADS, ITEMS>;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ tile::Scratch<THREADS> scratch;
+    __shared__ uint32_t s_work;
+    S st(smem, scratch);
+    const K* src_k = sub ? a.alt_k : a.in_k;
+    const uint32_t* src_v = sub ? a.alt_v : a.in_v;
+    for (;;) {
+        if (threadIdx.x == 0) s_work = atomicAdd(sub ? &a.ctl->sub_cta_next[cls] : &a.ctl->cta_next[cls], 1u);
+        __syncthreads();
+        const uint32_t w = s_work;
+        if (w >= (sub ? min(a.ctl->n_sub_cta[cls], a.max_sub) : a.ctl->n_cta[cls])) {
+            if (++cls > last) break;
+            __syncthreads();  // every thread has read s_work
+            continue;
+        }
+        uint32_t b, len;
+        if (sub) {
+            const uint2 r = *sub_entry(a, cls, w);
+            b = r.x;
+            len = r.y - r.x;
+        } else {
+            const uint32_t s = a.cta_list[(std::size_t)cls * a.nseg + w];
+            b = a.off[s];
+            len = a.off[s + 1] - b;
+        }
+        if (len > (uint32_t)S::CAP) {  // the classes end at the capacities
+            if (threadIdx.x == 0) dev::raise_error(a.err, dev::ERR_MISPLACED);
+            __syncthreads();
+            continue;
+        }
+        st.len = len;
+        st.rows = (len + THREADS - 1) / THREADS;
+        const uint32_t i0 = st.first_index();
+        K key[ITEMS];
+        uint32_t val[HAS_V ? ITEMS : 1];
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            const uint32_t idx = i0 + i * 16;
+            const bool in = i < (int)st.rows && idx < len;
+            key[i] = in ? src_k[b + idx] : K(0);
+            if (HAS_V) val[i] = in ? src_v[b + idx] : 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) key[i] = a.xf(key[i]);
+        if (!st.sort(key, val) && threadIdx.x == 0) dev::raise_error(a.err, dev::ERR_MISPLACED);
+        for (uint32_t i = threadIdx.x; i < len; i += THREADS) {
+            a.out_k[b + i] = tile::undo_xform(a.xf, st.keys[i]);
+            if (HAS_V) a.out_v[b + i] = st.vals[i];
+        }
+        __syncthreads();
+    }
+}
+
 // ---------------------------------------------------------------------------
-// Large segments: per-segment digit histograms -> absolute bin starts, in
-// three steps over the large-segment tile sequence that the passes use (so
-// a long segment is spread over many CTAs): zero the rows of the large
-// segments present; count runs of HIST_TILES tiles in shared memory and add
-// the counts to the segment's row whenever the segment changes or the run
+// Large segments: per-segment digit histograms -> absolute bin starts, over
+// the large-segment tile sequence that the passes use (so a long segment is
+// spread over many CTAs): count runs of HIST_TILES tiles in shared memory and
+// add the counts to the segment's row whenever the segment changes or the run
 // ends; turn every row into absolute bin starts.
 // ---------------------------------------------------------------------------
 constexpr uint32_t HIST_TILES = 8;
-
-template <typename K> __device__ __forceinline__ void seg_large_zero(const SegArgs<K>& a, uint32_t ctas)
-{
-    constexpr int P = Traits<K>::PASSES;
-    const uint32_t nl = min(a.ctl->n_large, a.max_large);
-    const std::size_t words = (std::size_t)nl * P * RADIX;
-    const std::size_t stride = (std::size_t)ctas * blockDim.x;
-    for (std::size_t i = (std::size_t)blockIdx.x * blockDim.x + threadIdx.x; i < words; i += stride) a.seg_hist[i] = 0;
-}
-
-template <typename K> __global__ void k_seg_large_zero(SegArgs<K> a) { seg_large_zero(a, gridDim.x); }
-
 
 template <typename K, int TILE> __device__ __forceinline__ void seg_large_count(const SegArgs<K>& a, uint32_t ctas)
 {
@@ -461,7 +530,7 @@ template <typename K, int TILE> __device__ __forceinline__ void seg_large_count(
     constexpr int BATCH = 8;  // keys in flight per thread
     __shared__ uint32_t sh[2][P * RADIX];  // two copies (warp parity)
     uint32_t* my = sh[(threadIdx.x >> 5) & 1];
-    const uint32_t total = a.ctl->large_tiles;
+    const uint32_t total = min(a.ctl->large_tiles, a.max_tiles);
     const uint32_t runs = (total + HIST_TILES - 1) / HIST_TILES;
     auto flush = [&](uint32_t j) {  // adds the counts to row j and clears them
         __syncthreads();
@@ -514,43 +583,32 @@ template <typename K, int TILE> __global__ void __launch_bounds__(256) k_seg_lar
 }
 
 
-template <typename K> __device__ __forceinline__ void seg_large_starts(const SegArgs<K>& a, uint32_t ctas)
-{
-    constexpr int P = Traits<K>::PASSES;
-    __shared__ uint32_t s_scratch[8];
-    const uint32_t nl = min(a.ctl->n_large, a.max_large);
-    for (uint32_t j = blockIdx.x; j < nl; j += ctas) {
-        const uint32_t b = a.off[a.large_list[j]];
-        for (int p = 0; p < P; ++p) {
-            uint32_t* row = a.seg_hist + ((std::size_t)j * P + p) * RADIX;
-            const uint32_t ex = dev::bins_exclusive_sum(row[threadIdx.x], s_scratch);
-            row[threadIdx.x] = b + ex;
-        }
-    }
-}
-
-template <typename K> __global__ void __launch_bounds__(256) k_seg_large_starts(SegArgs<K> a)
-{
-    seg_large_starts(a, gridDim.x);
-}
-
-
-// Per large segment (one CTA, thread d = bin d): the highest digit position
-// that varies inside the segment (its bins are not all in one) and, when
-// every bin there holds at most sub_cap keys, the MSD route: one pass on that
-// digit partitions the segment into its bins (stable), which become
-// sub-buckets for the warp and CTA sorts; else the full LSD passes. The bin
-// starts in seg_hist are absolute, from k_seg_large_starts.
-template <typename K> __device__ __forceinline__ void seg_route(const SegArgs<K>& a, uint32_t ctas)
+// Per large segment (one CTA, thread d = bin d): every digit's counts become
+// absolute bin starts. With the MSD route: then the highest digit position
+// that varies inside the segment (its bins are not all in one) and, when every
+// bin there leaves room for a window in sub_cap, the MSD route: one
+// pass on that digit partitions the segment into its bins (stable), and
+// ranges of neighbouring bins become sub-buckets for the warp and CTA sorts;
+// else the full LSD passes, over tiles appended to their own sequence.
+template <typename K, int TILE> __device__ __forceinline__ void seg_route(const SegArgs<K>& a, bool with_msd, uint32_t ctas)
 {
     constexpr int P = Traits<K>::PASSES;
     __shared__ uint32_t s_max[8];
+    __shared__ uint32_t s_scratch[8];
     __shared__ int s_top;
+    __shared__ uint32_t s_first;
     const uint32_t nl = min(a.ctl->n_large, a.max_large);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (uint32_t j = blockIdx.x; j < nl; j += ctas) {
         const uint32_t s = a.large_list[j];
         const uint32_t segb = a.off[s], sege = a.off[s + 1], len = sege - segb;
+        for (int p = 0; p < P; ++p) {
+            uint32_t* row = a.seg_hist + ((std::size_t)j * P + p) * RADIX;
+            const uint32_t ex = dev::bins_exclusive_sum(row[threadIdx.x], s_scratch);
+            row[threadIdx.x] = segb + ex;
+        }
+        if (!with_msd) continue;
+        __syncthreads();
         auto bin_size = [&](int p, uint32_t d) {
             const uint32_t* row = a.seg_hist + ((size_t)j * P + p) * RADIX;
             return (d == RADIX - 1 ? sege : row[d + 1]) - row[d];
@@ -576,23 +634,39 @@ template <typename K> __device__ __forceinline__ void seg_route(const SegArgs<K>
         uint32_t biggest = 0;
 #pragma unroll
         for (int w = 0; w < 8; ++w) biggest = max(biggest, s_max[w]);
-        const bool msd = top >= 0 && biggest <= a.sub_cap;
+        // room for a window's keys and its last bucket
+        const bool msd = top >= 0 && biggest + SUB_WINDOW <= a.sub_cap;
         if (threadIdx.x == 0) a.route[j] = msd ? (uint8_t)top : NO_ROUTE;
-        if (msd && size != 0) {  // a one-key bucket goes to the warp sort, which copies it
-            const uint32_t b = a.seg_hist[((size_t)j * P + top) * RADIX + threadIdx.x];
-            if (size <= (uint32_t)WARP_CAP) {
-                const uint32_t q = atomicAdd(&a.ctl->n_sub_warp, 1u);
-                if (q < a.max_sub) a.sub_warp_list[2 * q] = b, a.sub_warp_list[2 * q + 1] = b + size;
-            } else {
-                const uint32_t q = atomicAdd(&a.ctl->n_sub_cta, 1u);
-                if (q < a.max_sub) a.sub_cta_list[2 * q] = b, a.sub_cta_list[2 * q + 1] = b + size;
+        if (msd) {
+            const uint32_t* row = a.seg_hist + ((size_t)j * P + top) * RADIX;
+            const uint32_t d = threadIdx.x;
+            auto window = [&](uint32_t q) { return (row[q] - segb) / SUB_WINDOW; };
+            if (d == 0 || window(d) != window(d - 1)) {  // first bucket of its window: the range up to the next one's
+                uint32_t q = d + 1;
+                while (q < RADIX && window(q) == window(d)) ++q;
+                const uint32_t b = row[d], e = q < RADIX ? row[q] : sege;
+                if (e > b) {  // a range of one key goes to the warp sort, which copies it
+                    const int cls = e - b <= (uint32_t)WARP_CAP ? -1 : cta_class(e - b);
+                    const uint32_t at = atomicAdd(cls < 0 ? &a.ctl->n_sub_warp : &a.ctl->n_sub_cta[cls], 1u);
+                    if (at < a.max_sub) *sub_entry(a, cls, at) = make_uint2(b, e);
+                    else dev::raise_error(a.err, dev::ERR_BAD_SEGMENT);
+                }
             }
+        } else {
+            const uint32_t tiles = (len + TILE - 1) / TILE;
+            if (threadIdx.x == 0) a.lsd_begin[j] = s_first = atomicAdd(&a.ctl->lsd_tiles, tiles);
+            __syncthreads();
+            for (uint32_t t = threadIdx.x; t < tiles; t += blockDim.x)
+                if (s_first + t < a.max_tiles) a.lsd_seg[s_first + t] = j;
         }
         __syncthreads();
     }
 }
 
-template <typename K> __global__ void __launch_bounds__(256) k_seg_route(SegArgs<K> a) { seg_route(a, gridDim.x); }
+template <typename K, int TILE> __global__ void __launch_bounds__(256) k_seg_route(SegArgs<K> a, bool with_msd)
+{
+    seg_route<K, TILE>(a, with_msd, gridDim.x);
+}
 
 
 // One digit pass over every large segment's tiles (cf. onesweep::k_pass2:
@@ -602,21 +676,31 @@ template <typename K> __global__ void __launch_bounds__(256) k_seg_route(SegArgs
 // of the tile a grid ahead and an unrolled write-out of full tiles).
 constexpr int LARGE_PAD = 1;  // words between the half-warp count arrays of the large pass
 
-template <typename K, bool HAS_V, int THREADS, int ITEMS, int LBW>
-__device__ __forceinline__ void seg_large_pass(const SegArgs<K>& a, int slot, uint32_t ctas)
+//
+// MSD: the one pass of the segments on the MSD route, each on its own digit
+// position, over the sequence of all large segments' tiles; else LSD pass
+// `slot` over the tiles of the segments that take those. Returns at once when
+// its kind has no segment.
+template <typename K, bool HAS_V, int THREADS, int ITEMS, int LBW, bool MSD>
+__device__ __forceinline__ void seg_large_pass(const SegArgs<K>& a, int slot, bool with_msd, uint32_t ctas)
 {
     constexpr int P = Traits<K>::PASSES;
     constexpr int WARPS = THREADS / 32;
     constexpr int TILE = THREADS * ITEMS;
-    const uint32_t num_tiles = a.ctl->large_tiles;
-    const int shift = 8 * slot;
+    const uint32_t num_tiles = min(MSD || !with_msd ? a.ctl->large_tiles : a.ctl->lsd_tiles, a.max_tiles);
+    if (num_tiles == 0) return;
+    const uint32_t* tile_seg = MSD ? a.tile_seg : a.lsd_seg;
+    const uint32_t* tile_begin = MSD ? a.tile_begin : a.lsd_begin;
+    uint32_t* tile_ctr = MSD ? &a.ctl->msd_tile_ctr : &a.ctl->tile_ctr[slot];
     // pass s writes out when (P - 1 - s) is even; P is even, so pass 0 reads
     // the input and writes the scratch buffer.
-    const bool dst_out = ((P - 1 - slot) & 1) == 0;
+    // The MSD pass reads the input and writes the scratch buffer, from which
+    // its sub-buckets are finished.
+    const bool dst_out = !MSD && ((P - 1 - slot) & 1) == 0;
     K* dst_k = dst_out ? a.out_k : a.alt_k;
     uint32_t* dst_v = dst_out ? a.out_v : a.alt_v;
-    const K* src_k = slot == 0 ? a.in_k : (dst_out ? a.alt_k : a.out_k);
-    const uint32_t* src_v = slot == 0 ? a.in_v : (dst_out ? a.alt_v : a.out_v);
+    const K* src_k = MSD || slot == 0 ? a.in_k : (dst_out ? a.alt_k : a.out_k);
+    const uint32_t* src_v = MSD || slot == 0 ? a.in_v : (dst_out ? a.alt_v : a.out_v);
     const bool aligned_src =
         ((reinterpret_cast<uintptr_t>(src_k) | (HAS_V ? reinterpret_cast<uintptr_t>(src_v) : 0)) & 15) == 0;
 
@@ -638,25 +722,24 @@ __device__ __forceinline__ void seg_large_pass(const SegArgs<K>& a, int slot, ui
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int grp = 2 * warp + (lane >> 4), gl = lane & 15;
     if (tid == 0) s_abort = 0;
-    const uint64_t seq0 = a.seq0 + (uint64_t)slot * a.max_tiles;
+    // MSD: after the P LSD passes' sequence numbers
+    const uint64_t seq0 = a.seq0 + (uint64_t)(MSD ? P : slot) * a.max_tiles;
+    int shift = 8 * slot;
     auto digit = [&](K k) -> uint32_t { return (uint32_t)(a.xf(k) >> shift) & 0xFFu; };
 
     for (;;) {
         if (tid == 0) {
-            s_tile = atomicAdd(&a.ctl->tile_ctr[slot], 1u);
+            s_tile = atomicAdd(tile_ctr, 1u);
             // L2 prefetch of the tile a grid further on in the tile sequence
-            // (from where this pass reads it, if it takes part)
+            // (if it takes part)
             const uint32_t ahead = s_tile + ctas;
             if (aligned_src && ahead < num_tiles) {
-                const uint32_t ja = a.tile_seg[ahead];
-                const uint8_t ra = a.route[ja];
+                const uint32_t ja = tile_seg[ahead];
                 const uint32_t sa = a.large_list[ja];
-                const uint32_t ba = a.off[sa] + (ahead - a.tile_begin[ja]) * TILE;
-                const K* pk = ra == NO_ROUTE ? src_k : a.in_k;
-                const uint32_t* pv = ra == NO_ROUTE ? src_v : a.in_v;
-                if ((ra == NO_ROUTE || ra == slot) && ba + TILE <= a.off[sa + 1] && (ba % (16 / sizeof(K))) == 0) {
-                    dev::prefetch_l2(pk + ba, TILE * sizeof(K));
-                    if (HAS_V && (ba & 3) == 0) dev::prefetch_l2(pv + ba, TILE * 4);
+                const uint32_t ba = a.off[sa] + (ahead - tile_begin[ja]) * TILE;
+                if ((!MSD || a.route[ja] != NO_ROUTE) && ba + TILE <= a.off[sa + 1] && (ba % (16 / sizeof(K))) == 0) {
+                    dev::prefetch_l2(src_k + ba, TILE * sizeof(K));
+                    if (HAS_V && (ba & 3) == 0) dev::prefetch_l2(src_v + ba, TILE * 4);
                 }
             }
         }
@@ -664,23 +747,26 @@ __device__ __forceinline__ void seg_large_pass(const SegArgs<K>& a, int slot, ui
         __syncthreads();
         const uint32_t t = s_tile;
         if (t >= num_tiles) break;
-        const uint32_t j = a.tile_seg[t];
-        // a segment on the MSD route takes part in its one pass only, reading
-        // the input and writing the scratch buffer (its sub-buckets are then
-        // finished from there); its tiles publish nothing in the other passes,
-        // and no tile of another segment looks back into it
-        const uint8_t rt = a.route[j];
-        if (rt != NO_ROUTE && rt != slot) {
-            __syncthreads();  // every thread has read s_tile before thread 0 takes the next tile
-            continue;
+        const uint32_t j = tile_seg[t];
+        // a segment takes the MSD pass or the LSD passes; its tiles publish
+        // nothing in the others, and no tile of another segment looks back
+        // into it
+        if (MSD) {
+            const uint8_t rt = a.route[j];
+            if (rt == NO_ROUTE) {
+                __syncthreads();  // every thread has read s_tile before thread 0 takes the next tile
+                continue;
+            }
+            shift = 8 * rt;
         }
-        const K* tsrc_k = rt == NO_ROUTE ? src_k : a.in_k;
-        const uint32_t* tsrc_v = rt == NO_ROUTE ? src_v : a.in_v;
-        K* tdst_k = rt == NO_ROUTE ? dst_k : a.alt_k;
-        uint32_t* tdst_v = rt == NO_ROUTE ? dst_v : a.alt_v;
         const uint32_t s = a.large_list[j];
         const uint32_t segb = a.off[s], sege = a.off[s + 1];
-        const uint32_t lt = t - a.tile_begin[j];
+        const uint32_t lt = t - tile_begin[j];
+        if ((uint64_t)lt * TILE >= sege - segb) {  // a tile outside its segment: never read or written
+            if (tid == 0) dev::raise_error(a.err, dev::ERR_MISPLACED);
+            __syncthreads();
+            continue;
+        }
         const uint32_t tile_base = segb + lt * TILE;
         const uint32_t valid = min((uint32_t)TILE, sege - tile_base);
         const bool first = lt == 0;
@@ -691,10 +777,10 @@ __device__ __forceinline__ void seg_large_pass(const SegArgs<K>& a, int slot, ui
         uint32_t val[HAS_V ? ITEMS : 1];
         if (valid == (uint32_t)TILE) {
 #pragma unroll
-            for (int i = 0; i < ITEMS; ++i) key[i] = tsrc_k[wbase + i * 16];
+            for (int i = 0; i < ITEMS; ++i) key[i] = src_k[wbase + i * 16];
             if (HAS_V) {
 #pragma unroll
-                for (int i = 0; i < ITEMS; ++i) val[i] = tsrc_v[wbase + i * 16];
+                for (int i = 0; i < ITEMS; ++i) val[i] = src_v[wbase + i * 16];
             }
 #pragma unroll
             for (int i = 0; i < ITEMS; ++i) rd[i] = digit(key[i]);
@@ -703,8 +789,8 @@ __device__ __forceinline__ void seg_large_pass(const SegArgs<K>& a, int slot, ui
             for (int i = 0; i < ITEMS; ++i) {
                 const uint32_t idx = wbase + i * 16;
                 const bool in = idx < sege;
-                key[i] = in ? tsrc_k[idx] : K(0);
-                if (HAS_V) val[i] = in ? tsrc_v[idx] : 0u;
+                key[i] = in ? src_k[idx] : K(0);
+                if (HAS_V) val[i] = in ? src_v[idx] : 0u;
                 rd[i] = in ? digit(key[i]) : 0xFFu;  // padding ranks last
             }
         }
@@ -792,7 +878,7 @@ __device__ __forceinline__ void seg_large_pass(const SegArgs<K>& a, int slot, ui
                 }
                 dev::st_relaxed(&my_status[tid], pack_status(FLAG_PRE, seq0 + t, excl + agg));
             }
-            s_bin_off[tid] = a.seg_hist[((size_t)j * P + slot) * RADIX + tid] + excl - s_local[tid];
+            s_bin_off[tid] = a.seg_hist[((size_t)j * P + (shift >> 3)) * RADIX + tid] + excl - s_local[tid];
         }
         __syncthreads();
         const uint32_t limit = s_abort ? 0u : valid;
@@ -809,8 +895,8 @@ __device__ __forceinline__ void seg_large_pass(const SegArgs<K>& a, int slot, ui
 #pragma unroll
             for (int i = 0; i < ITEMS; ++i) {
                 if (o[i] >= segb && o[i] < sege) {
-                    tdst_k[o[i]] = key[i];
-                    if (HAS_V) tdst_v[o[i]] = val[i];
+                    dst_k[o[i]] = key[i];
+                    if (HAS_V) dst_v[o[i]] = val[i];
                 }
             }
         } else {
@@ -818,8 +904,8 @@ __device__ __forceinline__ void seg_large_pass(const SegArgs<K>& a, int slot, ui
                 const K kk = s_keys[q];
                 const uint32_t o = s_bin_off[digit(kk)] + q;
                 if (o >= segb && o < sege) {
-                    tdst_k[o] = kk;
-                    if (HAS_V) tdst_v[o] = s_vals[q];
+                    dst_k[o] = kk;
+                    if (HAS_V) dst_v[o] = s_vals[q];
                 }
             }
         }
@@ -827,20 +913,19 @@ __device__ __forceinline__ void seg_large_pass(const SegArgs<K>& a, int slot, ui
     }
 }
 
-template <typename K, bool HAS_V, int THREADS, int ITEMS, int MINB, int LBW>
-__global__ void __launch_bounds__(THREADS, MINB) k_seg_large_pass(SegArgs<K> a, int slot)
+template <typename K, bool HAS_V, int THREADS, int ITEMS, int MINB, int LBW, bool MSD>
+__global__ void __launch_bounds__(THREADS, MINB) k_seg_large_pass(SegArgs<K> a, int slot, bool with_msd)
 {
-    seg_large_pass<K, HAS_V, THREADS, ITEMS, LBW>(a, slot, gridDim.x);
+    seg_large_pass<K, HAS_V, THREADS, ITEMS, LBW, MSD>(a, slot, with_msd, gridDim.x);
 }
 
 // ---------------------------------------------------------------------------
 // The whole batch in one persistent launch: every phase above in order, with
 // a grid barrier wherever a phase reads what an earlier one wrote (the launch
 // is cooperative, so every CTA is resident). After classification the first
-// large_ctas CTAs take the large-segment phases -- the plan's scan (CTA 0)
-// while they zero the histogram rows; the tile map; the histogram count; the
-// bin starts; [the MSD route]; each digit pass; [the MSD route's bucket
-// sorts] -- with barriers among themselves, and the other CTAs sort the
+// large_ctas CTAs take the large-segment phases -- the tile map and zeroed
+// histogram rows; the histogram count; the bin starts [and the MSD route];
+// [its pass]; each digit pass; [the MSD route's bucket sorts] -- with barriers among themselves, and the other CTAs sort the
 // small and medium segments meanwhile (the two paths share nothing). With
 // large_ctas equal to the grid, every CTA takes both, the small and medium
 // sorts after the histogram count. A barrier wait is bounded (about one
@@ -880,7 +965,7 @@ __global__ void __launch_bounds__(256, 2) k_seg_batch(SegArgs<K> a, int msd, uin
     constexpr int P = Traits<K>::PASSES;
     constexpr int TILE = 256 * ITEMS;
     uint32_t gen = 0, lgen = 0;
-    seg_classify(a);
+    seg_classify<K, TILE>(a);
     if (!grid_barrier(&a.ctl->barrier, gen, gridDim.x, a.err)) return;
     const bool split = large_ctas < gridDim.x;
     if (blockIdx.x >= large_ctas) {
@@ -890,10 +975,7 @@ __global__ void __launch_bounds__(256, 2) k_seg_batch(SegArgs<K> a, int msd, uin
         return;
     }
     uint32_t* arrivals = &a.ctl->large_barrier;
-    if (blockIdx.x == 0) seg_plan_scan<K, TILE, 256>(a);
-    seg_large_zero(a, large_ctas);
-    if (!grid_barrier(arrivals, lgen, large_ctas, a.err)) return;
-    seg_plan_map(a, large_ctas);
+    seg_large_plan<K, TILE>(a, large_ctas);
     if (!grid_barrier(arrivals, lgen, large_ctas, a.err)) return;
     seg_large_count<K, TILE>(a, large_ctas);
     if (!split) {
@@ -902,14 +984,14 @@ __global__ void __launch_bounds__(256, 2) k_seg_batch(SegArgs<K> a, int msd, uin
         seg_small_cta<K, HAS_V, false>(a);
     }
     if (!grid_barrier(arrivals, lgen, large_ctas, a.err)) return;
-    seg_large_starts(a, large_ctas);
+    seg_route<K, TILE>(a, msd != 0, large_ctas);
     if (!grid_barrier(arrivals, lgen, large_ctas, a.err)) return;
     if (msd) {
-        seg_route(a, large_ctas);
+        seg_large_pass<K, HAS_V, 256, ITEMS, LBW, true>(a, 0, true, large_ctas);
         if (!grid_barrier(arrivals, lgen, large_ctas, a.err)) return;
     }
     for (int slot = 0; slot < P; ++slot) {
-        seg_large_pass<K, HAS_V, 256, ITEMS, LBW>(a, slot, large_ctas);
+        seg_large_pass<K, HAS_V, 256, ITEMS, LBW, false>(a, slot, msd != 0, large_ctas);
         if (!grid_barrier(arrivals, lgen, large_ctas, a.err)) return;
     }
     if (msd) {
@@ -922,6 +1004,17 @@ __global__ void __launch_bounds__(256, 2) k_seg_batch(SegArgs<K> a, int msd, uin
 // ---------------------------------------------------------------------------
 // Host
 // ---------------------------------------------------------------------------
+// Batches of few keys are bound by the launches and the longest CTA of each,
+// not by the work: up to FEW_KEYS the longer one-CTA classes share a launch,
+// up to VERY_FEW_KEYS all of them, and 32-bit keys keep to the LSD passes
+// (four passes of a tile or two each, about 13 us apiece, against the MSD
+// route's pass, its sub-bucket launches and the LSD launches that find nothing
+// to do: 347 segments of 264,000 floats and their scan take 86 us with the
+// former, 122 with the latter; eight passes of 64-bit keys lose to the route:
+// 181 us against 151 for 1,800 segments).
+constexpr std::size_t FEW_KEYS = std::size_t(1) << 22;
+constexpr std::size_t VERY_FEW_KEYS = std::size_t(1) << 18;
+
 template <typename K, bool HAS_V> struct LargeShape;
 template <bool HV> struct LargeShape<uint32_t, HV> {
     static constexpr int THREADS = 256, ITEMS = 24, MINB = 2, LBW = HV ? 1 : 4;
@@ -930,42 +1023,67 @@ template <bool HV> struct LargeShape<uint64_t, HV> {
     static constexpr int THREADS = 256, ITEMS = HV ? 20 : 24, MINB = 2, LBW = 4;
 };
 
-template <typename F> static void set_smem(F* kernel, std::size_t bytes)
-{
-    if (bytes > 0)  // static shared memory adds to this against the 48 KiB default
-        check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes),
-                   "cudaFuncSetAttribute");
-}
-
+// CTAs of the kernel that fit an SM with that much dynamic shared memory,
+// after the opt-in to it; asked once per device, kernel and amount (the two
+// queries take longer than a launch).
 template <typename F> static int occupancy(F* kernel, int threads, std::size_t smem)
 {
+    static std::mutex m;
+    static std::map<std::tuple<int, const void*, std::size_t>, int> known;
+    int dev = 0;
+    check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
+    const std::tuple<int, const void*, std::size_t> key(dev, (const void*)kernel, smem);
+    std::lock_guard<std::mutex> lock(m);
+    auto it = known.find(key);
+    if (it != known.end()) return it->second;
+    // static shared memory adds to the dynamic amount against the 48 KiB
+    // default, so the opt-in is always made; it only ever grows
+    static std::map<std::pair<int, const void*>, std::size_t> opted;
+    std::size_t& most = opted[{dev, (const void*)kernel}];
+    if (smem > most) {
+        check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                   "cudaFuncSetAttribute");
+        most = smem;
+    }
     int b = 0;
     check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, threads, smem),
                "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
-    return std::max(b, 1);
+    return known[key] = b;
 }
 
-// The one-CTA sorts of the segments (SUB: sub-buckets) of at most cap keys:
-// 512 threads when threads == 512 and their shared memory fits the opt-in,
-// else 256. (Keys-only u32 at the largest capacity: 16,384 keys in 224 KiB
-// with 512 threads, one CTA per SM either way, so twice the warps hide the
-// shared-memory round trips.)
-template <typename K, bool HAS_V, bool SUB>
-static void launch_cta_sort(device_context& ctx, const SegArgs<K>& a, uint32_t cap, int threads, cudaStream_t st)
+// The one-CTA sorts of the segments (sub: sub-buckets) of at most cap keys
+// among n, a launch per class (small batches: the larger CTA's launch takes
+// the lower classes too); `threads`: the first class's CTAs, 256 (16 keys per
+// thread) or 512 (8).
+template <typename K, bool HAS_V>
+static void launch_cta_sorts(device_context& ctx, const SegArgs<K>& a, bool sub, uint32_t cap, std::size_t n, int threads,
+                             cudaStream_t st)
 {
-    auto wide = &k_seg_small_cta<K, HAS_V, SUB, 512>;
-    const std::size_t wsmem = cta_sort_smem<K, HAS_V>(cap, 512);
-    cudaFuncAttributes fa{};
-    check_cuda(cudaFuncGetAttributes(&fa, wide), "cudaFuncGetAttributes");
-    if (threads == 512 && wsmem + fa.sharedSizeBytes <= ctx.smem_optin) {
-        set_smem(wide, wsmem);
-        wide<<<ctx.sm_count * occupancy(wide, 512, wsmem), 512, wsmem, st>>>(a);
-    } else {
-        auto kern = &k_seg_small_cta<K, HAS_V, SUB, SMALL_THREADS>;
-        const std::size_t smem = cta_sort_smem<K, HAS_V>(cap, SMALL_THREADS);
-        set_smem(kern, smem);
-        kern<<<ctx.sm_count * occupancy(kern, SMALL_THREADS, smem), SMALL_THREADS, smem, st>>>(a);
+    auto launch = [&](auto kern, int cta, std::size_t smem, uint32_t above, int cls, int last) {
+        const std::size_t most = n / (above + 1) + 1;  // segments of the class
+        const int grid = (int)std::min<std::size_t>(most, (std::size_t)ctx.sm_count * std::max(1, occupancy(kern, cta, smem)));
+        kern<<<grid, cta, smem, st>>>(a, cls, last, sub);
+    };
+    constexpr bool SMALL = sizeof(K) == 4;
+    const int lowest = n <= VERY_FEW_KEYS ? 0 : n <= FEW_KEYS ? 1 : 2;  // class that the largest CTA's launch starts at
+    const uint32_t above[CTA_CLASSES] = {(uint32_t)WARP_CAP, CLASS0_CAP, CLASS1_CAP};
+    int done = CTA_CLASSES;  // classes from this one up are launched
+    if (cap > CLASS1_CAP && n > CLASS1_CAP && max_cta_cap<K, HAS_V>() > CLASS1_CAP) {
+        done = lowest;
+        if constexpr (SMALL && !HAS_V)
+            launch(&k_seg_tile<K, HAS_V, 1024, 16, 1>, 1024, tile::Sorter<K, HAS_V, 1024, 16>::SMEM, above[done], done, 2);
+        else if constexpr (max_cta_cap<K, HAS_V>() > CLASS1_CAP)
+            launch(&k_seg_tile<K, HAS_V, 512, 20, 1>, 512, tile::Sorter<K, HAS_V, 512, 20>::SMEM, above[done], done, 2);
     }
+    if (done > 1 && cap > CLASS0_CAP && n > CLASS0_CAP) {
+        done = std::min(lowest, 1);
+        launch(&k_seg_tile<K, HAS_V, 512, 16, SMALL ? 2 : 1>, 512, tile::Sorter<K, HAS_V, 512, 16>::SMEM, above[done], done, 1);
+    }
+    if (done > 0 && threads == 512)
+        launch(&k_seg_tile<K, HAS_V, 512, 8, 2>, 512, tile::Sorter<K, HAS_V, 512, 8>::SMEM, WARP_CAP, 0, 0);
+    else if (done > 0)
+        launch(&k_seg_tile<K, HAS_V, 256, 16, SMALL ? 3 : 2>, 256, tile::Sorter<K, HAS_V, 256, 16>::SMEM, WARP_CAP, 0, 0);
+    check_cuda(cudaGetLastError(), "segmented sort cta launch");
 }
 
 template <typename K, bool HAS_V>
@@ -975,29 +1093,24 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
     constexpr int P = Traits<K>::PASSES;
     using LS = LargeShape<K, HAS_V>;
     constexpr int TILE = LS::THREADS * LS::ITEMS;
-    // Largest segment one CTA sorts in shared memory: two copies of keys (and
-    // values) plus a packed rank per element, and 16 KiB of warp histograms
-    // and peer masks (256 threads; 32 KiB with 512), must fit the 227 KiB
-    // opt-in (u32: 12 B/elem keys-only, 20 B/elem with values; u64: 20 and
-    // 28 B/elem).
-    constexpr int MAX_CAP = sizeof(K) == 4 ? (HAS_V ? 10240 : 16384) : (HAS_V ? 7168 : 10240);
+    constexpr int MAX_CAP = (int)max_cta_cap<K, HAS_V>();
     const uint32_t cta_cap =
         (uint32_t)std::max<int>(WARP_CAP + 1, std::min<int>(opt.cta_cap > 0 ? opt.cta_cap : MAX_CAP, MAX_CAP));
     const uint32_t max_large = (uint32_t)std::min<std::size_t>(nseg, n / (cta_cap + 1) + 1);
     const uint32_t max_tiles = (uint32_t)(n / TILE + max_large + 1);
 
     temp_buffer ctl(ctx.resource, sizeof(SegControl));
-    temp_buffer lists(ctx.resource, (2 * nseg + max_large + (max_large + 1)) * sizeof(uint32_t));
-    temp_buffer tile_seg(ctx.resource, (std::size_t)max_tiles * sizeof(uint32_t));
+    temp_buffer lists(ctx.resource, ((1 + CTA_CLASSES) * nseg + 3 * (std::size_t)max_large) * sizeof(uint32_t));
+    temp_buffer tile_seg(ctx.resource, 2 * (std::size_t)max_tiles * sizeof(uint32_t));
     temp_buffer seg_hist(ctx.resource, (std::size_t)max_large * P * RADIX * sizeof(uint32_t));
     const bool maybe_large = n > cta_cap;
     temp_buffer alt_k(ctx.resource, maybe_large ? n * sizeof(K) : 0);
     temp_buffer alt_v(ctx.resource, maybe_large && HAS_V ? n * sizeof(uint32_t) : 0);
-    // MSD route: per large segment its pass (or none), and at most 256
-    // sub-buckets per large segment (never more than n)
+    // MSD route: per large segment its pass (or none), and at most one
+    // sub-bucket per window of a segment's keys
     const uint32_t msd_cap = opt.msd_cap <= 0 ? 0u : (uint32_t)std::max<int>(WARP_CAP + 1, std::min(opt.msd_cap, MAX_CAP));
     const bool msd = maybe_large && msd_cap > 0;
-    const uint32_t max_sub = msd ? (uint32_t)std::min<std::size_t>((std::size_t)max_large * RADIX, n) : 0;
+    const uint32_t max_sub = msd ? (uint32_t)(n / SUB_WINDOW) + max_large : 0;
     temp_buffer route(ctx.resource, maybe_large ? max_large : 0);
     temp_buffer sub_lists(ctx.resource, (std::size_t)max_sub * 4 * sizeof(uint32_t));
     check_cuda(cudaMemsetAsync(ctl.get(), 0, sizeof(SegControl), ctx.stream), "cudaMemsetAsync");
@@ -1020,18 +1133,19 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
     uint32_t* l = lists.as<uint32_t>();
     a.warp_list = l;
     a.cta_list = l + nseg;
-    a.large_list = l + 2 * nseg;
-    a.tile_begin = l + 2 * nseg + max_large;
+    a.large_list = l + (1 + CTA_CLASSES) * nseg;
+    a.tile_begin = a.large_list + max_large;
     a.tile_seg = tile_seg.as<uint32_t>();
+    a.lsd_begin = msd ? a.tile_begin + max_large : a.tile_begin;
+    a.lsd_seg = msd ? a.tile_seg + max_tiles : a.tile_seg;
     a.seg_hist = seg_hist.as<uint32_t>();
     a.max_large = max_large;
     a.max_tiles = max_tiles;
     a.ring = ctx.lookback_ring;
-    a.seq0 = maybe_large ? ctx.reserve_seq((uint64_t)P * max_tiles) : 0;
+    a.seq0 = maybe_large ? ctx.reserve_seq((uint64_t)(P + 1) * max_tiles) : 0;
     a.err = ctx.d_error;
     a.route = route.as<uint8_t>();
-    a.sub_warp_list = sub_lists.as<uint32_t>();
-    a.sub_cta_list = sub_lists.as<uint32_t>() + 2 * (std::size_t)max_sub;
+    a.sub_lists = sub_lists.as<uint32_t>();
     a.max_sub = max_sub;
     a.sub_cap = msd_cap;
 
@@ -1051,9 +1165,7 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
         auto kern = &k_seg_batch<K, HAS_V, LS::ITEMS, LS::LBW>;
         int per_sm = 0;
         if (smem + 32 * 1024 <= ctx.smem_optin) {
-            set_smem(kern, smem);
-            check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem),
-                       "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+            per_sm = occupancy(kern, 256, smem);
         }
         if (per_sm > 0) {
             const uint32_t grid = (uint32_t)(ctx.sm_count * per_sm);
@@ -1080,7 +1192,7 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
     {
         kernel_timer kt(ctx, "segsort.classify");
         const int grid = (int)std::max<std::size_t>(1, std::min<std::size_t>((nseg + 255) / 256, (std::size_t)ctx.sm_count * 4));
-        k_seg_classify<K><<<grid, 256, 0, ctx.stream>>>(a);
+        k_seg_classify<K, TILE><<<grid, 256, 0, ctx.stream>>>(a);
         check_cuda(cudaGetLastError(), "segmented sort classify launch");
     }
     // Fork: the large-segment path runs on the auxiliary stream.
@@ -1092,50 +1204,52 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
         kernel_timer kt(ctx, "segsort.small_warp");
         const std::size_t smem = per_warp_smem * SMALL_WARPS;
         auto kern = &k_seg_small_warp<K, HAS_V, false>;
-        set_smem(kern, smem);
-        const int grid = ctx.sm_count * occupancy(kern, SMALL_THREADS, smem);
+        const int grid = (int)std::min<std::size_t>((nseg + SMALL_WARPS - 1) / SMALL_WARPS,
+                                                    (std::size_t)ctx.sm_count * std::max(1, occupancy(kern, SMALL_THREADS, smem)));
         kern<<<grid, SMALL_THREADS, smem, ctx.stream>>>(a);
         check_cuda(cudaGetLastError(), "segmented sort warp launch");
     }
     {
         kernel_timer kt(ctx, "segsort.small_cta");
-        launch_cta_sort<K, HAS_V, false>(ctx, a, cta_cap, opt.cta_threads, ctx.stream);
-        check_cuda(cudaGetLastError(), "segmented sort cta launch");
+        launch_cta_sorts<K, HAS_V>(ctx, a, false, cta_cap, n, opt.cta_threads, ctx.stream);
     }
     if (maybe_large) {
         {
             kernel_timer kt(ctx, "segsort.large_histogram", aux);
-            k_seg_plan<K, TILE><<<1, 1024, 0, aux>>>(a);
-            check_cuda(cudaGetLastError(), "segmented sort plan launch");
-            k_seg_large_zero<K><<<ctx.sm_count * 4, 256, 0, aux>>>(a);
+            const int tgrid = (int)std::min<std::size_t>(max_tiles, (std::size_t)ctx.sm_count * 4);
+            k_seg_large_plan<K, TILE><<<tgrid, 256, 0, aux>>>(a);
             auto hk = &k_seg_large_count<K, TILE>;
-            hk<<<ctx.sm_count * occupancy(hk, 256, 0), 256, 0, aux>>>(a);
-            k_seg_large_starts<K><<<ctx.sm_count * 4, 256, 0, aux>>>(a);
+            hk<<<std::min<int>(tgrid, ctx.sm_count * std::max(1, occupancy(hk, 256, 0))), 256, 0, aux>>>(a);
+            k_seg_route<K, TILE><<<(int)std::min<std::size_t>(max_large, (std::size_t)ctx.sm_count * 8), 256, 0, aux>>>(a, msd);
             check_cuda(cudaGetLastError(), "segmented sort histogram launch");
         }
-        if (msd) {
-            k_seg_route<K><<<ctx.sm_count * 4, 256, 0, aux>>>(a);
-            check_cuda(cudaGetLastError(), "segmented sort route launch");
-        }
-        auto pk = &k_seg_large_pass<K, HAS_V, LS::THREADS, LS::ITEMS, LS::MINB, LS::LBW>;
         const std::size_t psmem = large_pass_smem;
-        set_smem(pk, psmem);
-        const int pgrid = ctx.sm_count * occupancy(pk, LS::THREADS, psmem);
+        auto pass_grid = [&](auto kern) {
+            return (int)std::min<std::size_t>(max_tiles, (std::size_t)ctx.sm_count * std::max(1, occupancy(kern, LS::THREADS, psmem)));
+        };
+        if (msd) {
+            auto mk = &k_seg_large_pass<K, HAS_V, LS::THREADS, LS::ITEMS, LS::MINB, LS::LBW, true>;
+            const int mgrid = pass_grid(mk);
+            kernel_timer kt(ctx, "segsort.msd_pass", aux);
+            mk<<<mgrid, LS::THREADS, psmem, aux>>>(a, 0, true);
+            check_cuda(cudaGetLastError(), "segmented sort MSD pass launch");
+        }
+        auto pk = &k_seg_large_pass<K, HAS_V, LS::THREADS, LS::ITEMS, LS::MINB, LS::LBW, false>;
+        const int pgrid = pass_grid(pk);
         for (int s = 0; s < P; ++s) {
             kernel_timer kt(ctx, "segsort.large_pass", aux);
-            pk<<<pgrid, LS::THREADS, psmem, aux>>>(a, s);
+            pk<<<pgrid, LS::THREADS, psmem, aux>>>(a, s, msd);
             check_cuda(cudaGetLastError(), "segmented sort pass launch");
         }
         if (msd) {
             // the MSD route's sub-buckets: from the scratch buffer into the output
-            constexpr std::size_t per_warp =
-                2 * WARP_CAP * sizeof(K) + (HAS_V ? 2 * WARP_CAP * 4 : 0) + WARP_CAP * 4 + 2 * RADIX * 4;
+            kernel_timer kt(ctx, "segsort.sub_buckets", aux);
+            const std::size_t smem = per_warp_smem * SMALL_WARPS;
             auto wk = &k_seg_small_warp<K, HAS_V, true>;
-            set_smem(wk, per_warp * SMALL_WARPS);
-            wk<<<ctx.sm_count * occupancy(wk, SMALL_THREADS, per_warp * SMALL_WARPS), SMALL_THREADS,
-                 per_warp * SMALL_WARPS, aux>>>(a);
-            launch_cta_sort<K, HAS_V, true>(ctx, a, msd_cap, opt.cta_threads, aux);
-            check_cuda(cudaGetLastError(), "segmented sort sub-bucket launch");
+            const int grid = (int)std::min<std::size_t>((max_sub + SMALL_WARPS - 1) / SMALL_WARPS,
+                                                        (std::size_t)ctx.sm_count * std::max(1, occupancy(wk, SMALL_THREADS, smem)));
+            wk<<<grid, SMALL_THREADS, smem, aux>>>(a);
+            launch_cta_sorts<K, HAS_V>(ctx, a, true, msd_cap, n, opt.cta_threads, aux);
         }
     }
     // Join.
@@ -1147,7 +1261,8 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
 
 uint32_t segsort_cta_cap(int key_bytes, bool has_values)
 {
-    return key_bytes == 4 ? (has_values ? 10240u : 16384u) : (has_values ? 7168u : 10240u);
+    return key_bytes == 4 ? (has_values ? seg::max_cta_cap<uint32_t, true>() : seg::max_cta_cap<uint32_t, false>())
+                          : (has_values ? seg::max_cta_cap<uint64_t, true>() : seg::max_cta_cap<uint64_t, false>());
 }
 
 std::string segsort_batch_tuning_key(int key_bytes, bool has_values, std::size_t n, std::size_t num_segments)
@@ -1196,7 +1311,8 @@ void segmented_sort(device_context& ctx, const void* keys_in, void* keys_out, in
         launch_shape shape;
         o.msd_cap = ctx.tuning.lookup(segsort_msd_tuning_key(key_bytes, vals_in != nullptr, n, num_segments), shape)
                         ? shape.variant
-                        : 0;
+                    : key_bytes == 4 && n <= seg::FEW_KEYS ? 0
+                                                           : (int)segsort_cta_cap(key_bytes, vals_in != nullptr);
     }
     if (o.cta_threads == 0) {
         launch_shape shape;

@@ -15,9 +15,13 @@ struct seg_options {
     // order (every key equal), left untouched; only for in-place calls
     const uint8_t* skip = nullptr;
     // MSD route: a large segment whose highest varying digit splits it into
-    // buckets of at most msd_cap keys takes one pass on that digit, then the
-    // shared-memory sorts finish the buckets; 0: every large segment takes
-    // all digit passes; -1: the default (the tuning table's entry, else off)
+    // buckets that fit a one-CTA sort of msd_cap keys (with room for a window
+    // of neighbouring buckets) takes one pass on that digit, then the one-CTA
+    // sorts finish the buckets; 0: every large segment takes all digit
+    // passes; -1: the default (the tuning table's entry, else off for
+    // 32-bit keys in small batches and the one-CTA maximum otherwise: the
+    // batch of 200,000 lognormal segments of u64 pairs takes 12.1 ms with its
+    // scan, 27.0 with the one-CTA sorts of every digit and the route off)
     int msd_cap = -1;
     // 0: a launch per phase, the small/medium and large paths on two
     // streams; 1: the whole batch in one persistent (cooperative) launch with
@@ -25,14 +29,11 @@ struct seg_options {
     // eighths of its CTAs sorting the small and medium segments while the
     // others take the large ones; -1: the tuning table's entry, else 0
     int persistent = -1;
-    // threads of each one-CTA segment sort: 256, or 512 (where the shared
-    // memory of the CTA's capacity fits, else 256), which doubles the warps
-    // in flight. 0: the tuning table's entry for this workload (the
+    // threads of the one-CTA sorts of up to 4,096 keys: 256 (16 keys per
+    // thread) or 512 (8). 0: the tuning table's entry for this workload (the
     // segmented key with ":threads", stored by the autotuner), else its
-    // "segsort:cta_threads" entry, else 256.
-    // 512 pays for segments near the capacity (the learned sort's buckets:
-    // 2.50 -> 1.92 ms at 2^28 keys) and costs for batches of mostly short
-    // ones (200,000 lognormal segments of median 256: 24.7 -> 25.7 ms).
+    // "segsort:cta_threads" entry, else 256. The longer classes have 512 or
+    // 1,024 threads.
     int cta_threads = 0;
 };
 
