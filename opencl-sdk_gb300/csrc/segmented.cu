@@ -1104,8 +1104,8 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
     temp_buffer tile_seg(ctx.resource, 2 * (std::size_t)max_tiles * sizeof(uint32_t));
     temp_buffer seg_hist(ctx.resource, (std::size_t)max_large * P * RADIX * sizeof(uint32_t));
     const bool maybe_large = n > cta_cap;
-    temp_buffer alt_k(ctx.resource, maybe_large ? n * sizeof(K) : 0);
-    temp_buffer alt_v(ctx.resource, maybe_large && HAS_V ? n * sizeof(uint32_t) : 0);
+    temp_buffer alt_k(ctx.resource, maybe_large && opt.alt_keys == nullptr ? n * sizeof(K) : 0);
+    temp_buffer alt_v(ctx.resource, maybe_large && HAS_V && opt.alt_vals == nullptr ? n * sizeof(uint32_t) : 0);
     // MSD route: per large segment its pass (or none), and at most one
     // sub-bucket per window of a segment's keys
     const uint32_t msd_cap = opt.msd_cap <= 0 ? 0u : (uint32_t)std::max<int>(WARP_CAP + 1, std::min(opt.msd_cap, MAX_CAP));
@@ -1120,10 +1120,10 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
     SegArgs<K> a;
     a.in_k = in_k;
     a.out_k = out_k;
-    a.alt_k = alt_k.as<K>();
+    a.alt_k = opt.alt_keys != nullptr ? static_cast<K*>(opt.alt_keys) : alt_k.as<K>();
     a.in_v = in_v;
     a.out_v = out_v;
-    a.alt_v = alt_v.as<uint32_t>();
+    a.alt_v = opt.alt_vals != nullptr ? opt.alt_vals : alt_v.as<uint32_t>();
     a.off = off;
     a.skip = opt.skip;
     a.nseg = (uint32_t)nseg;
@@ -1343,6 +1343,14 @@ void segmented_sort(device_context& ctx, const void* keys_in, void* keys_out, in
             seg::run<uint64_t, false>(ctx, static_cast<const uint64_t*>(keys_in), static_cast<uint64_t*>(keys_out),
                                       nullptr, nullptr, n, offsets, num_segments, xf, o);
     }
+}
+
+void segmented_sort_xf(device_context& ctx, uint64_t* keys, uint32_t* vals, uint64_t xf_a, uint64_t xf_b, std::size_t n,
+                       const uint32_t* offsets, std::size_t num_segments, const seg_options& opt)
+{
+    const dev::KeyXform<uint64_t> xf{xf_a, xf_b};
+    if (vals != nullptr) seg::run<uint64_t, true>(ctx, keys, keys, vals, vals, n, offsets, num_segments, xf, opt);
+    else seg::run<uint64_t, false>(ctx, keys, keys, nullptr, nullptr, n, offsets, num_segments, xf, opt);
 }
 
 }  // namespace gbc

@@ -35,6 +35,9 @@ struct seg_options {
     // "segsort:cta_threads" entry, else 256. The longer classes have 512 or
     // 1,024 threads.
     int cta_threads = 0;
+    // scratch of the call's n keys (and values), or null: from the context's arena
+    void* alt_keys = nullptr;
+    uint32_t* alt_vals = nullptr;
 };
 
 //! Sorts every segment [offsets[i], offsets[i+1]) independently and stably.
@@ -44,6 +47,11 @@ struct seg_options {
 void segmented_sort(device_context& ctx, const void* keys_in, void* keys_out, int key_bytes, int key_kind,
                     const uint32_t* vals_in, uint32_t* vals_out, std::size_t n, const uint32_t* offsets,
                     std::size_t num_segments, bool descending, const seg_options& opt);
+
+//! The same in place for 64-bit keys (and values, or null) whose order is that
+//! of dev::KeyXform{xf_a, xf_b} applied to them.
+void segmented_sort_xf(device_context& ctx, uint64_t* keys, uint32_t* vals, uint64_t xf_a, uint64_t xf_b, std::size_t n,
+                       const uint32_t* offsets, std::size_t num_segments, const seg_options& opt);
 
 //! Scan restarted at every segment start (offsets as for segmented_sort;
 //! position 0 always starts a segment). Exclusive: a segment's first output

@@ -29,6 +29,7 @@
 
 #include "device_common.cuh"
 #include "runtime.hpp"
+#include "segmented.hpp"
 #include "sort_internal.hpp"
 #include "tile_sort.cuh"
 
@@ -1017,6 +1018,14 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1)
     }
 }
 
+}  // namespace onesweep
+}  // namespace gbc
+
+#include "sort_partial.cuh"
+
+namespace gbc {
+namespace onesweep {
+
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
@@ -1151,6 +1160,11 @@ static std::map<std::pair<int, const void*>, int> g_occupancy;  // (device, kern
 static std::mutex g_occupancy_mutex;
 
 template <typename K, bool HAS_V>
+static void run_passes(device_context& ctx, SortArgs<K> a, const PassVariant<K>& pv, int passes, bool copy);
+template <typename K, bool HAS_V>
+static void run_partial(device_context& ctx, const SortArgs<K>& a, const PassVariant<K>& pv);
+
+template <typename K, bool HAS_V>
 static void run_sort(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v,
                      uint32_t* out_v, std::size_t n, dev::KeyXform<K> xf, int variant)
 {
@@ -1207,8 +1221,25 @@ static void run_sort(device_context& ctx, const K* in_k, K* out_k, const uint32_
         check_cuda(cudaGetLastError(), "radix sort histogram launch");
     }
 
+    // The leading digits only, where that is enough (sort_partial.cuh).
+    if constexpr (sizeof(K) == 8) {
+        if (n >= partial::MIN_KEYS) {
+            run_partial<K, HAS_V>(ctx, a, pv);
+            return;
+        }
+    }
+    run_passes<K, HAS_V>(ctx, a, pv, P, true);
+}
+
+// The copy (unless no plan needs it) and `passes` digit passes of the plan in
+// a.ctl (a pass beyond the plan's returns at once).
+template <typename K, bool HAS_V>
+static void run_passes(device_context& ctx, SortArgs<K> a, const PassVariant<K>& pv, int passes, bool copy)
+{
+    const std::size_t n = a.n;
+    const uint32_t num_tiles = a.num_tiles;
     const int cgrid = (int)std::max<std::size_t>(1, std::min<std::size_t>((n + 255) / 256, (std::size_t)ctx.sm_count * 8));
-    {
+    if (copy) {
         kernel_timer kt(ctx, "sort.precopy");
         k_precopy<K><<<cgrid, 256, 0, ctx.stream>>>(a);
         check_cuda(cudaGetLastError(), "radix sort copy launch");
@@ -1216,12 +1247,12 @@ static void run_sort(device_context& ctx, const K* in_k, K* out_k, const uint32_
 
     // K2 x P
     const std::size_t psmem = pass_smem<K>(pv, HAS_V);
-    const bool ident = xf.a == 0 && xf.b == 0;
+    const bool ident = a.xf.a == 0 && a.xf.b == 0;
     auto* pk = ident ? pv.kernel_ident : pv.kernel;
     const int pblocks = prepare_kernel(pk, pv.threads, psmem, g_occupancy, g_occupancy_mutex);
     const int pgrid = (int)std::min<std::size_t>(num_tiles, (std::size_t)ctx.sm_count * pblocks);
     if (pv.hist == nullptr) {
-        for (int s = 0; s < P; ++s) {
+        for (int s = 0; s < passes; ++s) {
             kernel_timer kt(ctx, "sort.digit_pass");
             pk<<<pgrid, pv.threads, psmem, ctx.stream>>>(a, s);
             check_cuda(cudaGetLastError(), "radix sort pass launch");
@@ -1240,7 +1271,7 @@ static void run_sort(device_context& ctx, const K* in_k, K* out_k, const uint32_
     check_cuda(cudaMemsetAsync(a.chunk_off, 0, (std::size_t)a.chunks * RADIX * sizeof(uint32_t), ctx.stream),
                "cudaMemsetAsync");
     auto* hk = ident ? pv.hist_ident : pv.hist;
-    for (int s = 0; s < P; ++s) {
+    for (int s = 0; s < passes; ++s) {
         {
             kernel_timer kt(ctx, "sort.tile_histogram");
             hk<<<a.chunks * TH_SPLIT, TH_THREADS, 0, ctx.stream>>>(a, s);
@@ -1259,6 +1290,89 @@ static void run_sort(device_context& ctx, const K* in_k, K* out_k, const uint32_
             check_cuda(cudaGetLastError(), "radix sort pass launch");
         }
     }
+}
+
+// After the upfront histogram: the fewest leading digits that leave little out
+// of order, their passes, and the repair of what they leave.
+template <typename K, bool HAS_V> static void run_partial(device_context& ctx, const SortArgs<K>& a, const PassVariant<K>& pv)
+{
+    using namespace partial;
+    constexpr uint32_t SEGMENTS = 2 * MAX_LONG - 1;
+    const std::size_t n = a.n;
+    const bool segmented = n >= SEGMENTED_KEYS;
+    int bits = 0;
+    while ((std::size_t(1) << bits) < n) ++bits;
+    // one block: the control words and the plan of all digits (zeroed), then
+    // the tables and the set (all ones), then the lists
+    const std::size_t zeroed = 256 + sizeof(SortControl);
+    const uint32_t sample = sample_size(n);
+    const std::size_t ones = (std::size_t)CANDIDATES * 2 * sample * 8 + LONG_SET * 4;
+    const std::size_t max_faults = (n + FT_TILE - 1) / FT_TILE + 1;
+    temp_buffer head(ctx.resource, zeroed);
+    temp_buffer sets(ctx.resource, ones);
+    temp_buffer lists(ctx.resource, (4 * (std::size_t)MAX_LONG + max_faults) * sizeof(uint32_t) + SEGMENTS);
+    check_cuda(cudaMemsetAsync(head.get(), 0, zeroed, ctx.stream), "cudaMemsetAsync");
+    check_cuda(cudaMemsetAsync(sets.get(), 0xFF, ones, ctx.stream), "cudaMemsetAsync");
+    Args<K> p;
+    p.a = a;
+    p.ctl = head.as<Control>();
+    p.all = reinterpret_cast<SortControl*>(head.as<unsigned char>() + 256);
+    p.tables = sets.as<unsigned long long>();
+    p.sample = sample;
+    p.segmented = segmented;
+    p.set = reinterpret_cast<uint32_t*>(p.tables + (std::size_t)CANDIDATES * 2 * sample);
+    p.least = (bits + 3 + 7) / 8;
+    p.begin = lists.as<uint32_t>();
+    p.end = p.begin + MAX_LONG;
+    p.off = p.end + MAX_LONG;
+    p.fault = p.off + 2 * MAX_LONG;
+    uint8_t* skip = reinterpret_cast<uint8_t*>(p.fault + max_faults);
+    {
+        kernel_timer kt(ctx, "sort.sample");
+        k_sample<K><<<sample / 256, 256, 0, ctx.stream>>>(p);
+        if (segmented) k_odd_segments<<<(SEGMENTS + 255) / 256, 256, 0, ctx.stream>>>(skip, SEGMENTS);
+        check_cuda(cudaGetLastError(), "radix sort sample launch");
+    }
+    run_passes<K, HAS_V>(ctx, a, pv, FIRST_PASSES, true);
+    {
+        kernel_timer kt(ctx, "sort.faults");
+        const int per_sm = prepare_kernel(&k_faults<K, HAS_V>, 256, 0, g_occupancy, g_occupancy_mutex);
+        const int grid = (int)std::min<std::size_t>((n + FT_TILE - 1) / FT_TILE, (std::size_t)ctx.sm_count * per_sm);
+        k_faults<K, HAS_V><<<grid, 256, 0, ctx.stream>>>(p);
+        check_cuda(cudaGetLastError(), "radix sort fault search launch");
+    }
+    {
+        kernel_timer kt(ctx, "sort.repair");
+        k_repair<K, HAS_V><<<std::max<int>(1, std::min<int>((int)(max_faults / 256), ctx.sm_count * 2)), 256, 0, ctx.stream>>>(p);
+        if (segmented) {
+            const std::size_t smem = tile::Sorter<uint32_t, true, 1024, MAX_LONG / 1024>::SMEM;
+            prepare_kernel(&k_long_runs, 1024, smem, g_occupancy, g_occupancy_mutex);
+            k_long_runs<<<1, 1024, smem, ctx.stream>>>(p.ctl, p.all, p.begin, p.end, p.off, a.n, ctx.d_error);
+        } else {
+            const std::size_t smem = tile::Sorter<K, HAS_V, 512, 16>::SMEM;
+            prepare_kernel(&k_sort_long_runs<K, HAS_V>, 512, smem, g_occupancy, g_occupancy_mutex);
+            k_sort_long_runs<K, HAS_V><<<ctx.sm_count, 512, smem, ctx.stream>>>(p, ctx.d_error);
+        }
+        check_cuda(cudaGetLastError(), "radix sort repair launch");
+    }
+    if (segmented) {
+        seg_options so;
+        so.skip = skip;
+        so.persistent = 0;
+        so.cta_threads = 256;
+        so.msd_cap = (int)segsort_cta_cap(sizeof(K), HAS_V);
+        so.alt_keys = a.alt_keys;
+        so.alt_vals = a.alt_vals;
+        segmented_sort_xf(ctx, a.out_keys, a.out_vals, a.xf.a, a.xf.b, n, p.off, SEGMENTS, so);
+    }
+    // The second plan, from the order reached: nothing to do in the usual case.
+    SortArgs<K> all = a;
+    all.in_keys = a.out_keys;
+    all.in_vals = a.out_vals;
+    all.in_place = 1;
+    all.ctl = p.all;
+    all.seq0 = ctx.reserve_seq((uint64_t)Traits<K>::PASSES * a.num_tiles);
+    run_passes<K, HAS_V>(ctx, all, pv, Traits<K>::PASSES, false);
 }
 
 }  // namespace onesweep
