@@ -1377,6 +1377,30 @@ template <typename K, bool HAS_V> static void run_partial(device_context& ctx, c
 
 }  // namespace onesweep
 
+void radix_passes_pairs(device_context& ctx, const uint32_t* keys, uint32_t* keys_out, uint32_t* keys_alt,
+                        const uint32_t* vals, uint32_t* vals_out, uint32_t* vals_alt, std::size_t n,
+                        onesweep::SortControl* ctl, int passes)
+{
+    using namespace onesweep;
+    const PassVariant<uint32_t> pv = Variants<uint32_t, true>::get(0);
+    const uint32_t tile = (uint32_t)(pv.threads * pv.items);
+    SortArgs<uint32_t> a{};
+    a.in_keys = keys;
+    a.out_keys = keys_out;
+    a.alt_keys = keys_alt;
+    a.in_vals = vals;
+    a.out_vals = vals_out;
+    a.alt_vals = vals_alt;
+    a.n = (uint32_t)n;
+    a.in_place = keys == keys_out ? 1 : 0;
+    a.ctl = ctl;
+    a.num_tiles = (uint32_t)((n + tile - 1) / tile);
+    a.ring = ctx.lookback_ring;
+    a.seq0 = ctx.reserve_seq((uint64_t)passes * a.num_tiles);
+    a.err = ctx.d_error;
+    run_passes<uint32_t, true>(ctx, a, pv, passes, false);
+}
+
 int sort_variant_count(int key_bytes, bool has_values)
 {
     using namespace onesweep;

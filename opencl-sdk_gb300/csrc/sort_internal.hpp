@@ -39,6 +39,15 @@ struct SortControl {
 
 }  // namespace onesweep
 
+struct device_context;
+
+//! Digit passes of the plan in `ctl` (device; tile counters zero) over n u32
+//! pairs in unsigned ascending order; `keys` may be `keys_out` when the plan's
+//! number of passes is even.
+void radix_passes_pairs(device_context& ctx, const uint32_t* keys, uint32_t* keys_out, uint32_t* keys_alt,
+                        const uint32_t* vals, uint32_t* vals_out, uint32_t* vals_alt, std::size_t n,
+                        onesweep::SortControl* ctl, int passes);
+
 int sort_variant_count(int key_bytes, bool has_values);
 //! The variant used when the tuning table has no entry for the workload.
 int sort_default_variant(int key_bytes, bool has_values, std::size_t n);

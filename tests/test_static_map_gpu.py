@@ -95,3 +95,46 @@ def test_full_table_and_limits(gbc, ctx, orc):
         gbc.StaticMap(ctx, (1 << 31) + 1)
     with pytest.raises(gbc.InvalidArgumentError):
         m.insert(kb, kb, 2000)  # n beyond the buffers
+
+
+@pytest.mark.parametrize("case", ["half_full", "nearly_full", "few_keys_repeated", "sparse"])
+def test_insert_by_regions(gbc, ctx, orc, case):
+    """Tables of 2^25 slots, from n = capacity / 8 keys: filled region by region in shared memory, with what
+    does not fit a region inserted directly, on top of keys already present, the empty marker among the keys."""
+    cap, early = 1 << 25, 5000
+    rng = np.random.default_rng(4)
+    n = {"half_full": cap // 2, "nearly_full": int(cap * 0.93), "few_keys_repeated": cap // 4, "sparse": cap // 8 + 1}[case]
+    keys = np.arange(n, dtype=np.uint32) * np.uint32(2654435761)  # distinct
+    if case == "few_keys_repeated":  # two keys take three quarters of the input
+        keys[early:][rng.random(n - early) < 0.75] = 12345
+        keys[early::1000] = 67890
+    keys[early + 17] = 0xFFFFFFFF  # the empty marker is skipped
+    vals = rng.integers(0, 1 << 32, size=n, dtype=np.uint32)
+    distinct = np.sort(keys)
+    if case == "few_keys_repeated":
+        distinct = np.unique(distinct)
+    distinct = distinct[:-1]  # without the empty marker
+    m = gbc.StaticMap(ctx, cap)
+    assert m.capacity() == cap
+    kb, vb = gbc.DeviceBuffer.from_host(ctx, keys), gbc.DeviceBuffer.from_host(ctx, vals)
+    assert m.insert(kb, gbc.DeviceBuffer.from_host(ctx, keys ^ np.uint32(0xABCD)), early) == early  # directly
+    assert m.insert(kb, vb) == distinct.size - early
+    assert m.size() == distinct.size
+    assert m.insert(kb, vb) == 0
+    found = gbc.DeviceBuffer(ctx, n, np.uint32)
+    m.find(kb, found)
+    got = found.to_host()
+    assert np.array_equal(got[:early], keys[:early] ^ np.uint32(0xABCD))
+    assert got[early + 17] == 0xFFFFFFFF
+    once = np.ones(n, dtype=bool)
+    once[:early] = False
+    once[early + 17] = False
+    for k in (12345, 67890) if case == "few_keys_repeated" else ():
+        at = keys == k
+        assert np.unique(got[at]).size == 1 and got[at][0] in vals[at]  # one of the key's values
+        once &= ~at
+    assert np.array_equal(got[once], vals[once])
+    sk, _ = m.slots()
+    assert np.array_equal(np.sort(sk)[: distinct.size], distinct)
+    if case in ("few_keys_repeated", "sparse"):
+        assert orc.linear_probe_table_ok(sk, 0xFFFFFFFF)
