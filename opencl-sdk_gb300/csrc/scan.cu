@@ -25,6 +25,7 @@
 #include "../../include/compute_c.h"
 #include "device_common.cuh"
 #include "ops.cuh"
+#include "pipe.cuh"
 #include "runtime.hpp"
 #include "sort_internal.hpp"
 
@@ -346,195 +347,35 @@ __global__ void __launch_bounds__(THREADS, MINB) k_scan(ScanArgs<T> a)
 }
 
 // ---------------------------------------------------------------------------
-// The same scan for large aligned inputs, as a pipeline inside each CTA (one
-// per SM): a warp that takes tiles and copies them to shared memory several
-// tiles ahead, warps that fold a tile as soon as it has landed and publish its
-// aggregate, a warp that finds the tile's prefix, and warps that then scan the
-// tile and write it.
-//
-// In k_scan every warp waits at the CTA barrier while the first one looks
-// back, with no load in flight (2^30 int32: 2.04 ms, 0.62 of the copy rate).
-// A tile taken early there publishes late, and all its successors wait. Here a
-// tile's aggregate needs nothing but its own data, and prefixes are not
-// handed from tile to tile: each CTA keeps the prefix of its last tile and
-// adds the aggregates published since (about one per CTA), so nothing waits for
-// another tile's prefix. Tiles are taken from a counter, so a CTA only waits
-// for tiles that running CTAs hold, and the kernel needs no co-residency.
+// The same scan for large aligned inputs, as a pipeline of specialised warps
+// (pipe.cuh). In k_scan every warp waits at the CTA barrier while the first
+// one looks back, with no load in flight (2^30 int32: 2.04 ms, 0.62 of the copy
+// rate), and a tile taken early publishes late, which all its successors wait
+// for.
 //
 // Measured (2^30 int32 with the int64 total): the same 16 warps folding a tile
 // and writing an earlier one, prefixes read 128 tiles at a time, 2.12 ms; 256
-// at a time 1.53; folding and writing in warps of their own, 1.32 ms, 0.96 of
-// the copy rate. 2^28 int64 2.05 -> 0.89 ms.
+// at a time 1.53; folding and writing in warps of their own 1.33; with the
+// shape and the reads of pipe.cuh 1.21 ms, the copy rate. 2^28 int64 2.05 ->
+// 0.75 ms.
 // ---------------------------------------------------------------------------
-namespace pipe {
-
-constexpr int WRITERS = 16, FOLDERS = 8;               // warps that scan and write, and that fold
-constexpr int THREADS = (WRITERS + FOLDERS + 2) * 32;  // and the prefix warp and the copying warp
-constexpr int ROWS = 4;                                // rows of 512 bytes per writing warp and tile
-constexpr int STAGES = 6;
-constexpr int PER = 8;  // tiles' aggregates read per lane and round trip
-constexpr uint32_t TILE_BYTES = WRITERS * ROWS * 512;
-constexpr std::size_t SMEM = (std::size_t)STAGES * TILE_BYTES;
-constexpr uint32_t END = 0xFFFFFFFFu;
-// Waits inside a CTA outlast its wait for other CTAs, so that only the latter
-// gives up first and is reported.
-constexpr unsigned long long INNER_LIMIT_NS = 4 * dev::SPIN_LIMIT_NS;
-
-// The published aggregate of one tile: a word of (flag | tag | 32 bits of the
-// value), or two for 8-byte elements; every word carries its tag, so they are
-// read in one round trip with no order between them.
-template <typename T> struct Aggregate {
-    static constexpr int WORDS = sizeof(T) / 4;
-    static constexpr uint64_t SLOTS = onesweep::RING_BYTES / 8 / WORDS;
-    __device__ static uint64_t* at(uint64_t* ring, uint64_t seq) { return ring + (seq & (SLOTS - 1)) * WORDS; }
-    __device__ static uint64_t head(uint64_t seq) { return (FLAG_AGG << 62) | ((seq & TAG_MASK) << 32); }
-    __device__ static void publish(uint64_t* ring, uint64_t seq, T v)
-    {
-        const uint64_t bits = to_bits(v);
-#pragma unroll
-        for (int i = 0; i < WORDS; ++i) dev::st_relaxed(at(ring, seq) + i, head(seq) | (uint32_t)(bits >> (32 * i)));
-    }
-    __device__ static bool read(uint64_t* ring, uint64_t seq, T& v)
-    {
-        uint64_t bits = 0;
-        bool ok = true;
-#pragma unroll
-        for (int i = 0; i < WORDS; ++i) {
-            const uint64_t w = dev::ld_relaxed(at(ring, seq) + i);
-            ok &= (w >> 32) == (head(seq) >> 32);
-            bits |= (uint64_t)(uint32_t)w << (32 * i);
-        }
-        v = from_bits<T>(bits);
-        return ok;
-    }
-};
-
-// op over lanes 0 .. count - 1 in order, to every lane (count >= 1).
-template <typename T, typename Op> __device__ __forceinline__ T fold_lanes(T x, int count, Op op)
+template <typename T, typename Op, bool WIDE_SUM>
+__global__ void __launch_bounds__(pipe::THREADS, 1) k_scan_pipe(ScanArgs<T> a)
 {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const T y = __shfl_down_sync(FULL_MASK, x, o);
-        if ((lane & (2 * o - 1)) == 0 && lane + o < count) x = op(x, y);
-    }
-    return __shfl_sync(FULL_MASK, x, 0);
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(dev::smem_addr(bar)) : "memory");
-}
-__device__ __forceinline__ void fold_sync() { asm volatile("bar.sync 1, %0;" ::"n"(FOLDERS * 32) : "memory"); }
-
-template <typename T, typename Op, bool WIDE_SUM> __global__ void __launch_bounds__(THREADS, 1) k_scan_pipe(ScanArgs<T> a)
-{
+    using namespace pipe;
     constexpr int VEC = 16 / sizeof(T);
     constexpr uint32_t TILE = TILE_BYTES / sizeof(T);
-    constexpr int BLOCKS = WRITERS / FOLDERS;  // a tile's blocks (one per writing warp) per folding warp
     // Operators for which a thread may combine its rows before its lane's neighbours.
     constexpr bool ANY_ORDER = !std::is_same<Op, ops::Right>::value;
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES], ready[STAGES];
-    __shared__ uint32_t s_tile[STAGES];
-    __shared__ T s_prefix[STAGES];
-    __shared__ T s_total[2][WRITERS];      // a tile's block totals
-    __shared__ T s_before[STAGES][WRITERS];  // and their exclusive scan (entry 0 unused)
-    __shared__ volatile int s_abort;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __shared__ Shared<T> sh;
+    __shared__ T s_before[STAGES][WRITERS];
+    const Tiles tiles{a.num_tiles, a.tile_ctr, a.ring, a.seq0, a.err};
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const Op op;
-    if (tid == 0) {
-        for (int s = 0; s < STAGES; ++s) {
-            dev::mbar_init(&full[s], 1);
-            dev::mbar_init(&empty[s], WRITERS);
-            dev::mbar_init(&ready[s], 2);  // the prefix, and the blocks' scan
-            s_tile[s] = END;
-        }
-        s_abort = 0;
-        dev::fence_mbar_init();
-    }
-    __syncthreads();
-    auto wait = [&](uint64_t* bar, uint32_t parity) {
-        if (dev::mbar_try_wait(bar, parity)) return;
-        const unsigned long long start = dev::globaltimer();
-        for (uint32_t spin = 1; !dev::mbar_try_wait(bar, parity); ++spin)
-            if ((spin & 63) == 0 && dev::globaltimer() - start > INNER_LIMIT_NS) {
-                dev::raise_error(a.err, dev::ERR_LOOKBACK_TIMEOUT);
-                s_abort = 1;
-                return;
-            }
-    };
-    const uint32_t limit = a.num_tiles + STAGES;  // iterations of every role, at most
-
-    if (warp == WRITERS + FOLDERS + 1) {  // copies
-        if (lane != 0) return;
-        for (uint32_t k = 0; k < limit; ++k) {
-            const int s = k % STAGES;
-            if (k >= STAGES) wait(&empty[s], (k / STAGES - 1) & 1);
-            const uint32_t t = atomicAdd(a.tile_ctr, 1u);
-            if (t >= a.num_tiles) {
-                s_tile[s] = END;
-                mbar_arrive(&full[s]);
-                return;
-            }
-            s_tile[s] = t;
-            if ((uint64_t)(t + 1) * TILE <= a.n) {
-                dev::mbar_arrive_expect_tx(&full[s], TILE_BYTES);
-                dev::bulk_g2s(smem + (std::size_t)s * TILE_BYTES, a.in + (std::size_t)t * TILE, TILE_BYTES, &full[s]);
-            } else {
-                mbar_arrive(&full[s]);  // a partial tile is read where it lies
-            }
-        }
-        return;
-    }
-
-    if (warp == WRITERS + FOLDERS) {  // prefixes
-        T run = a.identity;  // of the tiles before `done`
-        uint32_t done = 0;
-        for (uint32_t k = 0; k < limit; ++k) {
-            const int s = k % STAGES;
-            wait(&full[s], (k / STAGES) & 1);
-            const uint32_t t = *(volatile uint32_t*)&s_tile[s];
-            if (t == END) return;
-            // windows of 32 * PER tiles (more than there are CTAs, so mostly
-            // one), PER consecutive ones per lane, all read before any is
-            // waited for
-            for (uint32_t w = done; w < t; w += 32 * PER) {
-                const uint32_t count = min(32u * PER, t - w);
-                T val[PER];
-                uint32_t missing = 0;
-#pragma unroll
-                for (int q = 0; q < PER; ++q)
-                    if ((uint32_t)(lane * PER + q) < count && !Aggregate<T>::read(a.ring, a.seq0 + w + lane * PER + q, val[q]))
-                        missing |= 1u << q;
-                const unsigned long long start = missing ? dev::globaltimer() : 0;
-                for (uint32_t spin = 1; missing != 0 && !s_abort; ++spin) {
-#pragma unroll
-                    for (int q = 0; q < PER; ++q)
-                        if ((missing >> q & 1u) && Aggregate<T>::read(a.ring, a.seq0 + w + lane * PER + q, val[q]))
-                            missing &= ~(1u << q);
-                    if ((spin & 63) == 0 && dev::globaltimer() - start > dev::SPIN_LIMIT_NS) {
-                        dev::raise_error(a.err, dev::ERR_LOOKBACK_TIMEOUT);
-                        s_abort = 1;
-                    }
-                }
-                __syncwarp();
-                T mine = val[0];
-#pragma unroll
-                for (int q = 1; q < PER; ++q)
-                    if ((uint32_t)(lane * PER + q) < count) mine = op(mine, val[q]);
-                const T sum = fold_lanes(mine, (int)((count + PER - 1) / PER), op);
-                run = w == 0 ? op(a.identity, sum) : op(run, sum);
-            }
-            done = t;
-            if (lane == 0) {
-                s_prefix[s] = run;
-                mbar_arrive(&ready[s]);  // releases the store
-            }
-            __syncwarp();
-        }
-        return;
-    }
+    sh.init();
+    if (warp == COPY_WARP) return copy_role(tiles, sh, smem, a.in, (uint64_t)a.n * sizeof(T));
+    if (warp == PREFIX_WARP) return prefix_role<ANY_ORDER>(tiles, sh, a.identity, op);
 
     // A row of 512 bytes of the tile: this lane's 16 bytes, from the stage or,
     // for a partial tile, from the input (the identity past its end).
@@ -554,24 +395,21 @@ template <typename T, typename Op, bool WIDE_SUM> __global__ void __launch_bound
     if (warp >= WRITERS) {  // folding
         const int f = warp - WRITERS;
         unsigned long long wide = 0;
-        for (uint32_t k = 0; k < limit; ++k) {
-            const int s = k % STAGES;
-            wait(&full[s], (k / STAGES) & 1);
-            const uint32_t t = *(volatile uint32_t*)&s_tile[s];
+        for (uint32_t k = 0; k < limit(tiles); ++k) {
+            const uint32_t t = sh.next(k, a.err);
             if (t == END) break;
             const bool whole = (uint64_t)(t + 1) * TILE <= a.n;
 #pragma unroll
             for (int b = 0; b < BLOCKS; ++b) {
                 T x[ROWS][VEC], acc[ROWS];
 #pragma unroll
-                for (int r = 0; r < ROWS; ++r) load_row(t, s, whole, (f * BLOCKS + b) * ROWS + r, x[r]);
+                for (int r = 0; r < ROWS; ++r) load_row(t, k % STAGES, whole, (f * BLOCKS + b) * ROWS + r, x[r]);
 #pragma unroll
                 for (int r = 0; r < ROWS; ++r) {
                     acc[r] = x[r][0];
 #pragma unroll
                     for (int j = 1; j < VEC; ++j) acc[r] = op(acc[r], x[r][j]);
                     if (WIDE_SUM) {
-                        // a partial tile's padding is the identity, zero for these sums
 #pragma unroll
                         for (int j = 0; j < VEC; ++j) {
                             if (!whole && (uint64_t)t * TILE + (((f * BLOCKS + b) * ROWS + r) * 32 + lane) * VEC + j >= a.n)
@@ -591,17 +429,9 @@ template <typename T, typename Op, bool WIDE_SUM> __global__ void __launch_bound
 #pragma unroll
                     for (int r = 1; r < ROWS; ++r) total = op(total, dev::warp_reduce(acc[r], op));
                 }
-                if (lane == 0) s_total[k & 1][f * BLOCKS + b] = total;
+                if (lane == 0) sh.total[k & 1][f * BLOCKS + b] = total;
             }
-            fold_sync();
-            if (f == 0) {
-                const T mine = s_total[k & 1][lane % WRITERS];
-                const T incl = dev::warp_inclusive_scan(mine, op);
-                if (lane == WRITERS - 1) Aggregate<T>::publish(a.ring, a.seq0 + t, incl);
-                if (lane < WRITERS - 1) s_before[s][lane + 1] = incl;
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&ready[s]);
-            }
+            publish_tile(tiles, sh, k, t, s_before[k % STAGES], op);
         }
         if (WIDE_SUM) {
 #pragma unroll
@@ -611,11 +441,9 @@ template <typename T, typename Op, bool WIDE_SUM> __global__ void __launch_bound
         return;
     }
 
-    // Scanning and writing: each warp its own block of the tile, at its own pace.
-    for (uint32_t k = 0; k < limit; ++k) {
+    for (uint32_t k = 0; k < limit(tiles); ++k) {  // scanning and writing
         const int s = k % STAGES;
-        wait(&full[s], (k / STAGES) & 1);
-        const uint32_t t = *(volatile uint32_t*)&s_tile[s];
+        const uint32_t t = sh.next(k, a.err);
         if (t == END) return;
         const bool whole = (uint64_t)(t + 1) * TILE <= a.n;
         T x[ROWS][VEC], incl[ROWS];
@@ -628,12 +456,12 @@ template <typename T, typename Op, bool WIDE_SUM> __global__ void __launch_bound
             for (int j = 1; j < VEC; ++j) acc = op(acc, x[r][j]);
             incl[r] = dev::warp_inclusive_scan(acc, op);
         }
-        wait(&ready[s], (k / STAGES) & 1);
-        T run_row = *(volatile T*)&s_prefix[s];  // before the block, then before each row
+        sh.wait(&sh.ready[s], k, a.err);
+        T run_row = *(volatile T*)&sh.prefix[s];  // before the block, then before each row
         if (warp > 0) run_row = op(run_row, s_before[s][warp]);
         __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[s]);  // the warp is done with the stage and its slots
-        if (s_abort) continue;
+        if (lane == 0) mbar_arrive(&sh.empty[s]);  // the warp is done with the stage and its slots
+        if (sh.abort) continue;
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) {
             const T left = __shfl_up_sync(FULL_MASK, incl[r], 1);
@@ -664,8 +492,6 @@ template <typename T, typename Op, bool WIDE_SUM> __global__ void __launch_bound
     }
 }
 
-}  // namespace pipe
-
 std::map<std::pair<int, const void*>, int> g_occ;  // (device, kernel): attributes and occupancy are per device
 std::mutex g_occ_m;
 
@@ -692,7 +518,7 @@ template <typename F> int blocks_per_sm(F* kernel, std::size_t smem = 0, int thr
 }
 
 // From this input size the pipelined kernel is the faster one (int32, k_scan
-// against it: 16 MiB 16.0 / 15.2 us, 32 MiB 25.2 / 22.5, 64 MiB 44.8 / 36.9).
+// against it: 16 MiB 16.0 / 15.2 us, 32 MiB 25.2 / 19.0, 64 MiB 44.8 / 32.6).
 constexpr std::size_t PIPE_MIN_BYTES = std::size_t(1) << 24;
 
 struct ScanLaunch {
@@ -738,7 +564,7 @@ struct ScanLaunch {
         const bool use_wide = can_wide && total_dev != nullptr;
         a.total = use_wide ? nullptr : total_dev;
         if (!use_wide) a.wide_sum = nullptr;
-        auto kernel = use_wide ? &pipe::k_scan_pipe<T, Op, can_wide> : &pipe::k_scan_pipe<T, Op, false>;
+        auto kernel = use_wide ? &k_scan_pipe<T, Op, can_wide> : &k_scan_pipe<T, Op, false>;
         blocks_per_sm(kernel, pipe::SMEM, pipe::THREADS);
         const int grid = (int)std::min<std::size_t>(a.num_tiles, (std::size_t)ctx.sm_count);
         {

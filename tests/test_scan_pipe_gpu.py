@@ -6,7 +6,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-TILE_BYTES = 32768
+TILE_BYTES = 40960
 MIN_BYTES = 1 << 24
 
 
