@@ -19,18 +19,15 @@
 //     word counts are turned into offsets by the library's single-pass scan
 //     (the reference's scan client at Compression.cpp:178), which also
 //     yields the total size;
-//   * pack: one warp per chunk, in rounds of 2,048 elements. Lane l packs
-//     elements 64 l .. 64 l + 63 of the round, which occupy exactly 2 x width
-//     whole words, so no word is shared between lanes (the reference ORs
-//     every element into global memory with atomics). The lanes' words are
-//     staged in shared memory at an odd per-lane stride (2 width + 1: the
-//     lanes hit different banks) and written out by the warp in order,
-//     coalesced;
-//   * unpack, delta mode with a mean width of at most 16 bits: one pass. A
+//   * pack: one warp per chunk, in rounds of 1,024 elements, which fill whole
+//     words: the encoded elements go to shared memory, and each lane puts
+//     together every 32nd word of the round from the elements in it (the
+//     reference ORs every element into global memory with atomics);
+//   * unpack, delta mode with a mean width of at most 26 bits: one pass. A
 //     thread decodes 32 consecutive elements from the `width` whole words
 //     that hold them (width a compile-time constant: one funnel shift per
-//     element), the tile sums its deltas, and its prefix comes from a
-//     decoupled look-back;
+//     element), the tile publishes the sum of its deltas, and its prefix is
+//     the sum of what the tiles before it have published;
 //   * unpack, otherwise: one thread per 4 elements (a 128-bit store),
 //     reading the 1-5 packed words that hold them; delta mode then runs the
 //     library's scan in place.
@@ -43,6 +40,7 @@
 
 #include "../../include/compute_c.h"
 #include "device_common.cuh"
+#include "pipe.cuh"
 #include "runtime.hpp"
 #include "sort_internal.hpp"
 
@@ -53,10 +51,8 @@ using dev::FULL_MASK;
 
 constexpr int THREADS = 256;
 constexpr int WARPS = THREADS / 32;
-constexpr int PACK_THREADS = 128;  // 4 warps x 8.1 KiB of staging: static shared memory
-constexpr int PACK_WARPS = PACK_THREADS / 32;
-constexpr uint32_t LANE_ELEMS = 64;          // per lane and round
-constexpr uint32_t ROUND = 32 * LANE_ELEMS;  // per warp and round
+constexpr int PACK_ROWS = 8;                     // rows of 128 elements per round
+constexpr uint32_t ROUND = PACK_ROWS * 128;      // elements per warp and round
 
 __device__ __forceinline__ uint32_t zigzag(uint32_t d) { return (d << 1) ^ (0u - (d >> 31)); }
 __device__ __forceinline__ uint32_t unzigzag(uint32_t v) { return (v >> 1) ^ (0u - (v & 1u)); }
@@ -122,17 +118,20 @@ __global__ void __launch_bounds__(THREADS) k_bp_analyze(const uint32_t* __restri
     }
 }
 
-// One warp per chunk: the header triple and the chunk's packed words.
+// One warp per chunk: the header triple and the chunk's packed words. Bound by
+// DRAM where the loads are (8 x 16 bytes per lane in flight); lane-private runs
+// of 64 elements, read 256 bytes apart, took 389 us for 2 10^8 timestamps, this
+// 223 (0.64 of the copy rate).
 template <bool DELTA>
-__global__ void __launch_bounds__(PACK_THREADS) k_bp_pack(const uint32_t* __restrict__ in, uint32_t n, uint32_t chunk,
+__global__ void __launch_bounds__(THREADS) k_bp_pack(const uint32_t* __restrict__ in, uint32_t n, uint32_t chunk,
                                                      uint32_t chunks, const uint32_t* __restrict__ hdr,
                                                      const uint32_t* __restrict__ offsets, uint32_t* __restrict__ out)
 {
-    __shared__ uint32_t stage[PACK_WARPS][32 * 65];  // per lane 2 x width + 1 <= 65 words
+    __shared__ __align__(16) uint32_t stage[WARPS][ROUND];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t* my = stage[warp];
     const bool vec = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
-    for (uint32_t c = blockIdx.x * PACK_WARPS + warp; c < chunks; c += gridDim.x * PACK_WARPS) {
+    for (uint32_t c = blockIdx.x * WARPS + warp; c < chunks; c += gridDim.x * WARPS) {
         const uint32_t start = c * chunk, count = min(chunk, n - start);
         const uint32_t base = hdr[2 * c], width = hdr[2 * c + 1], off = offsets[c];
         if (lane == 0) {
@@ -142,47 +141,46 @@ __global__ void __launch_bounds__(PACK_THREADS) k_bp_pack(const uint32_t* __rest
         }
         if (width == 0) continue;
         uint32_t* packed = out + 3 * (size_t)chunks + off;
-        const uint32_t lane_words = 2 * width, pitch = lane_words + 1;
+        // x / width for x <= 32 * ROUND = 2^15: the quotient's error term stays below 1 / width
+        const uint32_t inverse = (uint32_t)(((1ull << 32) + width - 1) / width);
+        uint32_t before = DELTA && start > 0 ? in[start - 1] : 0u;  // the element before the round
         for (uint32_t r0 = 0; r0 < count; r0 += ROUND) {
-            // this lane's elements of the round
-            const uint32_t j0 = r0 + lane * LANE_ELEMS;
-            const uint32_t mine = j0 < count ? min(LANE_ELEMS, count - j0) : 0u;
-            uint64_t acc = 0;
-            uint32_t bits = 0, k = 0;
-            auto put = [&](uint32_t v) {
-                acc |= (uint64_t)(v - base) << bits;
-                bits += width;
-                if (bits >= 32) {
-                    my[lane * pitch + k++] = (uint32_t)acc;
-                    acc >>= 32;
-                    bits -= 32;
-                }
-            };
-            const uint32_t i0 = start + j0;
-            if (vec && mine == LANE_ELEMS) {
-                uint32_t prev = DELTA && i0 > 0 ? in[i0 - 1] : 0u;
-#pragma unroll 4
-                for (uint32_t q = 0; q < LANE_ELEMS; q += 4) {
-                    const uint4 w = *reinterpret_cast<const uint4*>(in + i0 + q);
-                    uint32_t e[4];
-                    encode4<DELTA>(w, prev, e);
-                    prev = w.w;
+            const uint32_t rcount = min(ROUND, count - r0), i0 = start + r0 + 4 * lane;
+            uint4 w[PACK_ROWS];
 #pragma unroll
-                    for (int t = 0; t < 4; ++t) put(e[t]);
+            for (int r = 0; r < PACK_ROWS; ++r) {
+                const uint32_t j = r * 128 + 4 * lane, i = i0 + r * 128;
+                if (vec && j + 4 <= rcount) {
+                    w[r] = dev::ld_stream(reinterpret_cast<const uint4*>(in + i));
+                } else {  // past the end: never packed
+                    w[r].x = j < rcount ? in[i] : 0u;
+                    w[r].y = j + 1 < rcount ? in[i + 1] : 0u;
+                    w[r].z = j + 2 < rcount ? in[i + 2] : 0u;
+                    w[r].w = j + 3 < rcount ? in[i + 3] : 0u;
                 }
-            } else {
-                for (uint32_t q = 0; q < mine; ++q) put(encode_at<DELTA>(in, i0 + q));
             }
-            if (bits > 0) my[lane * pitch + k++] = (uint32_t)acc;  // the partial last word
+#pragma unroll
+            for (int r = 0; r < PACK_ROWS; ++r) {
+                uint32_t prev = 0;
+                if (DELTA) {
+                    prev = __shfl_up_sync(FULL_MASK, w[r].w, 1);
+                    if (lane == 0) prev = before;
+                    before = __shfl_sync(FULL_MASK, w[r].w, 31);
+                }
+                uint32_t e[4];
+                encode4<DELTA>(w[r], prev, e);
+                reinterpret_cast<uint4*>(my)[r * 32 + lane] = make_uint4(e[0] - base, e[1] - base, e[2] - base, e[3] - base);
+            }
             __syncwarp();
-            // the round's words, in order: lane l's words are words
-            // [l * 2 width, ...) of the round
-            const uint32_t rcount = min(ROUND, count - r0);
-            const uint32_t rwords = (uint32_t)(((uint64_t)rcount * width + 31) / 32);
-            uint32_t* dst = packed + (size_t)(r0 / 32) * width;  // r0 * width / 32 (r0 is a multiple of 2048)
+            const uint32_t rwords = (rcount * width + 31) / 32;
+            uint32_t* dst = packed + (size_t)(r0 / 32) * width;  // r0 * width / 32 (r0 is a multiple of ROUND)
             for (uint32_t m = lane; m < rwords; m += 32) {
-                const uint32_t l = m / lane_words, kk = m - l * lane_words;
-                dst[m] = my[l * pitch + kk];
+                uint32_t j = __umulhi(32 * m, inverse);  // the element holding the word's first bit (width 1: 2^32 wraps)
+                if (width == 1) j = 32 * m;
+                const uint32_t skip = 32 * m - j * width;
+                uint32_t word = my[j] >> skip;
+                for (uint32_t have = width - skip; have < 32 && ++j < rcount; have += width) word |= my[j] << have;
+                dst[m] = word;
             }
             __syncwarp();
         }
@@ -237,37 +235,23 @@ __global__ void __launch_bounds__(THREADS) k_bp_unpack(const uint32_t* __restric
     }
 }
 
-// ---- fused unpack (and, in delta mode, the prefix sum that undoes it) -------
-// Lane-private whole words: a thread decodes 32 consecutive elements of one
-// chunk, which occupy exactly `width` whole words of the packed area (element
-// j sits at bit j * width and 32 * width bits are width words), so with the
-// width as a compile-time constant every shift and word index is a constant
-// (one funnel shift, a mask and an add per element). A CTA's 8,192 elements
-// form one tile. In delta mode the tile's deltas are scanned in place
-// (thread, warp, CTA) and the tile's prefix comes from a decoupled look-back
-// over the context's status ring, so the prefix sum costs no pass of its own.
-// The decoded tile is staged in shared memory at an odd stride and written
-// out coalesced.
+// ---- unpack by lane-private whole words ---------------------------------------
+// A thread decodes 32 consecutive elements of one chunk, which occupy exactly
+// `width` whole words of the packed area (element j sits at bit j * width and
+// 32 * width bits are width words), so with the width as a compile-time
+// constant every shift and word index is a constant (one funnel shift, a mask
+// and an add per element). A CTA's 8,192 elements form one tile. In delta mode
+// the tile's deltas are scanned in place (thread, warp, CTA), its sum is
+// published at once, and its prefix is the sum of the published ones: every
+// thread keeps its share of those before the CTA's last tile and adds its
+// share of those since (about one per running CTA, read in one round trip).
+// Nothing waits for another tile's prefix: the decoupled look-back that this
+// replaces took 542 us for 2 10^8 timestamps, a first pass for the sums and a
+// second one 350, this 319. The decoded tile is staged in shared memory at
+// an odd stride and written out coalesced.
 constexpr int UT = 256;             // threads per CTA
 constexpr int UE = 32;              // elements per thread
 constexpr int UTILE = UT * UE;      // elements per tile
-constexpr int U_LBL = 4;            // look-back: 32 x 4 tiles per round trip
-constexpr uint64_t U_SLOTS = onesweep::RING_BYTES / 8;
-constexpr uint64_t U_AGG = 1, U_PRE = 2, U_TAG = (1ull << 30) - 1;
-
-__device__ __forceinline__ void u_publish(uint64_t* ring, uint64_t seq, uint64_t flag, uint32_t v)
-{
-    dev::st_relaxed(&ring[seq & (U_SLOTS - 1)], (flag << 62) | ((seq & U_TAG) << 32) | v);
-}
-
-__device__ __forceinline__ bool u_read(const uint64_t* ring, uint64_t seq, uint64_t& flag, uint32_t& v)
-{
-    const uint64_t w = dev::ld_relaxed(&ring[seq & (U_SLOTS - 1)]);
-    flag = w >> 62;
-    if (flag == 0 || ((w >> 32) & U_TAG) != (seq & U_TAG)) return false;
-    v = (uint32_t)w;
-    return true;
-}
 
 // Elements of the lane's 32 (all in one chunk) from its W packed words at p;
 // `words_left` bounds the reads at the end of the buffer.
@@ -310,25 +294,36 @@ __device__ __forceinline__ void decode_dispatch(uint32_t width, const uint32_t* 
     }
 }
 
-template <bool DELTA>
-__global__ void __launch_bounds__(UT, 2)
-    k_bp_unpack_tiles(const uint32_t* __restrict__ data, uint64_t words, uint32_t n, uint32_t chunk_shift,
-                      uint32_t chunks, uint32_t* __restrict__ out, uint32_t num_tiles, uint32_t* tile_ctr,
-                      uint64_t* ring, uint64_t seq0, int* err)
+// The sum of one value per thread over the CTA, to every thread.
+__device__ __forceinline__ uint32_t cta_sum(uint32_t x, uint32_t* scratch)
 {
+    x = __reduce_add_sync(FULL_MASK, x);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = x;
+    __syncthreads();
+    uint32_t all = 0;
+#pragma unroll
+    for (int w = 0; w < UT / 32; ++w) all += scratch[w];
+    return all;
+}
+
+template <bool DELTA>
+__global__ void __launch_bounds__(UT)
+    k_bp_unpack_tiles(const uint32_t* __restrict__ data, uint64_t words, uint32_t n, uint32_t chunk_shift,
+                      uint32_t chunks, uint32_t* __restrict__ out, pipe::Tiles tiles)
+{
+    using Sum = pipe::Aggregate<uint32_t>;
     __shared__ uint32_t s_out[UT * (UE + 1)];
     __shared__ uint32_t s_warp[UT / 32];
-    __shared__ uint32_t s_prefix;
     __shared__ uint32_t s_tile;
-    __shared__ int s_abort;  // a look-back wait gave up: the outputs are unknown, nothing is written
+    uint32_t share = 0, done = 0;  // of the sums of the tiles before `done`
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t* packed = data + 3 * (size_t)chunks;
-    if (tid == 0) s_abort = 0;
     for (;;) {
-        if (tid == 0) s_tile = atomicAdd(tile_ctr, 1u);
+        if (tid == 0) s_tile = atomicAdd(tiles.counter, 1u);
         __syncthreads();
         const uint32_t t = s_tile;
-        if (t >= num_tiles) break;
+        if (t >= tiles.num_tiles) break;
         const uint32_t i0 = t * UTILE + tid * UE;  // the thread's first element
         uint32_t v[UE];
         if (i0 < n) {
@@ -350,112 +345,72 @@ __global__ void __launch_bounds__(UT, 2)
             for (int e = 0; e < UE; ++e) v[e] = 0;
         }
         if (DELTA) {
-            // undo the zigzag, then the thread's, the warp's and the CTA's
-            // inclusive sums (wrapping)
+            // undo the zigzag, then the thread's inclusive sums (wrapping)
 #pragma unroll
             for (int e = 0; e < UE; ++e) v[e] = unzigzag(v[e]);
 #pragma unroll
             for (int e = 1; e < UE; ++e) v[e] += v[e - 1];
+        }
+        bool abort = false;
+        if (DELTA) {
+            const uint32_t sum = cta_sum(v[UE - 1], s_warp);
+            if (tid == 0) Sum::publish(tiles.ring, tiles.seq0 + t, sum);
+            for (uint32_t k = done + tid; k < t; k += UT) {
+                uint32_t x;
+                if (!Sum::read(tiles.ring, tiles.seq0 + k, x)) {
+                    const unsigned long long start = dev::globaltimer();
+                    for (uint32_t spin = 1; !Sum::read(tiles.ring, tiles.seq0 + k, x); ++spin) {
+                        if ((spin & 63) == 0 && dev::globaltimer() - start > dev::SPIN_LIMIT_NS) {
+                            dev::raise_error(tiles.err, dev::ERR_LOOKBACK_TIMEOUT);
+                            abort = true;
+                            break;
+                        }
+                        if (spin > 4) __nanosleep(64);
+                    }
+                    if (abort) break;
+                }
+                share += x;
+            }
+            done = t;
+            const uint32_t before = cta_sum(share, s_warp);
             uint32_t inc = v[UE - 1];
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const uint32_t y = __shfl_up_sync(FULL_MASK, inc, o);
                 if (lane >= o) inc += y;
             }
+            __syncthreads();
             if (lane == 31) s_warp[warp] = inc;
-            const uint32_t lane_excl = inc - v[UE - 1];
             __syncthreads();
-            if (warp == 0) {
-                uint32_t wt = lane < UT / 32 ? s_warp[lane] : 0u;
+            uint32_t add = before + inc - v[UE - 1];
 #pragma unroll
-                for (int o = 1; o < UT / 32; o <<= 1) {
-                    const uint32_t y = __shfl_up_sync(FULL_MASK, wt, o);
-                    if (lane >= o) wt += y;
-                }
-                const uint32_t agg = __shfl_sync(FULL_MASK, wt, UT / 32 - 1);
-                // exclusive warp offsets
-                const uint32_t wexcl = __shfl_up_sync(FULL_MASK, wt, 1);
-                if (lane < UT / 32) s_warp[lane] = lane == 0 ? 0u : wexcl;
-                const uint64_t my_seq = seq0 + t;
-                if (lane == 0) u_publish(ring, my_seq, t == 0 ? U_PRE : U_AGG, agg);
-                uint32_t excl = 0;
-                if (t > 0) {
-                    bool gave_up = false;
-                    int64_t w_end = t;
-                    for (;;) {
-                        uint64_t flag[U_LBL];
-                        uint32_t val[U_LBL];
-#pragma unroll
-                        for (int q = 0; q < U_LBL; ++q) {
-                            const int64_t k = w_end - 32 * U_LBL + lane * U_LBL + q;
-                            flag[q] = U_PRE;  // before tile 0: an empty inclusive prefix
-                            val[q] = 0;
-                            if (k >= 0 && !u_read(ring, seq0 + (uint64_t)k, flag[q], val[q])) {
-                                const unsigned long long start = dev::globaltimer();
-                                for (uint32_t spin = 1;; ++spin) {
-                                    if (u_read(ring, seq0 + (uint64_t)k, flag[q], val[q])) break;
-                                    if ((spin & 255) == 0 && dev::globaltimer() - start > dev::SPIN_LIMIT_NS) {
-                                        gave_up = true;
-                                        flag[q] = U_PRE;
-                                        val[q] = 0;
-                                        break;
-                                    }
-                                    if (spin > 32) __nanosleep(64);
-                                }
-                            }
-                        }
-                        int hi = -1;  // this lane's nearest inclusive prefix
-#pragma unroll
-                        for (int q = 0; q < U_LBL; ++q)
-                            if (flag[q] == U_PRE) hi = q;
-                        const uint32_t pre = __ballot_sync(FULL_MASK, hi >= 0);
-                        const int L = pre ? 31 - __clz(pre) : -1;
-                        uint32_t contrib = 0;
-                        if (lane >= L) {
-                            const int q0 = lane == L ? hi : 0;
-#pragma unroll
-                            for (int q = 0; q < U_LBL; ++q)
-                                if (q >= q0) contrib += val[q];
-                        }
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) contrib += __shfl_xor_sync(FULL_MASK, contrib, o);
-                        excl += contrib;
-                        if (pre) break;
-                        w_end -= 32 * U_LBL;
-                    }
-                    if (__any_sync(FULL_MASK, gave_up) && lane == 0) {
-                        dev::raise_error(err, dev::ERR_LOOKBACK_TIMEOUT);
-                        s_abort = 1;
-                    }
-                    if (lane == 0) u_publish(ring, my_seq, U_PRE, excl + agg);
-                }
-                if (lane == 0) s_prefix = excl;
-            }
-            __syncthreads();
-            const uint32_t add = s_prefix + s_warp[warp] + lane_excl;
+            for (int w = 0; w < UT / 32; ++w)
+                if (w < warp) add += s_warp[w];
 #pragma unroll
             for (int e = 0; e < UE; ++e) v[e] += add;
         }
-        // stage at stride UE + 1 (conflict-free both ways) and write coalesced
+        // after a timed-out wait the prefix is unknown: nothing is written any more
+        if (__syncthreads_or(abort)) break;
+        {
+            // stage at stride UE + 1 (conflict-free both ways) and write coalesced
 #pragma unroll
-        for (int e = 0; e < UE; ++e) s_out[tid * (UE + 1) + e] = v[e];
-        __syncthreads();
-        const uint32_t tb = t * UTILE;
-        if (s_abort) {
-            // after a timed-out wait the prefix is unknown: nothing is written
-        } else if (tb + UTILE <= n) {
+            for (int e = 0; e < UE; ++e) s_out[tid * (UE + 1) + e] = v[e];
+            __syncthreads();
+            const uint32_t tb = t * UTILE;
+            if (tb + UTILE <= n) {
 #pragma unroll 8
-            for (int k = 0; k < UE; ++k) {
-                const uint32_t idx = k * UT + tid;
-                out[tb + idx] = s_out[(idx / UE) * (UE + 1) + idx % UE];
+                for (int k = 0; k < UE; ++k) {
+                    const uint32_t idx = k * UT + tid;
+                    out[tb + idx] = s_out[(idx / UE) * (UE + 1) + idx % UE];
+                }
+            } else {
+                for (int k = 0; k < UE; ++k) {
+                    const uint32_t idx = k * UT + tid;
+                    if (tb + idx < n) out[tb + idx] = s_out[(idx / UE) * (UE + 1) + idx % UE];
+                }
             }
-        } else {
-            for (int k = 0; k < UE; ++k) {
-                const uint32_t idx = k * UT + tid;
-                if (tb + idx < n) out[tb + idx] = s_out[(idx / UE) * (UE + 1) + idx % UE];
-            }
+            __syncthreads();
         }
-        __syncthreads();
     }
 }
 
@@ -511,14 +466,13 @@ std::size_t bitpack_compress(device_context& ctx, const uint32_t* in, std::size_
     check_cuda(cudaStreamSynchronize(ctx.stream), "cudaStreamSynchronize");
     const std::size_t out_words = 3 * (std::size_t)chunks + packed;
     uint32_t* out = make_output(out_words);
-    const int pgrid = grid_for(ctx, chunks, PACK_WARPS);
     {
         kernel_timer kt(ctx, "bitpack.pack");
         if (delta)
-            k_bp_pack<true><<<pgrid, PACK_THREADS, 0, ctx.stream>>>(in, (uint32_t)n, (uint32_t)chunk, chunks,
+            k_bp_pack<true><<<grid, THREADS, 0, ctx.stream>>>(in, (uint32_t)n, (uint32_t)chunk, chunks,
                                                               hdr.as<uint32_t>(), offs.as<uint32_t>(), out);
         else
-            k_bp_pack<false><<<pgrid, PACK_THREADS, 0, ctx.stream>>>(in, (uint32_t)n, (uint32_t)chunk, chunks,
+            k_bp_pack<false><<<grid, THREADS, 0, ctx.stream>>>(in, (uint32_t)n, (uint32_t)chunk, chunks,
                                                                hdr.as<uint32_t>(), offs.as<uint32_t>(), out);
         check_cuda(cudaGetLastError(), "bitpack pack launch");
     }
@@ -538,28 +492,31 @@ void bitpack_decompress(device_context& ctx, const uint32_t* data, std::size_t w
     ctx.activate();
     uint32_t shift = 0;
     while ((std::size_t(1) << shift) < chunk) ++shift;
-    // Delta mode with a mean packed width of at most 16 bits (known from the
-    // compressed size): one pass that decodes and sums (the timestamp recipe
-    // at 2^28: 0.73 ms against 0.91 for unpack + scan). Wider data, and plain
-    // mode, decode faster as 4-element groups (the lane-private form issues
-    // W scattered loads per lane: 1.1 ms against 0.42 at 32 bits).
+    // Delta mode with a mean packed width of at most 26 bits (known from the
+    // compressed size): whole words per lane in one pass (2 10^8 elements, one
+    // pass / two: 7 bits 0.32 / 0.56 ms, 18 bits 0.35 / 0.56, 25 bits 0.43 /
+    // 0.56). Wider data, and plain mode, decode faster as 4-element groups (the
+    // lane-private form issues W scattered loads per lane: 2^28 words, plain,
+    // 1.1 ms against 0.42 at 32 bits).
     const uint64_t packed_words = words - 3 * (uint64_t)chunks;
-    const bool one_pass = delta && packed_words * 32 <= (uint64_t)n * 16;
+    const bool one_pass = delta && packed_words * 32 <= (uint64_t)n * 26;
     launch_shape sh;
     const int forced = ctx.tuning.lookup("bitpack:unpack", sh) ? sh.variant : -1;  // 0: one pass, 1: two passes
     if (forced == 0 || (forced != 1 && one_pass)) {
         const uint32_t num_tiles = (uint32_t)((n + UTILE - 1) / UTILE);
-        uint32_t* tile_ctr = reinterpret_cast<uint32_t*>(ctx.d_small + 3072);
-        check_cuda(cudaMemsetAsync(tile_ctr, 0, 4, ctx.stream), "cudaMemsetAsync");
-        const uint64_t seq0 = ctx.reserve_seq(num_tiles);
+        pipe::Tiles tiles;
+        tiles.num_tiles = num_tiles;
+        tiles.counter = reinterpret_cast<uint32_t*>(ctx.d_small + 3072);
+        check_cuda(cudaMemsetAsync(tiles.counter, 0, 4, ctx.stream), "cudaMemsetAsync");
+        tiles.ring = ctx.lookback_ring;
+        tiles.seq0 = ctx.reserve_seq(num_tiles);
+        tiles.err = ctx.d_error;
         auto kern = delta ? &k_bp_unpack_tiles<true> : &k_bp_unpack_tiles<false>;
         int per_sm = 1;
         check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, UT, 0), "cudaOccupancy");
-        const int grid = (int)std::max<std::size_t>(
-            1, std::min<std::size_t>(num_tiles, (std::size_t)ctx.sm_count * std::max(per_sm, 1)));
+        const int grid = (int)std::min<std::size_t>(num_tiles, (std::size_t)ctx.sm_count * std::max(per_sm, 1));
         kernel_timer kt(ctx, "bitpack.unpack");
-        kern<<<grid, UT, 0, ctx.stream>>>(data, (uint64_t)words, (uint32_t)n, shift, chunks, out, num_tiles, tile_ctr,
-                                          ctx.lookback_ring, seq0, ctx.d_error);
+        kern<<<grid, UT, 0, ctx.stream>>>(data, (uint64_t)words, (uint32_t)n, shift, chunks, out, tiles);
         check_cuda(cudaGetLastError(), "bitpack unpack launch");
         return;
     }
