@@ -19,7 +19,9 @@
 // measured slower: occupancy. Four or eight interleaved copies of each
 // warp's histogram, lane l counting into copy l % copies, measured no faster
 // for 2^30 bytes (0.41 / 0.37 ms against 0.38) and slower for floats: the
-// shared atomic instruction rate, not bank conflicts, is the limit.)
+// shared atomic instruction rate, not bank conflicts, is the limit.) Many
+// bytes are therefore counted in pairs, one atomic for two of them
+// (k_histogram_pairs).
 #include <cmath>
 #include <cstring>
 #include <limits>
@@ -101,6 +103,142 @@ __global__ void __launch_bounds__(THREADS)
     }
 }
 
+// ---------------------------------------------------------------------------
+// Bytes in pairs: one CTA per SM counts its share of the input into 65,536
+// 16-bit counters, two to a word (128 KiB), and adds them up by value after
+// every batch. The bin rule is applied to the 256 values' totals at the end.
+//
+// A counter may wrap, and carry into its neighbour: either loses 65,535 or
+// 65,536 from the sum of all counters and nothing adds to it, so a batch whose
+// counters do not add up to its pairs is counted again, by bytes, into per-warp
+// 32-bit histograms, and so is the rest of the CTA's share. A first batch too
+// small to wrap tells whether one pair is so frequent that this is to be
+// expected (or that its atomics meet on one address).
+//
+// 2^30 uniform bytes: 384 -> 269 us (one read at the copy rate 158; loading
+// alone takes 150, the pairs' atomics 234, and with the counters' old values
+// returned, to see them wrap, 293).
+// ---------------------------------------------------------------------------
+constexpr int PAIR_THREADS = 1024, PAIR_WARPS = PAIR_THREADS / 32;
+constexpr int PAIR_FIRST = 4;    // 16-byte loads per thread in the first batch: 32,768 pairs
+constexpr int PAIR_BATCH = 64;   // and in the others: 524,288 pairs
+constexpr uint32_t PAIR_COMMON = 32768 / 10;  // a pair's count in the first batch that rules pairs out
+constexpr std::size_t PAIR_SMEM = 32768 * 4;
+// Below, the CTAs' 128 KiB to clear and add up cost too much where the pairs are
+// given up (uniform / one value in nine places of ten / constant bytes, by
+// bytes and by pairs: 2^26 29.7 / 24.3 / 22.7 and 27.6 / 36.9 / 36.5 us; 2^28
+// 101.6 / 74.8 / 74.7 and 76.0 / 73.5 / 70.6).
+constexpr std::size_t PAIR_MIN = std::size_t(1) << 28;
+
+template <typename T> __global__ void __launch_bounds__(PAIR_THREADS, 1)
+    k_histogram_pairs(const T* __restrict__ in, uint32_t n, uint32_t* __restrict__ hist, uint32_t bins, float lower, float upper)
+{
+    extern __shared__ uint32_t sh[];  // pair (a, b): half b / 128 of word (b % 128) * 256 + a
+    __shared__ uint32_t s_value[256], s_sum, s_most;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const uint4* vin = reinterpret_cast<const uint4*>(in);
+    const uint32_t nv = n / 16;
+    const uint32_t first = (uint32_t)((uint64_t)nv * blockIdx.x / gridDim.x);
+    const uint32_t last = (uint32_t)((uint64_t)nv * (blockIdx.x + 1) / gridDim.x);
+    if (tid < 256) s_value[tid] = 0;
+    auto clear = [&] {
+        __syncthreads();
+        for (int i = tid; i < (int)(PAIR_SMEM / 16); i += PAIR_THREADS) reinterpret_cast<uint4*>(sh)[i] = make_uint4(0, 0, 0, 0);
+        __syncthreads();
+    };
+    // f(word) for the four words of every vector of [b, e), four loads in flight
+    auto words = [&](uint32_t b, uint32_t e, auto f) {
+        uint32_t v = b + tid;
+        for (; v + 3 * PAIR_THREADS < e; v += 4 * PAIR_THREADS) {
+            uint4 w[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) w[q] = dev::ld_stream(vin + v + q * PAIR_THREADS);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) f(w[q].x), f(w[q].y), f(w[q].z), f(w[q].w);
+        }
+        for (; v < e; v += PAIR_THREADS) {
+            const uint4 w = dev::ld_stream(vin + v);
+            f(w.x), f(w.y), f(w.z), f(w.w);
+        }
+    };
+    auto pair = [&](uint32_t x) { atomicAdd(&sh[x & 0x7FFFu], x & 0x8000u ? 0x10000u : 1u); };
+
+    uint32_t b = first;  // what is left of the share
+    clear();
+    for (uint32_t size = PAIR_FIRST * PAIR_THREADS; b < last; size = PAIR_BATCH * PAIR_THREADS) {
+        const uint32_t e = min(last, b + size);
+        words(b, e, [&](uint32_t w) { pair(w & 0xFFFFu), pair(w >> 16); });
+        if (tid == 0) s_sum = s_most = 0;
+        __syncthreads();
+        // by first value: a value and a quarter of the rows per thread
+        uint32_t sum = 0, most = 0;
+        for (int r = 0; r < 32; ++r) {
+            const uint32_t w = sh[((tid >> 8) * 32 + r) * 256 + (tid & 255)];
+            sum += (w & 0xFFFFu) + (w >> 16);
+            most = max(most, max(w & 0xFFFFu, w >> 16));
+        }
+        const uint32_t warp_sum = __reduce_add_sync(dev::FULL_MASK, sum);
+        most = __reduce_max_sync(dev::FULL_MASK, most);
+        if ((tid & 31) == 0) {
+            atomicAdd(&s_sum, warp_sum);
+            atomicMax(&s_most, most);
+        }
+        __syncthreads();
+        if (s_sum != (e - b) * 8) break;  // a counter has wrapped: this batch again
+        const bool common = b == first && s_most > PAIR_COMMON;
+        if (sum != 0) atomicAdd(&s_value[tid & 255], sum);
+        // by second value: eight threads per row, 32 words each, every lane of
+        // a warp in a bank of its own
+        uint32_t low = 0, high = 0;
+        const int row = tid >> 3, seg = tid & 7;
+        for (int i = 0; i < 32; ++i) {
+            const uint32_t w = sh[row * 256 + seg * 32 + ((i + tid) & 31)];
+            low += w & 0xFFFFu;
+            high += w >> 16;
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) {
+            low += __shfl_down_sync(dev::FULL_MASK, low, o, 8);
+            high += __shfl_down_sync(dev::FULL_MASK, high, o, 8);
+        }
+        if (seg == 0) {
+            if (low != 0) atomicAdd(&s_value[row], low);
+            if (high != 0) atomicAdd(&s_value[row + 128], high);
+        }
+        b = e;
+        clear();
+        if (common) break;
+    }
+    if (b < last) {  // the rest by bytes
+        clear();
+        uint32_t* my = sh + warp * 256;
+        words(b, last, [&](uint32_t w) {
+            atomicAdd(&my[w & 0xFF], 1u);
+            atomicAdd(&my[w >> 8 & 0xFF], 1u);
+            atomicAdd(&my[w >> 16 & 0xFF], 1u);
+            atomicAdd(&my[w >> 24], 1u);
+        });
+        __syncthreads();
+        if (tid < 256) {
+            uint32_t s = 0;
+            for (int w = 0; w < PAIR_WARPS; ++w) s += sh[w * 256 + tid];
+            s_value[tid] += s;
+        }
+    }
+    __syncthreads();
+    if (blockIdx.x == 0 && tid < (int)(n - 16 * nv))
+        atomicAdd(&s_value[reinterpret_cast<const uint8_t*>(in)[16 * (std::size_t)nv + tid]], 1u);
+    __syncthreads();
+    if (tid < 256 && s_value[tid] != 0) {
+        const float x = (float)(T)(uint8_t)tid, scale = (float)bins / (upper - lower);
+        if (x >= lower && x < upper) {
+            uint32_t bin = (uint32_t)((x - lower) * scale);
+            if (bin >= bins) bin = bins - 1;
+            atomicAdd(&hist[bin], s_value[tid]);
+        }
+    }
+}
+
 // True when, for every value v of T, the device's float rule gives exactly
 // bin v - offset (or excludes v exactly when v - offset is outside [0, bins)).
 // Evaluated over all 2^8 / 2^16 values with the same float operations the
@@ -136,6 +274,18 @@ void launch(device_context& ctx, const void* in, uint32_t n, uint32_t* hist, uin
     using ACC = typename std::conditional<std::is_same<T, double>::value, double, float>::type;
     const ACC lo = static_cast<ACC>(lower), hi = static_cast<ACC>(upper);
     constexpr int VEC = 16 / sizeof(T);
+    if constexpr (sizeof(T) == 1) {
+        if (n >= PAIR_MIN && (reinterpret_cast<uintptr_t>(in) & 15) == 0 && ctx.smem_optin >= PAIR_SMEM + 4096) {
+            auto kernel = &k_histogram_pairs<T>;
+            if (first_use_on_device((const void*)kernel))
+                check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAIR_SMEM),
+                           "cudaFuncSetAttribute");
+            kernel_timer kt(ctx, "histogram.pairs");
+            kernel<<<ctx.sm_count, PAIR_THREADS, PAIR_SMEM, ctx.stream>>>(static_cast<const T*>(in), n, hist, bins, lo, hi);
+            check_cuda(cudaGetLastError(), "histogram launch");
+            return;
+        }
+    }
     const std::size_t warp_bytes = (std::size_t)bins * 4 * WARPS;
     const std::size_t cta_bytes = (std::size_t)bins * 4;
     int m;
