@@ -1043,8 +1043,8 @@ template <typename K> struct PassVariant {
 
 template <typename K, bool HAS_V> struct Variants;
 
-// Variant 0 is the default when the tuning table has no entry; the order
-// below puts the fastest measured shape first (keys only and key-value
+// sort_default_variant picks the shape when the tuning table has no entry:
+// entry 0 except where a note below says otherwise (keys only and key-value
 // differ).
 #define GBC_P1(K, HV, T, I, M) PassVariant<K>{T, I, false, false, &k_pass<K, HV, T, I, M>, &k_pass<K, HV, T, I, M>}
 #define GBC_P1B(K, HV, T, I, B) \
@@ -1062,11 +1062,18 @@ template <typename K, bool HAS_V> struct Variants;
                    &k_tile_hist<K, false, T * I>, &k_tile_hist<K, true, T * I>}
 template <bool HV> struct Variants<uint32_t, HV> {
     static constexpr int count = 13;
-    // The tile-offset form (PAD 1), the default for keys without values from
-    // 2^27 keys when the tuning table has no entry (2^28 uniform: 4.77 ms
-    // against 5.04; 2^27: 2.45 against 2.53; smaller sizes and key-value
-    // sorts are faster with the look-back).
-    static constexpr int TILE_OFFSETS = 11;
+    // 32 keys a thread, the default for keys without values from 2^21 keys: a
+    // third fewer tiles to look back over, and longer runs of a digit to write
+    // (against 24: 2^21 87 us for 95, 2^24 341 for 370, 2^28 4.43 ms for 5.01
+    // and 4.58 with the tile-offset form; at 2^20 68 us for 67, as the last
+    // wave is short). 40 gain 2 % more at 2^28 and lose 3 % at 2^22. Pairs
+    // stay at 24: 28 and 32 cost 3 to 6 % from 2^22.
+    static constexpr int LONG_TILES = 7;
+    // 8 a thread, the default to 2^18 elements: the passes are then a chain of
+    // launches that each take a tile's latency, with most SMs idle (2^14 keys
+    // 43 us for 49, pairs 48 for 55; 2^18 56 for 56 and 56 for 64; at 2^19
+    // pairs 71 for 65).
+    static constexpr int SHORT_TILES = 8;
     static PassVariant<uint32_t> get(int i)
     {
         static const PassVariant<uint32_t> v[count] = {
@@ -1078,10 +1085,11 @@ template <bool HV> struct Variants<uint32_t, HV> {
             HV ? GBC_P2R(uint32_t, HV, 256, 24, 2, 4, false, true, 1) : GBC_P2R(uint32_t, HV, 256, 24, 2, 4, true, true, 1),
             HV ? GBC_P2R(uint32_t, HV, 256, 24, 2, 4, false, true, 2) : GBC_P2R(uint32_t, HV, 256, 24, 2, 4, true, true, 2),
             HV ? GBC_P2(uint32_t, HV, 256, 24, 2, 4, true, true) : GBC_P2(uint32_t, HV, 256, 24, 2, 4, false, true),
-            GBC_P2(uint32_t, HV, 512, 12, 2, 4, false, true),
-            GBC_P2(uint32_t, HV, 384, 16, 2, 4, false, true),
+            HV ? GBC_P2(uint32_t, HV, 512, 12, 2, 4, false, true) : GBC_P2H(uint32_t, HV, 256, 32, 2, 4, false, true, 1),
+            GBC_P2XPK(uint32_t, HV, 256, 8, 4, 4, false, true, 0, true, 1, HV),
             GBC_P1(uint32_t, HV, 256, 16, false),
             GBC_P1B(uint32_t, HV, 256, 16, 3),
+            // with a pass that counts each tile's digits first, no look-back
             GBC_P2T(uint32_t, HV, 256, 24, 2, true, true, 1, HV),
             GBC_P2T(uint32_t, HV, 256, 24, 2, true, true, 0, HV),
         };
@@ -1090,6 +1098,9 @@ template <bool HV> struct Variants<uint32_t, HV> {
 };
 template <bool HV> struct Variants<uint64_t, HV> {
     static constexpr int count = 9;
+    // As for 32 bits: 2^14 keys 85 us for 100, 2^18 102 for 114 (pairs 107 for
+    // 118); at 2^20 167 for 138. Longer tiles than entry 0's gain nothing here.
+    static constexpr int SHORT_TILES = 6;
     static PassVariant<uint64_t> get(int i)
     {
         static const PassVariant<uint64_t> v[count] = {
@@ -1099,7 +1110,7 @@ template <bool HV> struct Variants<uint64_t, HV> {
             HV ? GBC_P2(uint64_t, HV, 256, 24, 2, 4, false, true) : GBC_P2(uint64_t, HV, 256, 20, 2, 4, false, true),
             GBC_P2(uint64_t, HV, 256, 16, 2, 4, false, true),
             GBC_P2(uint64_t, HV, 256, 12, 2, 4, false, true),
-            GBC_P2(uint64_t, HV, 256, 16, 2, 1, false, true),
+            GBC_P2H(uint64_t, HV, 256, 8, 4, 4, false, true, 1),
             GBC_P1(uint64_t, HV, 256, 12, false),
             GBC_P1(uint64_t, HV, 256, 12, true),
         };
@@ -1411,7 +1422,10 @@ int sort_variant_count(int key_bytes, bool has_values)
 int sort_default_variant(int key_bytes, bool has_values, std::size_t n)
 {
     using namespace onesweep;
-    return key_bytes == 4 && !has_values && n >= (std::size_t(1) << 27) ? Variants<uint32_t, false>::TILE_OFFSETS : 0;
+    const bool small = n <= (std::size_t(1) << 18), large = n >= (std::size_t(1) << 21);
+    if (key_bytes == 8) return small ? Variants<uint64_t, false>::SHORT_TILES : 0;
+    if (small) return Variants<uint32_t, false>::SHORT_TILES;
+    return large && !has_values ? Variants<uint32_t, false>::LONG_TILES : 0;
 }
 
 std::string sort_tuning_key(int key_bytes, bool has_values, std::size_t n)
