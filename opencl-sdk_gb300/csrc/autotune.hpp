@@ -17,7 +17,6 @@ struct autotune_result {
     double best_ms = 0;       // its mean time per call
     std::vector<int> candidates;
     std::vector<double> ms;   // mean time per call of every candidate
-    double persistent_ms = 0;  // segmented: the fastest one-launch form's time
 };
 
 //! Plain radix sort: every compiled digit-pass variant (tile shape, CTAs per
@@ -27,11 +26,10 @@ struct autotune_result {
 autotune_result autotune_sort(device_context& ctx, const void* keys_in, void* keys_out, int key_bytes, int key_kind,
                               const uint32_t* vals_in, uint32_t* vals_out, std::size_t n, int repetitions);
 
-//! Segmented sort, in four stages on the caller's batch: the capacity of the
+//! Segmented sort, in three stages on the caller's batch: the capacity of the
 //! one-CTA size class (segments up to that length are sorted in one CTA's
 //! shared memory, longer ones by the batched onesweep), the MSD route's
-//! bucket capacity, the one-CTA sorts' thread count (256 or 512), and the
-//! launch form (the launch sequence or one persistent launch); each is
+//! bucket capacity, and the one-CTA sorts' thread count (256 or 512); each is
 //! stored under its own key. keys_in must differ from keys_out.
 autotune_result autotune_segmented_sort(device_context& ctx, const void* keys_in, void* keys_out, int key_bytes,
                                         int key_kind, const uint32_t* vals_in, uint32_t* vals_out, std::size_t n,

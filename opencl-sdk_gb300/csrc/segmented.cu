@@ -91,8 +91,6 @@ struct SegControl {
     uint32_t msd_tile_ctr;
     uint32_t n_sub_warp, n_sub_cta[CTA_CLASSES];  // sub-bucket list lengths (MSD route)
     uint32_t sub_warp_next, sub_cta_next[CTA_CLASSES];
-    uint32_t barrier;                    // arrivals at the persistent batch's first grid barrier
-    uint32_t large_barrier;              // ... and at those among its large-segment CTAs
 };
 
 template <typename K> struct SegArgs {
@@ -207,58 +205,36 @@ template <typename K, int TILE> __device__ __forceinline__ void seg_large_plan(c
 template <typename K, int TILE> __global__ void k_seg_large_plan(SegArgs<K> a) { seg_large_plan<K, TILE>(a, gridDim.x); }
 
 // ---------------------------------------------------------------------------
-// Shared-memory LSD sort of one segment by a group of GW warps (GW = 1: a
-// warp on its own; GW = the CTA's warps: the whole CTA). Stable: items are ranked
-// in index order (warp chunk, row, lane) and scattered by digit.
-// ---------------------------------------------------------------------------
-template <int GW> __device__ __forceinline__ void group_sync()
-{
-    if (GW == 1) __syncwarp();
-    else __syncthreads();
-}
-
+// Shared-memory LSD sort of one segment by a warp. Stable: items are ranked in
+// index order (row, lane) and scattered by digit.
+//
 // Ranking is by shared-memory peer masks, as in the digit pass: each lane ORs
-// its bit into its digit's mask word (GW x 256 words in `masks`, all zero
-// between rows), reads the word back (its peers) and the warp's count of the
-// digit so far; the lowest peer stores the new count and clears the mask.
+// its bit into its digit's mask word (256 words in `wm`, all zero between
+// rows), reads the word back (its peers) and the count of the digit so far;
+// the lowest peer stores the new count and clears the mask.
 // (__match_any_sync ranked the same rows about 1.7x slower on this GPU.)
-template <typename K, bool HAS_V, int GW>
-__device__ void group_sort(K* k0, K* k1, uint32_t* v0, uint32_t* v1, uint32_t* rd, uint32_t* hist,
-                           uint32_t* masks, uint32_t* scratch, uint32_t len, dev::KeyXform<K> xf, int gw, int lane,
-                           bool& in_k1)
+// ---------------------------------------------------------------------------
+template <typename K, bool HAS_V>
+__device__ void warp_sort(K* k0, K* k1, uint32_t* v0, uint32_t* v1, uint32_t* rd, uint32_t* wh, uint32_t* wm, uint32_t len,
+                          dev::KeyXform<K> xf, int lane, bool& in_k1)
 {
     constexpr int P = Traits<K>::PASSES;
     // Which digit positions vary inside the segment.
     K diff = 0;
     const K first = xf(k0[0]);
-    for (uint32_t i = gw * 32 + lane; i < len; i += GW * 32) diff |= xf(k0[i]) ^ first;
+    for (uint32_t i = lane; i < len; i += 32) diff |= xf(k0[i]) ^ first;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) diff |= __shfl_xor_sync(FULL_MASK, diff, o);
-    if (GW > 1) {
-        // combine the warps' masks (scratch holds 2 x 32 words)
-        if (lane == 0) {
-            scratch[gw * 2] = (uint32_t)diff;
-            scratch[gw * 2 + 1] = (uint32_t)((uint64_t)diff >> 32);
-        }
-        __syncthreads();
-        uint64_t all = 0;
-        for (int w = 0; w < GW; ++w) all |= (uint64_t)scratch[w * 2] | ((uint64_t)scratch[w * 2 + 1] << 32);
-        diff = (K)all;
-        __syncthreads();
-    }
-    const uint32_t chunk = ((len + GW * 32 - 1) / (GW * 32)) * 32;  // items per warp, whole rows
-    const uint32_t rows = chunk / 32;
+    const uint32_t rows = (len + 31) / 32;
     in_k1 = false;
     for (int p = 0; p < P; ++p) {
         if ((((uint64_t)diff >> (8 * p)) & 0xFF) == 0) continue;
         const int shift = 8 * p;
-        for (int i = (GW > 1 ? threadIdx.x : lane); i < GW * RADIX; i += GW * 32) hist[i] = 0;
-        group_sync<GW>();
-        uint32_t* wh = hist + gw * RADIX;
-        uint32_t* wm = masks + gw * RADIX;
+        for (int i = lane; i < RADIX; i += 32) wh[i] = 0;
+        __syncwarp();
         const uint32_t lt = dev::lanemask_lt();
         for (uint32_t r = 0; r < rows; ++r) {
-            const uint32_t idx = gw * chunk + r * 32 + lane;
+            const uint32_t idx = r * 32 + lane;
             const bool valid = idx < len;
             // padding ranks in bin 255 (counted there, never placed)
             const uint32_t d = valid ? (uint32_t)(xf(k0[idx]) >> shift) & 0xFFu : 0xFFu;
@@ -275,38 +251,23 @@ __device__ void group_sort(K* k0, K* k1, uint32_t* v0, uint32_t* v1, uint32_t* r
             __syncwarp();
             if (valid) rd[idx] = ((before + __popc(lower)) << 8) | d;
         }
-        group_sync<GW>();
-        // digit starts and per-warp offsets
-        if (GW == 1) {
-            uint32_t c[8], s = 0;
+        __syncwarp();
+        // digit starts
+        uint32_t c[8], s = 0;
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                c[q] = hist[lane * 8 + q];
-                s += c[q];
-            }
-            const uint32_t incl = dev::warp_inclusive_scan(s, [](uint32_t x, uint32_t y) { return x + y; });
-            uint32_t run = incl - s;
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                hist[lane * 8 + q] = run;
-                run += c[q];
-            }
-        } else {
-            uint32_t count = 0;
-            if (threadIdx.x < RADIX) {
-                for (int w = 0; w < GW; ++w) {
-                    const uint32_t c = hist[w * RADIX + threadIdx.x];
-                    hist[w * RADIX + threadIdx.x] = count;
-                    count += c;
-                }
-            }
-            const uint32_t start = dev::bins_exclusive_sum(count, scratch + 64);
-            if (threadIdx.x < RADIX)
-                for (int w = 0; w < GW; ++w) hist[w * RADIX + threadIdx.x] += start;
+        for (int q = 0; q < 8; ++q) {
+            c[q] = wh[lane * 8 + q];
+            s += c[q];
         }
-        group_sync<GW>();
+        uint32_t run = dev::warp_inclusive_scan(s, [](uint32_t x, uint32_t y) { return x + y; }) - s;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            wh[lane * 8 + q] = run;
+            run += c[q];
+        }
+        __syncwarp();
         for (uint32_t r = 0; r < rows; ++r) {
-            const uint32_t idx = gw * chunk + r * 32 + lane;
+            const uint32_t idx = r * 32 + lane;
             if (idx < len) {
                 const uint32_t x = rd[idx];
                 const uint32_t pos = wh[x & 0xFF] + (x >> 8);
@@ -314,7 +275,7 @@ __device__ void group_sort(K* k0, K* k1, uint32_t* v0, uint32_t* v1, uint32_t* r
                 if (HAS_V) v1[pos] = v0[idx];
             }
         }
-        group_sync<GW>();
+        __syncwarp();
         K* tk = k0;
         k0 = k1;
         k1 = tk;
@@ -367,7 +328,7 @@ template <typename K, bool HAS_V, bool SUB> __device__ __forceinline__ void seg_
         }
         __syncwarp();
         bool flipped = false;
-        if (len > 1) group_sort<K, HAS_V, 1>(k0, k1, v0, v1, rd, hist, masks, nullptr, len, a.xf, 0, lane, flipped);
+        if (len > 1) warp_sort<K, HAS_V>(k0, k1, v0, v1, rd, hist, masks, len, a.xf, lane, flipped);
         const K* rk = flipped ? k1 : k0;
         const uint32_t* rv = flipped ? v1 : v0;
         for (uint32_t i = lane; i < len; i += 32) {
@@ -382,73 +343,6 @@ template <typename K, bool HAS_V, bool SUB>
 __global__ void __launch_bounds__(SMALL_THREADS) k_seg_small_warp(SegArgs<K> a)
 {
     seg_small_warp<K, HAS_V, SUB>(a);
-}
-
-// The one-CTA sorts inside the persistent batch kernel: every class of up to
-// cta_cap (SUB: sub_cap) keys with the same shared-memory sort, which holds
-// any length in the shared memory that the kernel was launched with.
-template <typename K, bool HAS_V, bool SUB> __device__ __forceinline__ void seg_small_cta(const SegArgs<K>& a)
-{
-    constexpr int THREADS = SMALL_THREADS;
-    constexpr int WARPS = THREADS / 32;
-    static_assert(THREADS % 32 == 0 && THREADS >= RADIX && WARPS <= 32, "one thread per bin; scratch holds 32 warps");
-    extern __shared__ __align__(16) unsigned char smem[];
-    const uint32_t cap = SUB ? a.sub_cap : a.cta_cap;
-    K* k0 = reinterpret_cast<K*>(smem);
-    K* k1 = k0 + cap;
-    uint32_t* v0 = reinterpret_cast<uint32_t*>(k1 + cap);
-    uint32_t* v1 = v0 + (HAS_V ? cap : 0);
-    uint32_t* rd = v1 + (HAS_V ? cap : 0);
-    uint32_t* hist = rd + cap;
-    uint32_t* masks = hist + WARPS * RADIX;
-    for (int i = threadIdx.x; i < WARPS * RADIX; i += THREADS) masks[i] = 0;
-    __shared__ uint32_t scratch[64 + 8];
-    __shared__ uint32_t s_work;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const K* src_k = SUB ? a.alt_k : a.in_k;
-    const uint32_t* src_v = SUB ? a.alt_v : a.in_v;
-    int cls = 0;
-    for (;;) {
-        if (threadIdx.x == 0) s_work = atomicAdd(SUB ? &a.ctl->sub_cta_next[cls] : &a.ctl->cta_next[cls], 1u);
-        __syncthreads();
-        const uint32_t w = s_work;
-        if (w >= (SUB ? min(a.ctl->n_sub_cta[cls], a.max_sub) : a.ctl->n_cta[cls])) {
-            if (++cls == CTA_CLASSES) break;
-            __syncthreads();  // every thread has read s_work
-            continue;
-        }
-        uint32_t b, len;
-        if (SUB) {
-            const uint2 r = *sub_entry(a, cls, w);
-            b = r.x;
-            len = r.y - r.x;
-        } else {
-            const uint32_t s = a.cta_list[(std::size_t)cls * a.nseg + w];
-            b = a.off[s];
-            len = a.off[s + 1] - b;
-        }
-        for (uint32_t i = threadIdx.x; i < len; i += THREADS) {
-            k0[i] = src_k[b + i];
-            if (HAS_V) v0[i] = src_v[b + i];
-        }
-        __syncthreads();
-        bool flipped = false;
-        group_sort<K, HAS_V, WARPS>(k0, k1, v0, v1, rd, hist, masks, scratch, len, a.xf, warp, lane, flipped);
-        const K* rk = flipped ? k1 : k0;
-        const uint32_t* rv = flipped ? v1 : v0;
-        for (uint32_t i = threadIdx.x; i < len; i += THREADS) {
-            a.out_k[b + i] = rk[i];
-            if (HAS_V) a.out_v[b + i] = rv[i];
-        }
-        __syncthreads();
-    }
-}
-
-//! Shared memory of that sort: two copies of keys (and values) and a packed
-//! rank per element, then a histogram and a peer-mask array per warp.
-template <typename K, bool HAS_V> constexpr std::size_t cta_sort_smem(uint32_t cap, int threads)
-{
-    return (std::size_t)cap * (2 * sizeof(K) + (HAS_V ? 8 : 0) + 4) + 2 * (std::size_t)(threads / 32) * RADIX * 4;
 }
 
 // The one-CTA sorts of classes cls to last (tile_sort.cuh): persistent CTAs
@@ -920,88 +814,6 @@ __global__ void __launch_bounds__(THREADS, MINB) k_seg_large_pass(SegArgs<K> a, 
 }
 
 // ---------------------------------------------------------------------------
-// The whole batch in one persistent launch: every phase above in order, with
-// a grid barrier wherever a phase reads what an earlier one wrote (the launch
-// is cooperative, so every CTA is resident). After classification the first
-// large_ctas CTAs take the large-segment phases -- the tile map and zeroed
-// histogram rows; the histogram count; the bin starts [and the MSD route];
-// [its pass]; each digit pass; [the MSD route's bucket sorts] -- with barriers among themselves, and the other CTAs sort the
-// small and medium segments meanwhile (the two paths share nothing). With
-// large_ctas equal to the grid, every CTA takes both, the small and medium
-// sorts after the histogram count. A barrier wait is bounded (about one
-// second): a CTA that gives up records ERR_LOOKBACK_TIMEOUT and returns, so
-// no later phase runs on incomplete data, and the others give up at their
-// next barrier in turn.
-// ---------------------------------------------------------------------------
-// The first `parties` CTAs of the grid take part; `generation` counts the
-// barriers passed (kept by thread 0).
-__device__ __forceinline__ bool grid_barrier(uint32_t* arrivals, uint32_t& generation, uint32_t parties, int* err)
-{
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        s_ok = 1;
-        __threadfence();
-        atomicAdd(arrivals, 1u);
-        const uint32_t target = ++generation * parties;
-        const unsigned long long t0 = dev::globaltimer();
-        for (uint32_t spin = 1; dev::ld_acquire(arrivals) < target; ++spin) {
-            if ((spin & 63) == 0 && dev::globaltimer() - t0 > dev::SPIN_LIMIT_NS) {
-                dev::raise_error(err, dev::ERR_LOOKBACK_TIMEOUT);
-                s_ok = 0;
-                break;
-            }
-            if (spin > 16) __nanosleep(64);
-        }
-        __threadfence();
-    }
-    __syncthreads();
-    return s_ok != 0;
-}
-
-template <typename K, bool HAS_V, int ITEMS, int LBW>
-__global__ void __launch_bounds__(256, 2) k_seg_batch(SegArgs<K> a, int msd, uint32_t large_ctas)
-{
-    constexpr int P = Traits<K>::PASSES;
-    constexpr int TILE = 256 * ITEMS;
-    uint32_t gen = 0, lgen = 0;
-    seg_classify<K, TILE>(a);
-    if (!grid_barrier(&a.ctl->barrier, gen, gridDim.x, a.err)) return;
-    const bool split = large_ctas < gridDim.x;
-    if (blockIdx.x >= large_ctas) {
-        seg_small_warp<K, HAS_V, false>(a);
-        __syncthreads();
-        seg_small_cta<K, HAS_V, false>(a);
-        return;
-    }
-    uint32_t* arrivals = &a.ctl->large_barrier;
-    seg_large_plan<K, TILE>(a, large_ctas);
-    if (!grid_barrier(arrivals, lgen, large_ctas, a.err)) return;
-    seg_large_count<K, TILE>(a, large_ctas);
-    if (!split) {
-        seg_small_warp<K, HAS_V, false>(a);
-        __syncthreads();
-        seg_small_cta<K, HAS_V, false>(a);
-    }
-    if (!grid_barrier(arrivals, lgen, large_ctas, a.err)) return;
-    seg_route<K, TILE>(a, msd != 0, large_ctas);
-    if (!grid_barrier(arrivals, lgen, large_ctas, a.err)) return;
-    if (msd) {
-        seg_large_pass<K, HAS_V, 256, ITEMS, LBW, true>(a, 0, true, large_ctas);
-        if (!grid_barrier(arrivals, lgen, large_ctas, a.err)) return;
-    }
-    for (int slot = 0; slot < P; ++slot) {
-        seg_large_pass<K, HAS_V, 256, ITEMS, LBW, false>(a, slot, msd != 0, large_ctas);
-        if (!grid_barrier(arrivals, lgen, large_ctas, a.err)) return;
-    }
-    if (msd) {
-        seg_small_warp<K, HAS_V, true>(a);
-        __syncthreads();
-        seg_small_cta<K, HAS_V, true>(a);
-    }
-}
-
-// ---------------------------------------------------------------------------
 // Host
 // ---------------------------------------------------------------------------
 // Batches of few keys are bound by the launches and the longest CTA of each,
@@ -1151,44 +963,9 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
 
     constexpr std::size_t per_warp_smem =
         2 * WARP_CAP * sizeof(K) + (HAS_V ? 2 * WARP_CAP * 4 : 0) + WARP_CAP * 4 + 2 * RADIX * 4;
-    auto cta_smem = [](uint32_t cap) { return cta_sort_smem<K, HAS_V>(cap, SMALL_THREADS); };
     // the large pass: two half-warp count arrays of RADIX + LARGE_PAD words per warp, and a tile
     constexpr std::size_t large_pass_smem = (std::size_t)(LS::THREADS / 32) * (RADIX + LARGE_PAD) * 8 +
                                             (std::size_t)TILE * sizeof(K) + (HAS_V ? (std::size_t)TILE * 4 : 0);
-    if (opt.persistent > 0) {
-        // One cooperative launch of every phase; its shared memory is the
-        // largest any phase needs. Falls through to the launch sequence below
-        // when not even one CTA per SM fits.
-        const std::size_t pass_smem = large_pass_smem;
-        const std::size_t smem = std::max({per_warp_smem * SMALL_WARPS, cta_smem(cta_cap), pass_smem,
-                                           msd ? cta_smem(msd_cap) : std::size_t(0)});
-        auto kern = &k_seg_batch<K, HAS_V, LS::ITEMS, LS::LBW>;
-        int per_sm = 0;
-        if (smem + 32 * 1024 <= ctx.smem_optin) {
-            per_sm = occupancy(kern, 256, smem);
-        }
-        if (per_sm > 0) {
-            const uint32_t grid = (uint32_t)(ctx.sm_count * per_sm);
-            // persistent >= 2: that many eighths (less one) of the grid sort
-            // the small and medium segments while the rest take the large ones
-            const uint32_t small_ctas = opt.persistent >= 2 ? grid * (uint32_t)std::min(opt.persistent - 1, 6) / 8 : 0;
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(grid);
-            cfg.blockDim = dim3(256);
-            cfg.dynamicSmemBytes = smem;
-            cfg.stream = ctx.stream;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeCooperative;
-            attr[0].val.cooperative = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            kernel_timer kt(ctx, "segsort.batch");
-            check_cuda(cudaLaunchKernelEx(&cfg, kern, a, msd ? 1 : 0, grid - small_ctas),
-                       "segmented sort batch launch");
-            return;
-        }
-    }
-
     {
         kernel_timer kt(ctx, "segsort.classify");
         const int grid = (int)std::max<std::size_t>(1, std::min<std::size_t>((nseg + 255) / 256, (std::size_t)ctx.sm_count * 4));
@@ -1319,12 +1096,6 @@ void segmented_sort(device_context& ctx, const void* keys_in, void* keys_out, in
         if (ctx.tuning.lookup(segsort_threads_tuning_key(key_bytes, vals_in != nullptr, n, num_segments), shape) ||
             ctx.tuning.lookup(segsort_cta_threads_tuning_key(), shape))
             o.cta_threads = shape.variant;
-    }
-    if (o.persistent < 0) {
-        launch_shape shape;
-        o.persistent = ctx.tuning.lookup(segsort_batch_tuning_key(key_bytes, vals_in != nullptr, n, num_segments), shape)
-                           ? shape.variant
-                           : 0;
     }
     if (key_bytes == 4) {
         const auto xf = dev::make_xform<uint32_t>(key_kind, descending);

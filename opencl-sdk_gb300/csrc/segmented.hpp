@@ -23,12 +23,6 @@ struct seg_options {
     // batch of 200,000 lognormal segments of u64 pairs takes 12.1 ms with its
     // scan, 27.0 with the one-CTA sorts of every digit and the route off)
     int msd_cap = -1;
-    // 0: a launch per phase, the small/medium and large paths on two
-    // streams; 1: the whole batch in one persistent (cooperative) launch with
-    // grid barriers between its phases; 2..7: the same with (persistent - 1)
-    // eighths of its CTAs sorting the small and medium segments while the
-    // others take the large ones; -1: the tuning table's entry, else 0
-    int persistent = -1;
     // threads of the one-CTA sorts of up to 4,096 keys: 256 (16 keys per
     // thread) or 512 (8). 0: the tuning table's entry for this workload (the
     // segmented key with ":threads", stored by the autotuner), else its
@@ -60,7 +54,8 @@ void segmented_scan(device_context& ctx, const void* in, void* out, std::size_t 
                     const void* identity, bool exclusive, const uint32_t* offsets, std::size_t num_segments);
 
 std::string segsort_tuning_key(int key_bytes, bool has_values, std::size_t n, std::size_t num_segments);
-//! The tuning-table key of the batch's launch form (seg_options::persistent).
+//! The tuning-table key of the batch's launch form. There is one form, the launch
+//! sequence; entries that older tables hold for others change nothing.
 std::string segsort_batch_tuning_key(int key_bytes, bool has_values, std::size_t n, std::size_t num_segments);
 //! The tuning-table key of the one-CTA sorts' thread count (256 or 512; one
 //! entry for every segmented sort of the context).

@@ -1369,7 +1369,6 @@ template <typename K, bool HAS_V> static void run_partial(device_context& ctx, c
     if (segmented) {
         seg_options so;
         so.skip = skip;
-        so.persistent = 0;
         so.cta_threads = 256;
         so.msd_cap = (int)segsort_cta_cap(sizeof(K), HAS_V);
         so.alt_keys = a.alt_keys;
