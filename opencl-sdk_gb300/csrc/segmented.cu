@@ -86,6 +86,7 @@ struct SegControl {
     uint32_t n_warp, n_cta[CTA_CLASSES], n_large;  // list lengths
     uint32_t large_tiles;                          // tiles of all large segments
     uint32_t lsd_tiles;                            // tiles of those not on the MSD route
+    uint32_t rest_tiles;                           // tiles of those counted a second time
     uint32_t warp_next, cta_next[CTA_CLASSES];     // work queue heads
     uint32_t tile_ctr[8];
     uint32_t msd_tile_ctr;
@@ -113,6 +114,13 @@ template <typename K> struct SegArgs {
     uint32_t* tile_seg;     // large tile -> index into large_list
     uint32_t* lsd_begin;    // the same for the segments that take the LSD passes
     uint32_t* lsd_seg;      // (tile_begin and tile_seg themselves without the MSD route)
+    // Counting in two steps (null: all digits at once): the one digit position
+    // counted first (or ALL_DIGITS), the bits that differ inside the segment, and
+    // the tile sequence of the segments whose other digits are counted after all
+    uint8_t* guess;
+    unsigned long long* vary;
+    uint32_t* rest_begin;
+    uint32_t* rest_seg;
     uint32_t* seg_hist;     // [large][PASSES][256]: bin start (absolute) per pass
     uint32_t max_large;
     uint32_t max_tiles;
@@ -138,7 +146,9 @@ template <typename K> __device__ __forceinline__ uint2* sub_entry(const SegArgs<
     return cls == -1 || cls == 1 ? base + i : base + (a.max_sub - 1 - i);
 }
 
-constexpr uint8_t NO_ROUTE = 0xFF;
+constexpr uint8_t NO_ROUTE = 0xFF, REST = 0xFE;  // REST: known after the second count
+constexpr uint8_t ALL_DIGITS = 0xFF;
+enum : int { COUNT_ALL, COUNT_FIRST, COUNT_REST };  // steps of counting and routing
 
 // ---------------------------------------------------------------------------
 // Classification
@@ -202,7 +212,59 @@ template <typename K, int TILE> __device__ __forceinline__ void seg_large_plan(c
     for (std::size_t i = (std::size_t)blockIdx.x * blockDim.x + threadIdx.x; i < words; i += stride) a.seg_hist[i] = 0;
 }
 
-template <typename K, int TILE> __global__ void k_seg_large_plan(SegArgs<K> a) { seg_large_plan<K, TILE>(a, gridDim.x); }
+// The digit position that a large segment's MSD pass will probably use: the
+// highest one that varies among 512 of its keys (16 rows of 32 neighbours),
+// unless its largest bin is then surely too large for that route. A wrong
+// guess costs a second count, nothing else.
+template <typename K> __device__ __forceinline__ void seg_guess(const SegArgs<K>& a)
+{
+    constexpr int ROWS = 16, WARPS = 8;
+    __shared__ uint32_t s_count[WARPS][RADIX];
+    const uint32_t nl = min(a.ctl->n_large, a.max_large);
+    const int lane = threadIdx.x & 31;
+    uint32_t* count = s_count[threadIdx.x >> 5];
+    for (uint32_t j = blockIdx.x * WARPS + (threadIdx.x >> 5); j < nl; j += gridDim.x * WARPS) {
+        const uint32_t s = a.large_list[j];
+        const uint32_t b = a.off[s], len = a.off[s + 1] - b;
+        K k[ROWS];
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) k[r] = a.in_k[b + min(len / ROWS * r + lane, len - 1)];
+        unsigned long long v = 0;
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            k[r] = a.xf(k[r]);
+            v |= k[r] ^ k[0];
+        }
+        v |= k[0] ^ __shfl_sync(FULL_MASK, k[0], 0);
+        v = (unsigned long long)__reduce_or_sync(FULL_MASK, (uint32_t)(v >> 32)) << 32 |
+            __reduce_or_sync(FULL_MASK, (uint32_t)v);
+        int top = v == 0 ? -1 : (63 - __clzll((long long)v)) / 8;
+        if (top >= 0) {
+            for (int d = lane; d < RADIX; d += 32) count[d] = 0;
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) atomicAdd(&count[(uint32_t)(k[r] >> (8 * top)) & 0xFFu], 1u);
+            __syncwarp();
+            uint32_t m = 0;
+            for (int d = lane; d < RADIX; d += 32) m = max(m, count[d]);
+            m = __reduce_max_sync(FULL_MASK, m);
+            // three deviations below the estimate
+            const float least = ((float)m - 3.0f * sqrtf((float)m)) * (1.0f / (32 * ROWS)) * (float)len;
+            if (least > (float)a.sub_cap) top = -1;
+            __syncwarp();
+        }
+        if (lane == 0) {
+            a.guess[j] = top < 0 ? ALL_DIGITS : (uint8_t)top;
+            a.vary[j] = 0;
+        }
+    }
+}
+
+template <typename K, int TILE> __global__ void __launch_bounds__(256) k_seg_large_plan(SegArgs<K> a)
+{
+    seg_large_plan<K, TILE>(a, gridDim.x);
+    if (a.guess != nullptr) seg_guess<K>(a);
+}
 
 // ---------------------------------------------------------------------------
 // Shared-memory LSD sort of one segment by a warp. Stable: items are ranked in
@@ -415,21 +477,39 @@ __global__ void __launch_bounds__(THREADS, MINB) k_seg_tile(SegArgs<K> a, int cl
 // spread over many CTAs): count runs of HIST_TILES tiles in shared memory and
 // add the counts to the segment's row whenever the segment changes or the run
 // ends; turn every row into absolute bin starts.
+//
+// Shared-memory additions bound the count, one per key and digit. The MSD
+// route needs one digit, so batches of more than TWO_STEP_KEYS count in two steps:
+// COUNT_FIRST the digit that a sample points to and which bits differ at all
+// (which tells whether the guess was right), COUNT_REST every digit of the
+// segments that cannot take the route with it.
 // ---------------------------------------------------------------------------
 constexpr uint32_t HIST_TILES = 8;
 
-template <typename K, int TILE> __device__ __forceinline__ void seg_large_count(const SegArgs<K>& a, uint32_t ctas)
+template <typename K, int TILE, int STEP>
+__device__ __forceinline__ void seg_large_count(const SegArgs<K>& a, uint32_t ctas)
 {
     constexpr int P = Traits<K>::PASSES;
     constexpr int BATCH = 8;  // keys in flight per thread
     __shared__ uint32_t sh[2][P * RADIX];  // two copies (warp parity)
     uint32_t* my = sh[(threadIdx.x >> 5) & 1];
-    const uint32_t total = min(a.ctl->large_tiles, a.max_tiles);
+    const uint32_t total = min(STEP == COUNT_REST ? a.ctl->rest_tiles : a.ctl->large_tiles, a.max_tiles);
+    const uint32_t* tile_seg = STEP == COUNT_REST ? a.rest_seg : a.tile_seg;
+    const uint32_t* tile_begin = STEP == COUNT_REST ? a.rest_begin : a.tile_begin;
     const uint32_t runs = (total + HIST_TILES - 1) / HIST_TILES;
+    unsigned long long vary = 0;
     auto flush = [&](uint32_t j) {  // adds the counts to row j and clears them
         __syncthreads();
         uint32_t* row = a.seg_hist + (std::size_t)j * P * RADIX;
-        for (int i = threadIdx.x; i < P * RADIX; i += 256) {
+        const uint32_t g = STEP == COUNT_FIRST ? a.guess[j] : ALL_DIGITS;
+        if (g != ALL_DIGITS) {
+            const uint32_t hi = sizeof(K) == 8 ? __reduce_or_sync(FULL_MASK, (uint32_t)(vary >> 32)) : 0u;
+            const uint32_t lo = __reduce_or_sync(FULL_MASK, (uint32_t)vary);
+            if ((threadIdx.x & 31) == 0 && (hi | lo) != 0) atomicOr(&a.vary[j], (unsigned long long)hi << 32 | lo);
+            vary = 0;
+        }
+        const int first = g == ALL_DIGITS ? 0 : (int)g * RADIX, end = g == ALL_DIGITS ? P * RADIX : first + RADIX;
+        for (int i = first + threadIdx.x; i < end; i += 256) {
             const uint32_t v = sh[0][i] + sh[1][i];
             if (v != 0) atomicAdd(&row[i], v);
             sh[0][i] = 0;
@@ -441,16 +521,18 @@ template <typename K, int TILE> __device__ __forceinline__ void seg_large_count(
     __syncthreads();
     for (uint32_t r = blockIdx.x; r < runs; r += ctas) {
         const uint32_t t0 = r * HIST_TILES, t1 = min(total, t0 + HIST_TILES);
-        uint32_t j = a.tile_seg[t0];
+        uint32_t j = tile_seg[t0];
         for (uint32_t t = t0; t < t1; ++t) {
-            const uint32_t jt = a.tile_seg[t];  // the same for every thread
+            const uint32_t jt = tile_seg[t];  // the same for every thread
             if (jt != j) {
                 flush(j);
                 j = jt;
             }
             const uint32_t s = a.large_list[jt];
-            const uint32_t b = a.off[s] + (t - a.tile_begin[jt]) * TILE;
+            const uint32_t b = a.off[s] + (t - tile_begin[jt]) * TILE;
             const uint32_t e = min(a.off[s + 1], b + TILE);
+            const uint32_t g = STEP == COUNT_FIRST ? a.guess[jt] : ALL_DIGITS;
+            const K x0 = g != ALL_DIGITS ? a.xf(a.in_k[a.off[s]]) : K(0);
             for (uint32_t i0 = b; i0 < e; i0 += 256 * BATCH) {
                 K k[BATCH];
 #pragma unroll
@@ -462,6 +544,11 @@ template <typename K, int TILE> __device__ __forceinline__ void seg_large_count(
                 for (int q = 0; q < BATCH; ++q) {
                     if (i0 + q * 256 + threadIdx.x >= e) break;
                     const K x = a.xf(k[q]);
+                    if (STEP == COUNT_FIRST && g != ALL_DIGITS) {
+                        atomicAdd(&my[g * RADIX + ((uint32_t)(x >> ((8 * g) & (8 * P - 1))) & 0xFFu)], 1u);
+                        vary |= x ^ x0;
+                        continue;
+                    }
 #pragma unroll
                     for (int p = 0; p < P; ++p) atomicAdd(&my[p * RADIX + (uint32_t)((x >> (8 * p)) & 0xFF)], 1u);
                 }
@@ -471,9 +558,9 @@ template <typename K, int TILE> __device__ __forceinline__ void seg_large_count(
     }
 }
 
-template <typename K, int TILE> __global__ void __launch_bounds__(256) k_seg_large_count(SegArgs<K> a)
+template <typename K, int TILE, int STEP> __global__ void __launch_bounds__(256) k_seg_large_count(SegArgs<K> a)
 {
-    seg_large_count<K, TILE>(a, gridDim.x);
+    seg_large_count<K, TILE, STEP>(a, gridDim.x);
 }
 
 
@@ -484,7 +571,10 @@ template <typename K, int TILE> __global__ void __launch_bounds__(256) k_seg_lar
 // pass on that digit partitions the segment into its bins (stable), and
 // ranges of neighbouring bins become sub-buckets for the warp and CTA sorts;
 // else the full LSD passes, over tiles appended to their own sequence.
-template <typename K, int TILE> __device__ __forceinline__ void seg_route(const SegArgs<K>& a, bool with_msd, uint32_t ctas)
+// COUNT_FIRST: a segment of which one digit was counted takes the MSD route
+// with it or is put off to COUNT_REST, with its counts cleared.
+template <typename K, int TILE, int STEP>
+__device__ __forceinline__ void seg_route(const SegArgs<K>& a, bool with_msd, uint32_t ctas)
 {
     constexpr int P = Traits<K>::PASSES;
     __shared__ uint32_t s_max[8];
@@ -496,7 +586,9 @@ template <typename K, int TILE> __device__ __forceinline__ void seg_route(const 
     for (uint32_t j = blockIdx.x; j < nl; j += ctas) {
         const uint32_t s = a.large_list[j];
         const uint32_t segb = a.off[s], sege = a.off[s + 1], len = sege - segb;
-        for (int p = 0; p < P; ++p) {
+        if (STEP == COUNT_REST && a.route[j] != REST) continue;
+        const int one = STEP == COUNT_FIRST && a.guess[j] != ALL_DIGITS ? a.guess[j] : -1;  // the only row that is counted
+        for (int p = one < 0 ? 0 : one; p < (one < 0 ? P : one + 1); ++p) {
             uint32_t* row = a.seg_hist + ((std::size_t)j * P + p) * RADIX;
             const uint32_t ex = dev::bins_exclusive_sum(row[threadIdx.x], s_scratch);
             row[threadIdx.x] = segb + ex;
@@ -509,7 +601,11 @@ template <typename K, int TILE> __device__ __forceinline__ void seg_route(const 
         };
         if (threadIdx.x == 0) s_top = -1;
         __syncthreads();
-        for (int p = P - 1; p >= 0; --p) {
+        if (one >= 0) {
+            const unsigned long long v = a.vary[j];
+            if (threadIdx.x == 0) s_top = v == 0 ? -1 : (63 - __clzll((long long)v)) / 8;
+        }
+        for (int p = one < 0 ? P - 1 : -1; p >= 0; --p) {
             // a position varies when no bin holds the whole segment
             const bool whole = bin_size(p, threadIdx.x) == len;
             if (__syncthreads_or(whole) == 0) {
@@ -519,7 +615,7 @@ template <typename K, int TILE> __device__ __forceinline__ void seg_route(const 
         }
         __syncthreads();
         const int top = s_top;
-        uint32_t size = top >= 0 ? bin_size(top, threadIdx.x) : len;
+        uint32_t size = top >= 0 && (one < 0 || top == one) ? bin_size(top, threadIdx.x) : len;
         uint32_t m = size;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(FULL_MASK, m, o));
@@ -529,8 +625,8 @@ template <typename K, int TILE> __device__ __forceinline__ void seg_route(const 
 #pragma unroll
         for (int w = 0; w < 8; ++w) biggest = max(biggest, s_max[w]);
         // room for a window's keys and its last bucket
-        const bool msd = top >= 0 && biggest + SUB_WINDOW <= a.sub_cap;
-        if (threadIdx.x == 0) a.route[j] = msd ? (uint8_t)top : NO_ROUTE;
+        const bool msd = top >= 0 && (one < 0 || top == one) && biggest + SUB_WINDOW <= a.sub_cap;
+        if (threadIdx.x == 0) a.route[j] = msd ? (uint8_t)top : (uint8_t)(one < 0 ? NO_ROUTE : REST);
         if (msd) {
             const uint32_t* row = a.seg_hist + ((size_t)j * P + top) * RADIX;
             const uint32_t d = threadIdx.x;
@@ -548,18 +644,22 @@ template <typename K, int TILE> __device__ __forceinline__ void seg_route(const 
             }
         } else {
             const uint32_t tiles = (len + TILE - 1) / TILE;
-            if (threadIdx.x == 0) a.lsd_begin[j] = s_first = atomicAdd(&a.ctl->lsd_tiles, tiles);
+            const bool rest = one >= 0;
+            if (threadIdx.x == 0)
+                (rest ? a.rest_begin : a.lsd_begin)[j] = s_first =
+                    atomicAdd(rest ? &a.ctl->rest_tiles : &a.ctl->lsd_tiles, tiles);
             __syncthreads();
             for (uint32_t t = threadIdx.x; t < tiles; t += blockDim.x)
-                if (s_first + t < a.max_tiles) a.lsd_seg[s_first + t] = j;
+                if (s_first + t < a.max_tiles) (rest ? a.rest_seg : a.lsd_seg)[s_first + t] = j;
+            if (rest) a.seg_hist[((std::size_t)j * P + max(one, 0)) * RADIX + threadIdx.x] = 0;
         }
         __syncthreads();
     }
 }
 
-template <typename K, int TILE> __global__ void __launch_bounds__(256) k_seg_route(SegArgs<K> a, bool with_msd)
+template <typename K, int TILE, int STEP> __global__ void __launch_bounds__(256) k_seg_route(SegArgs<K> a, bool with_msd)
 {
-    seg_route<K, TILE>(a, with_msd, gridDim.x);
+    seg_route<K, TILE, STEP>(a, with_msd, gridDim.x);
 }
 
 
@@ -582,7 +682,7 @@ __device__ __forceinline__ void seg_large_pass(const SegArgs<K>& a, int slot, bo
     constexpr int WARPS = THREADS / 32;
     constexpr int TILE = THREADS * ITEMS;
     const uint32_t num_tiles = min(MSD || !with_msd ? a.ctl->large_tiles : a.ctl->lsd_tiles, a.max_tiles);
-    if (num_tiles == 0) return;
+    if (num_tiles == 0 || (MSD && a.ctl->lsd_tiles == a.ctl->large_tiles)) return;  // no segment of this kind
     const uint32_t* tile_seg = MSD ? a.tile_seg : a.lsd_seg;
     const uint32_t* tile_begin = MSD ? a.tile_begin : a.lsd_begin;
     uint32_t* tile_ctr = MSD ? &a.ctl->msd_tile_ctr : &a.ctl->tile_ctr[slot];
@@ -818,14 +918,24 @@ __global__ void __launch_bounds__(THREADS, MINB) k_seg_large_pass(SegArgs<K> a, 
 // ---------------------------------------------------------------------------
 // Batches of few keys are bound by the launches and the longest CTA of each,
 // not by the work: up to FEW_KEYS the longer one-CTA classes share a launch,
-// up to VERY_FEW_KEYS all of them, and 32-bit keys keep to the LSD passes
-// (four passes of a tile or two each, about 13 us apiece, against the MSD
-// route's pass, its sub-bucket launches and the LSD launches that find nothing
-// to do: 347 segments of 264,000 floats and their scan take 86 us with the
-// former, 122 with the latter; eight passes of 64-bit keys lose to the route:
-// 181 us against 151 for 1,800 segments).
+// up to VERY_FEW_KEYS all of them.
+//
+// 32-bit keys keep to the LSD passes (four) up to ROUTE_32BIT_KEYS: the MSD
+// route's launches cost a batch that cannot use it about 30 us, and such keys
+// are common (floats of a normal distribution). Segments of 500,000 keys, LSD
+// alone / with the route: 3.4e7 normal floats 793 / 829 us, 6.7e7 1470 / 1496;
+// uniform keys 771 / 708, 1426 / 1263. 64-bit keys, with eight passes to save,
+// take the route at any size (1,800 segments 181 / 151 us; 5e6 keys 477 / 281).
+//
+// The count takes one digit first (see seg_large_count) above TWO_STEP_KEYS:
+// 200,000 lognormal segments of u64 pairs take 11.67 ms for 12.11; 6.7e7 u64
+// keys in segments of 40,000 1741 us for 1854, 1.9e7 592 for 622; at 5e6 the
+// two extra launches cost what it saves. Segments whose highest digit the
+// sample misses are counted twice: 3405 us for 3353.
 constexpr std::size_t FEW_KEYS = std::size_t(1) << 22;
 constexpr std::size_t VERY_FEW_KEYS = std::size_t(1) << 18;
+constexpr std::size_t ROUTE_32BIT_KEYS = std::size_t(1) << 26;
+constexpr std::size_t TWO_STEP_KEYS = std::size_t(1) << 24;
 
 template <typename K, bool HAS_V> struct LargeShape;
 template <bool HV> struct LargeShape<uint32_t, HV> {
@@ -925,6 +1035,8 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
     const uint32_t max_sub = msd ? (uint32_t)(n / SUB_WINDOW) + max_large : 0;
     temp_buffer route(ctx.resource, maybe_large ? max_large : 0);
     temp_buffer sub_lists(ctx.resource, (std::size_t)max_sub * 4 * sizeof(uint32_t));
+    const bool two_steps = msd && n > TWO_STEP_KEYS;
+    temp_buffer rest(ctx.resource, two_steps ? (std::size_t)max_large * 16 + (std::size_t)max_tiles * 4 : 0);
     check_cuda(cudaMemsetAsync(ctl.get(), 0, sizeof(SegControl), ctx.stream), "cudaMemsetAsync");
     if (maybe_large && !msd)
         check_cuda(cudaMemsetAsync(route.get(), NO_ROUTE, max_large, ctx.stream), "cudaMemsetAsync");
@@ -950,6 +1062,10 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
     a.tile_seg = tile_seg.as<uint32_t>();
     a.lsd_begin = msd ? a.tile_begin + max_large : a.tile_begin;
     a.lsd_seg = msd ? a.tile_seg + max_tiles : a.tile_seg;
+    a.vary = two_steps ? rest.as<unsigned long long>() : nullptr;
+    a.rest_begin = two_steps ? reinterpret_cast<uint32_t*>(a.vary + max_large) : nullptr;
+    a.rest_seg = two_steps ? a.rest_begin + max_large : nullptr;
+    a.guess = two_steps ? reinterpret_cast<uint8_t*>(a.rest_seg + max_tiles) : nullptr;
     a.seg_hist = seg_hist.as<uint32_t>();
     a.max_large = max_large;
     a.max_tiles = max_tiles;
@@ -995,9 +1111,20 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
             kernel_timer kt(ctx, "segsort.large_histogram", aux);
             const int tgrid = (int)std::min<std::size_t>(max_tiles, (std::size_t)ctx.sm_count * 4);
             k_seg_large_plan<K, TILE><<<tgrid, 256, 0, aux>>>(a);
-            auto hk = &k_seg_large_count<K, TILE>;
-            hk<<<std::min<int>(tgrid, ctx.sm_count * std::max(1, occupancy(hk, 256, 0))), 256, 0, aux>>>(a);
-            k_seg_route<K, TILE><<<(int)std::min<std::size_t>(max_large, (std::size_t)ctx.sm_count * 8), 256, 0, aux>>>(a, msd);
+            auto count = [&](auto hk) {
+                hk<<<(int)std::min<std::size_t>(max_tiles, (std::size_t)ctx.sm_count * std::max(1, occupancy(hk, 256, 0))), 256, 0,
+                     aux>>>(a);
+            };
+            const int rgrid = (int)std::min<std::size_t>(max_large, (std::size_t)ctx.sm_count * 8);
+            if (two_steps) {
+                count(&k_seg_large_count<K, TILE, COUNT_FIRST>);
+                k_seg_route<K, TILE, COUNT_FIRST><<<rgrid, 256, 0, aux>>>(a, true);
+                count(&k_seg_large_count<K, TILE, COUNT_REST>);
+                k_seg_route<K, TILE, COUNT_REST><<<rgrid, 256, 0, aux>>>(a, true);
+            } else {
+                count(&k_seg_large_count<K, TILE, COUNT_ALL>);
+                k_seg_route<K, TILE, COUNT_ALL><<<rgrid, 256, 0, aux>>>(a, msd);
+            }
             check_cuda(cudaGetLastError(), "segmented sort histogram launch");
         }
         const std::size_t psmem = large_pass_smem;
@@ -1088,7 +1215,7 @@ void segmented_sort(device_context& ctx, const void* keys_in, void* keys_out, in
         launch_shape shape;
         o.msd_cap = ctx.tuning.lookup(segsort_msd_tuning_key(key_bytes, vals_in != nullptr, n, num_segments), shape)
                         ? shape.variant
-                    : key_bytes == 4 && n <= seg::FEW_KEYS ? 0
+                    : key_bytes == 4 && n <= seg::ROUTE_32BIT_KEYS ? 0
                                                            : (int)segsort_cta_cap(key_bytes, vals_in != nullptr);
     }
     if (o.cta_threads == 0) {
