@@ -192,10 +192,13 @@ template <typename T> struct Shared {
 __device__ __forceinline__ uint32_t limit(const Tiles& a) { return a.num_tiles + STAGES; }
 
 // The copying warp: whole tiles of TILE_BYTES from `in` (16-byte aligned); a
-// last partial tile is announced without a copy.
-template <typename T>
-__device__ void copy_role(const Tiles& a, Shared<T>& sh, unsigned char* stages, const void* in, uint64_t bytes)
+// last partial tile is announced without a copy. SIDE: bytes per tile of a
+// second array, copied along into side_stages.
+template <uint32_t SIDE = 0, typename T>
+__device__ void copy_role(const Tiles& a, Shared<T>& sh, unsigned char* stages, const void* in, uint64_t bytes,
+                          unsigned char* side_stages = nullptr, const void* side = nullptr)
 {
+    static_assert(SIDE % 16 == 0, "bulk copies");
     if ((threadIdx.x & 31) != 0) return;
     for (uint32_t k = 0; k < limit(a); ++k) {
         const int s = k % STAGES;
@@ -208,9 +211,12 @@ __device__ void copy_role(const Tiles& a, Shared<T>& sh, unsigned char* stages, 
         }
         sh.tile[s] = t;
         if ((uint64_t)(t + 1) * TILE_BYTES <= bytes) {
-            dev::mbar_arrive_expect_tx(&sh.full[s], TILE_BYTES);
+            dev::mbar_arrive_expect_tx(&sh.full[s], TILE_BYTES + SIDE);
             dev::bulk_g2s(stages + (std::size_t)s * TILE_BYTES, static_cast<const unsigned char*>(in) + (std::size_t)t * TILE_BYTES,
                           TILE_BYTES, &sh.full[s]);
+            if (SIDE > 0)
+                dev::bulk_g2s(side_stages + (std::size_t)s * SIDE, static_cast<const unsigned char*>(side) + (std::size_t)t * SIDE,
+                              SIDE, &sh.full[s]);
         } else {
             mbar_arrive(&sh.full[s]);
         }

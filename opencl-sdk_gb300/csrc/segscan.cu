@@ -14,9 +14,11 @@
 // segment starting in the tile, then the tile's starts are set in a shared
 // bitmask.
 #include <cstring>
+#include <memory>
 
 #include "device_common.cuh"
 #include "ops.cuh"
+#include "pipe.cuh"
 #include "runtime.hpp"
 #include "segmented.hpp"
 #include "sort_internal.hpp"
@@ -327,6 +329,195 @@ __global__ void __launch_bounds__(THREADS) k_segscan(SegScanArgs<T> a)
     }
 }
 
+// ---------------------------------------------------------------------------
+// Large inputs of 4-byte elements: the same scan as a pipeline inside each CTA
+// (pipe.cuh), with a tile's (head, value) pair as its aggregate. The look-back
+// form above is bound by the chain of publish and look-back from tile to tile
+// (int32 over 200,000 lognormal segments, 3.8e8 elements: 1186 us, this one 649
+// with its head bits).
+//
+// Head flags come as one bit per element, set in memory beforehand and copied
+// with the tile: finding a tile's segments inside the kernel would cost a
+// search (four dependent loads at least) per tile.
+// ---------------------------------------------------------------------------
+template <typename T> struct HeadValue {
+    uint32_t head;  // a segment starts among the elements
+    T v;            // their combination from the last start on
+};
+template <typename T, typename Op> struct HeadOp {
+    Op op;
+    __device__ HeadValue<T> operator()(const HeadValue<T>& a, const HeadValue<T>& b) const
+    {
+        return {a.head | b.head, b.head ? b.v : op(a.v, b.v)};
+    }
+};
+
+// Sets the bit of every segment start below n, and of position 0. Neighbouring
+// starts share a word: one atomic per word and warp.
+__global__ void __launch_bounds__(256) k_heads(const uint32_t* off, uint32_t nseg, uint32_t n, uint32_t* heads)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&heads[0], 1u);
+    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < nseg; i0 += stride) {
+        const uint64_t i = i0 + lane;
+        const uint32_t o = i < nseg ? off[i] : 0xFFFFFFFFu;
+        const uint32_t word = o < n ? o >> 5 : 0xFFFFFFFFu;
+        const uint32_t peers = __match_any_sync(FULL_MASK, word);
+        const uint32_t bits = __reduce_or_sync(peers, 1u << (o & 31));
+        if (o < n && lane == (uint32_t)__ffs(peers) - 1) atomicOr(&heads[word], bits);
+    }
+}
+
+template <typename T> struct SegPipeArgs {
+    const T* in;
+    T* out;
+    const uint32_t* heads;
+    uint32_t n;
+    T identity;
+    int exclusive;
+    pipe::Tiles tiles;
+};
+
+constexpr uint32_t HEAD_TILE_BYTES = pipe::TILE_BYTES / 4 / 8;
+constexpr std::size_t SEG_PIPE_SMEM = pipe::SMEM + pipe::STAGES * HEAD_TILE_BYTES;
+
+template <typename T, typename Op>
+__global__ void __launch_bounds__(pipe::THREADS, 1) k_segscan_pipe(SegPipeArgs<T> a)
+{
+    using namespace pipe;
+    static_assert(sizeof(T) == 4, "four elements per lane and row");
+    constexpr int VEC = 4;
+    constexpr uint32_t TILE = TILE_BYTES / 4;
+    using Pair = HeadValue<T>;
+    extern __shared__ __align__(128) unsigned char smem[];
+    unsigned char* head_stages = smem + pipe::SMEM;
+    __shared__ Shared<Pair> sh;
+    __shared__ Pair s_before[STAGES][WRITERS];
+    const Tiles& tiles = a.tiles;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const Op op;
+    const HeadOp<T, Op> pair_op{};
+    sh.init();
+    if (warp == COPY_WARP)
+        return copy_role<HEAD_TILE_BYTES>(tiles, sh, smem, a.in, (uint64_t)a.n * 4, head_stages, a.heads);
+    // position 0 is a start, so nothing of `first` reaches an output
+    if (warp == PREFIX_WARP) return prefix_role<false>(tiles, sh, Pair{0u, a.identity}, pair_op);
+
+    // This lane's elements of a row of the tile and their head bits.
+    auto load_row = [&](uint32_t t, int s, bool whole, int row, T (&x)[VEC]) -> uint32_t {
+        const uint32_t word = row * 4 + lane / 8;
+        uint32_t h;
+        if (whole) {
+            const uint4 v = reinterpret_cast<const uint4*>(smem + (std::size_t)s * TILE_BYTES)[row * 32 + lane];
+            memcpy(x, &v, 16);
+            h = reinterpret_cast<const uint32_t*>(head_stages + s * HEAD_TILE_BYTES)[word];
+        } else {
+#pragma unroll
+            for (int j = 0; j < VEC; ++j) {
+                const uint64_t at = (uint64_t)t * TILE + (row * 32 + lane) * VEC + j;
+                x[j] = at < a.n ? a.in[at] : a.identity;
+            }
+            h = a.heads[(std::size_t)t * (TILE / 32) + word];
+        }
+        return (h >> (lane * 4 & 31)) & 15u;
+    };
+    // The lane's combination from its last head (or its first element) on,
+    // then the same from the row's start to the lane; returns the lanes with
+    // heads. A lane combines with lanes back to the last one with a head only.
+    auto scan_row = [&](const T (&x)[VEC], uint32_t h, T& v) -> uint32_t {
+        v = x[0];
+#pragma unroll
+        for (int j = 1; j < VEC; ++j) v = (h >> j & 1u) ? x[j] : op(v, x[j]);
+        const uint32_t lanes = __ballot_sync(FULL_MASK, h != 0);
+        const uint32_t mine = lanes & (0xFFFFFFFFu >> (31 - lane));
+        const int from = mine != 0 ? 31 - __clz((int)mine) : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const T y = __shfl_up_sync(FULL_MASK, v, o);
+            if (lane - o >= from) v = op(y, v);
+        }
+        return lanes;
+    };
+
+    if (warp >= WRITERS) {  // folding
+        const int f = warp - WRITERS;
+        for (uint32_t k = 0; k < limit(tiles); ++k) {
+            const uint32_t t = sh.next(k, tiles.err);
+            if (t == END) break;
+            const bool whole = (uint64_t)(t + 1) * TILE <= a.n;
+#pragma unroll
+            for (int b = 0; b < BLOCKS; ++b) {
+                Pair total{0u, a.identity};
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r) {
+                    T x[VEC], v;
+                    const uint32_t h = load_row(t, k % STAGES, whole, (f * BLOCKS + b) * ROWS + r, x);
+                    const uint32_t lanes = scan_row(x, h, v);
+                    const Pair row{lanes != 0 ? 1u : 0u, v};
+                    total = r == 0 ? row : pair_op(total, row);  // lane 31's
+                }
+                if (lane == 31) sh.total[k & 1][f * BLOCKS + b] = total;
+            }
+            publish_tile(tiles, sh, k, t, s_before[k % STAGES], pair_op);
+        }
+        return;
+    }
+
+    for (uint32_t k = 0; k < limit(tiles); ++k) {  // scanning and writing
+        const int s = k % STAGES;
+        const uint32_t t = sh.next(k, tiles.err);
+        if (t == END) return;
+        const bool whole = (uint64_t)(t + 1) * TILE <= a.n;
+        T x[ROWS][VEC], incl[ROWS];
+        uint32_t h[ROWS], lanes[ROWS];
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) h[r] = load_row(t, s, whole, warp * ROWS + r, x[r]);
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) lanes[r] = scan_row(x[r], h[r], incl[r]);
+        sh.wait(&sh.ready[s], k, tiles.err);
+        T before = const_cast<const volatile Pair&>(sh.prefix[s]).v;  // since the last start before the block, then each row
+        if (warp > 0) {
+            const Pair p = s_before[s][warp];
+            before = p.head ? p.v : op(before, p.v);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh.empty[s]);  // the warp is done with the stage and its slots
+        if (sh.abort) continue;
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            const T left = __shfl_up_sync(FULL_MASK, incl[r], 1);
+            T run = before;
+            if (lane > 0) run = (lanes[r] & dev::lanemask_lt()) != 0 ? left : op(before, left);
+            const T last = __shfl_sync(FULL_MASK, incl[r], 31);
+            before = lanes[r] != 0 ? last : op(before, last);
+            T o[VEC];
+#pragma unroll
+            for (int j = 0; j < VEC; ++j) {
+                const bool head = (h[r] >> j & 1u) != 0;
+                const T inc = head ? x[r][j] : op(run, x[r][j]);
+                o[j] = a.exclusive ? (head ? a.identity : run) : inc;
+                run = inc;
+            }
+            const uint32_t at = t * TILE + ((warp * ROWS + r) * 32 + lane) * VEC;
+            if (whole) {
+                uint4 w;
+                memcpy(&w, o, 16);
+                *reinterpret_cast<uint4*>(a.out + at) = w;
+            } else {
+#pragma unroll
+                for (int j = 0; j < VEC; ++j)
+                    if (at + j < a.n) a.out[at + j] = o[j];
+            }
+        }
+    }
+}
+
+// From here the pipeline wins for every segment length (int32, look-back /
+// pipeline in us, segments of 20, 1000 and 100,000 elements): 2^26 elements 324 /
+// 184, 229 / 137, 180 / 138; 2^24 74 / 66, 62 / 55, 51 / 55; 2^23 39 / 42, 34 / 38, 28 / 37.
+constexpr std::size_t PIPE_MIN = std::size_t(1) << 25;
+
 struct SegScanLaunch {
     device_context& ctx;
     const void* in;
@@ -338,6 +529,57 @@ struct SegScanLaunch {
     std::size_t nseg;
 
     template <typename T, typename Op> void run()
+    {
+        if constexpr (sizeof(T) == 4) {
+            if (n >= PIPE_MIN && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0 &&
+                ctx.smem_optin >= SEG_PIPE_SMEM + 8192 && run_pipe<T, Op>())
+                return;
+        }
+        run_lookback<T, Op>();
+    }
+
+    // False when there is no memory for the head bits (or, under capture, none
+    // in the pool): the look-back form needs none.
+    template <typename T, typename Op> bool run_pipe()
+    {
+        constexpr uint32_t TILE = pipe::TILE_BYTES / sizeof(T);
+        SegPipeArgs<T> a;
+        a.tiles.num_tiles = (uint32_t)((n + TILE - 1) / TILE);
+        const std::size_t head_bytes = (std::size_t)a.tiles.num_tiles * HEAD_TILE_BYTES;
+        std::unique_ptr<temp_buffer> heads;
+        try {
+            heads = std::make_unique<temp_buffer>(ctx.resource, head_bytes);
+        } catch (const out_of_memory&) {
+            return false;
+        } catch (const unsupported_error&) {
+            return false;
+        }
+        check_cuda(cudaMemsetAsync(heads->get(), 0, head_bytes, ctx.stream), "cudaMemsetAsync");
+        kernel_timer kt(ctx, "segscan.pipe");
+        const int hgrid = (int)std::max<std::size_t>(1, std::min<std::size_t>((nseg + 255) / 256, (std::size_t)ctx.sm_count * 8));
+        k_heads<<<hgrid, 256, 0, ctx.stream>>>(off, (uint32_t)nseg, (uint32_t)n, heads->as<uint32_t>());
+        a.in = static_cast<const T*>(in);
+        a.out = static_cast<T*>(out);
+        a.heads = heads->as<uint32_t>();
+        a.n = (uint32_t)n;
+        std::memcpy(&a.identity, identity, sizeof(T));
+        a.exclusive = exclusive ? 1 : 0;
+        a.tiles.ring = ctx.lookback_ring;
+        a.tiles.seq0 = ctx.reserve_seq(a.tiles.num_tiles);
+        a.tiles.err = ctx.d_error;
+        unsigned char* ctl = ctx.d_small + 256;
+        check_cuda(cudaMemsetAsync(ctl, 0, 64, ctx.stream), "cudaMemsetAsync");
+        a.tiles.counter = reinterpret_cast<uint32_t*>(ctl);
+        auto kernel = &k_segscan_pipe<T, Op>;
+        check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SEG_PIPE_SMEM),
+                   "cudaFuncSetAttribute");
+        const int grid = (int)std::min<std::size_t>(a.tiles.num_tiles, (std::size_t)ctx.sm_count);
+        kernel<<<grid, pipe::THREADS, SEG_PIPE_SMEM, ctx.stream>>>(a);
+        check_cuda(cudaGetLastError(), "segmented scan launch");
+        return true;
+    }
+
+    template <typename T, typename Op> void run_lookback()
     {
         constexpr int VEC = 16 / sizeof(T);
         constexpr int ROWS = sizeof(T) == 4 ? 4 : 8;
