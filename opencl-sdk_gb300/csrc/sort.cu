@@ -25,6 +25,7 @@
 // fixed and graph-capturable).
 #include <algorithm>
 #include <cstring>
+#include <memory>
 #include <string>
 
 #include "device_common.cuh"
@@ -1173,7 +1174,21 @@ static std::mutex g_occupancy_mutex;
 template <typename K, bool HAS_V>
 static void run_passes(device_context& ctx, SortArgs<K> a, const PassVariant<K>& pv, int passes, bool copy);
 template <typename K, bool HAS_V>
-static void run_partial(device_context& ctx, const SortArgs<K>& a, const PassVariant<K>& pv);
+static bool run_partial(device_context& ctx, const SortArgs<K>& a, const PassVariant<K>& pv);
+
+// K1: the digit counts and the plan of the passes.
+template <typename K> static void run_upfront(device_context& ctx, const SortArgs<K>& a)
+{
+    constexpr int P = Traits<K>::PASSES;
+    constexpr int HT = 256, NSUB = 2;
+    const std::size_t hsmem = (std::size_t)NSUB * P * RADIX * 4;
+    const int hblocks = prepare_kernel(k_upfront<K, HT, NSUB>, HT, hsmem, g_occupancy, g_occupancy_mutex);
+    const std::size_t hwork = ((std::size_t)a.n + HT * 16 - 1) / (HT * 16);
+    const int hgrid = (int)std::max<std::size_t>(1, std::min<std::size_t>(hwork, (std::size_t)ctx.sm_count * hblocks));
+    kernel_timer kt(ctx, "sort.upfront_histogram");
+    k_upfront<K, HT, NSUB><<<hgrid, HT, hsmem, ctx.stream>>>(a);
+    check_cuda(cudaGetLastError(), "radix sort histogram launch");
+}
 
 template <typename K, bool HAS_V>
 static void run_sort(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v,
@@ -1220,24 +1235,11 @@ static void run_sort(device_context& ctx, const K* in_k, K* out_k, const uint32_
     a.chunks = 0;
     a.tiles_per_chunk = 0;
 
-    // K1
-    constexpr int HT = 256, NSUB = 2;
-    const std::size_t hsmem = (std::size_t)NSUB * P * RADIX * 4;
-    const int hblocks = prepare_kernel(k_upfront<K, HT, NSUB>, HT, hsmem, g_occupancy, g_occupancy_mutex);
-    const std::size_t hwork = (n + HT * 16 - 1) / (HT * 16);
-    const int hgrid = (int)std::max<std::size_t>(1, std::min<std::size_t>(hwork, (std::size_t)ctx.sm_count * hblocks));
-    {
-        kernel_timer kt(ctx, "sort.upfront_histogram");
-        k_upfront<K, HT, NSUB><<<hgrid, HT, hsmem, ctx.stream>>>(a);
-        check_cuda(cudaGetLastError(), "radix sort histogram launch");
-    }
+    run_upfront<K>(ctx, a);
 
     // The leading digits only, where that is enough (sort_partial.cuh).
     if constexpr (sizeof(K) == 8) {
-        if (n >= partial::MIN_KEYS) {
-            run_partial<K, HAS_V>(ctx, a, pv);
-            return;
-        }
+        if (n >= partial::MIN_KEYS && run_partial<K, HAS_V>(ctx, a, pv)) return;
     }
     run_passes<K, HAS_V>(ctx, a, pv, P, true);
 }
@@ -1305,7 +1307,8 @@ static void run_passes(device_context& ctx, SortArgs<K> a, const PassVariant<K>&
 
 // After the upfront histogram: the fewest leading digits that leave little out
 // of order, their passes, and the repair of what they leave.
-template <typename K, bool HAS_V> static void run_partial(device_context& ctx, const SortArgs<K>& a, const PassVariant<K>& pv)
+// False, with nothing enqueued, when there is no memory for its tables.
+template <typename K, bool HAS_V> static bool run_partial(device_context& ctx, const SortArgs<K>& a, const PassVariant<K>& pv)
 {
     using namespace partial;
     constexpr uint32_t SEGMENTS = 2 * MAX_LONG - 1;
@@ -1319,9 +1322,15 @@ template <typename K, bool HAS_V> static void run_partial(device_context& ctx, c
     const uint32_t sample = sample_size(n);
     const std::size_t ones = (std::size_t)CANDIDATES * 2 * sample * 8 + LONG_SET * 4;
     const std::size_t max_faults = (n + FT_TILE - 1) / FT_TILE + 1;
-    temp_buffer head(ctx.resource, zeroed);
-    temp_buffer sets(ctx.resource, ones);
-    temp_buffer lists(ctx.resource, (4 * (std::size_t)MAX_LONG + max_faults) * sizeof(uint32_t) + SEGMENTS);
+    std::unique_ptr<temp_buffer> head_b, sets_b, lists_b;
+    try {
+        head_b = std::make_unique<temp_buffer>(ctx.resource, zeroed);
+        sets_b = std::make_unique<temp_buffer>(ctx.resource, ones);
+        lists_b = std::make_unique<temp_buffer>(ctx.resource, (4 * (std::size_t)MAX_LONG + max_faults) * sizeof(uint32_t) + SEGMENTS);
+    } catch (const out_of_memory&) {
+        return false;
+    }
+    temp_buffer &head = *head_b, &sets = *sets_b, &lists = *lists_b;
     check_cuda(cudaMemsetAsync(head.get(), 0, zeroed, ctx.stream), "cudaMemsetAsync");
     check_cuda(cudaMemsetAsync(sets.get(), 0xFF, ones, ctx.stream), "cudaMemsetAsync");
     Args<K> p;
@@ -1366,6 +1375,13 @@ template <typename K, bool HAS_V> static void run_partial(device_context& ctx, c
         }
         check_cuda(cudaGetLastError(), "radix sort repair launch");
     }
+    // The second plan, from the order reached: nothing to do in the usual case.
+    SortArgs<K> all = a;
+    all.in_keys = a.out_keys;
+    all.in_vals = a.out_vals;
+    all.in_place = 1;
+    all.ctl = p.all;
+    bool copy = false;  // that plan has all passes, an even number, or none
     if (segmented) {
         seg_options so;
         so.skip = skip;
@@ -1373,16 +1389,18 @@ template <typename K, bool HAS_V> static void run_partial(device_context& ctx, c
         so.msd_cap = (int)segsort_cta_cap(sizeof(K), HAS_V);
         so.alt_keys = a.alt_keys;
         so.alt_vals = a.alt_vals;
-        segmented_sort_xf(ctx, a.out_keys, a.out_vals, a.xf.a, a.xf.b, n, p.off, SEGMENTS, so);
+        try {
+            segmented_sort_xf(ctx, a.out_keys, a.out_vals, a.xf.a, a.xf.b, n, p.off, SEGMENTS, so);
+        } catch (const out_of_memory&) {
+            // it takes its memory before it enqueues anything: every digit, then
+            check_cuda(cudaMemsetAsync(p.all, 0, sizeof(SortControl), ctx.stream), "cudaMemsetAsync");
+            run_upfront<K>(ctx, all);
+            copy = true;
+        }
     }
-    // The second plan, from the order reached: nothing to do in the usual case.
-    SortArgs<K> all = a;
-    all.in_keys = a.out_keys;
-    all.in_vals = a.out_vals;
-    all.in_place = 1;
-    all.ctl = p.all;
     all.seq0 = ctx.reserve_seq((uint64_t)Traits<K>::PASSES * a.num_tiles);
-    run_passes<K, HAS_V>(ctx, all, pv, Traits<K>::PASSES, false);
+    run_passes<K, HAS_V>(ctx, all, pv, Traits<K>::PASSES, copy);
+    return true;
 }
 
 }  // namespace onesweep
