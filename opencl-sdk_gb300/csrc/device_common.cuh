@@ -225,6 +225,15 @@ __device__ __forceinline__ T warp_reduce(T x, Op op)
     return __shfl_sync(FULL_MASK, x, 0);
 }
 
+// First statement of a kernel that is launched by launch_chained: waits until the
+// kernels before have finished and their writes are visible. Launched
+// otherwise it does nothing. (Asking for the next launch as early as here put
+// its waiting CTAs beside this kernel's: 2^28 pairs 6.09 ms for 6.04.)
+__device__ __forceinline__ void chain()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Exclusive sum of one value per thread over the first 256 threads of the CTA
 // (the 256 radix bins). Every thread of the CTA must call it; threads >= 256
 // contribute nothing. `scratch` holds 8 words.
@@ -249,4 +258,26 @@ __device__ __forceinline__ uint32_t bins_exclusive_sum(uint32_t v, uint32_t* scr
 }
 
 }  // namespace dev
+
+// Launches a kernel that begins with dev::chain() and follows another kernel in
+// the stream: its launch overlaps the end of that one instead of following it,
+// which saves about 3 us a launch. It is what small sorts consist of (2^15 32-bit
+// keys 48 -> 36 us, 64-bit 85 -> 67), and the passes of a plan that has ended
+// (equal 64-bit keys, 2^26 of them: 369 -> 324 us).
+template <typename... P, typename... A>
+void launch_chained(void (*kernel)(P...), int grid, int threads, std::size_t smem, cudaStream_t stream, A... args)
+{
+    cudaLaunchAttribute attr[1] = {};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // the caller looks at cudaGetLastError
+}
+
 }  // namespace gbc

@@ -264,6 +264,7 @@ template <typename K, int THREADS> __global__ void __launch_bounds__(THREADS) k_
 // num_runs. Each thread takes a contiguous range of chunks.
 __global__ void __launch_bounds__(SCAN_THREADS) k_rbk_scan_chunks(uint4* chunks, uint32_t num, uint32_t* num_runs)
 {
+    dev::chain();
     static_assert(SCAN_THREADS == 32 * 32, "one lane of warp 0 per warp");
     __shared__ State s_w[SCAN_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -312,6 +313,7 @@ template <int Q> __device__ __forceinline__ int staged(int t, int q)
 // directly spreads each load over 32 lines: 2^29 64-bit keys, 1.79 ms).
 template <typename K, int THREADS> __global__ void __launch_bounds__(THREADS) k_rbk_runs(RbkArgs<K> a)
 {
+    dev::chain();
     constexpr int TILE = THREADS * ITEMS;
     constexpr int SUB = CHUNK / TILE;
     constexpr int WARPS = THREADS / 32;
@@ -471,12 +473,12 @@ void reduce_by_key(device_context& ctx, const void* keys, int key_bytes, const u
         }
         {
             kernel_timer kt(ctx, "reduce_by_key.scan");
-            k_rbk_scan_chunks<<<1, SCAN_THREADS, 0, ctx.stream>>>(a.chunks, num_chunks, num_runs_device);
+            launch_chained(&k_rbk_scan_chunks, 1, SCAN_THREADS, 0, ctx.stream, a.chunks, num_chunks, num_runs_device);
             check_cuda(cudaGetLastError(), "reduce_by_key scan launch");
         }
         {
             kernel_timer kt(ctx, "reduce_by_key.runs");
-            k_rbk_runs<K, THREADS><<<num_chunks, THREADS, 0, ctx.stream>>>(a);
+            launch_chained(&k_rbk_runs<K, THREADS>, (int)num_chunks, THREADS, 0, ctx.stream, a);
             check_cuda(cudaGetLastError(), "reduce_by_key runs launch");
         }
     };

@@ -404,6 +404,7 @@ template <typename K, bool HAS_V, bool SUB> __device__ __forceinline__ void seg_
 template <typename K, bool HAS_V, bool SUB>
 __global__ void __launch_bounds__(SMALL_THREADS) k_seg_small_warp(SegArgs<K> a)
 {
+    dev::chain();
     seg_small_warp<K, HAS_V, SUB>(a);
 }
 
@@ -417,6 +418,7 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_seg_small_warp(SegArgs<K> a)
 template <typename K, bool HAS_V, int THREADS, int ITEMS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) k_seg_tile(SegArgs<K> a, int cls, int last, bool sub)
 {
+    dev::chain();
     using S = tile::Sorter<K, HAS_V, THREADS, ITEMS>;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ tile::Scratch<THREADS> scratch;
@@ -560,6 +562,7 @@ __device__ __forceinline__ void seg_large_count(const SegArgs<K>& a, uint32_t ct
 
 template <typename K, int TILE, int STEP> __global__ void __launch_bounds__(256) k_seg_large_count(SegArgs<K> a)
 {
+    dev::chain();
     seg_large_count<K, TILE, STEP>(a, gridDim.x);
 }
 
@@ -659,6 +662,7 @@ __device__ __forceinline__ void seg_route(const SegArgs<K>& a, bool with_msd, ui
 
 template <typename K, int TILE, int STEP> __global__ void __launch_bounds__(256) k_seg_route(SegArgs<K> a, bool with_msd)
 {
+    dev::chain();
     seg_route<K, TILE, STEP>(a, with_msd, gridDim.x);
 }
 
@@ -910,6 +914,7 @@ __device__ __forceinline__ void seg_large_pass(const SegArgs<K>& a, int slot, bo
 template <typename K, bool HAS_V, int THREADS, int ITEMS, int MINB, int LBW, bool MSD>
 __global__ void __launch_bounds__(THREADS, MINB) k_seg_large_pass(SegArgs<K> a, int slot, bool with_msd)
 {
+    dev::chain();
     seg_large_pass<K, HAS_V, THREADS, ITEMS, LBW, MSD>(a, slot, with_msd, gridDim.x);
 }
 
@@ -984,7 +989,7 @@ static void launch_cta_sorts(device_context& ctx, const SegArgs<K>& a, bool sub,
     auto launch = [&](auto kern, int cta, std::size_t smem, uint32_t above, int cls, int last) {
         const std::size_t most = n / (above + 1) + 1;  // segments of the class
         const int grid = (int)std::min<std::size_t>(most, (std::size_t)ctx.sm_count * std::max(1, occupancy(kern, cta, smem)));
-        kern<<<grid, cta, smem, st>>>(a, cls, last, sub);
+        launch_chained(kern, grid, cta, smem, st, a, cls, last, sub);
     };
     constexpr bool SMALL = sizeof(K) == 4;
     const int lowest = n <= VERY_FEW_KEYS ? 0 : n <= FEW_KEYS ? 1 : 2;  // class that the largest CTA's launch starts at
@@ -1112,18 +1117,18 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
             const int tgrid = (int)std::min<std::size_t>(max_tiles, (std::size_t)ctx.sm_count * 4);
             k_seg_large_plan<K, TILE><<<tgrid, 256, 0, aux>>>(a);
             auto count = [&](auto hk) {
-                hk<<<(int)std::min<std::size_t>(max_tiles, (std::size_t)ctx.sm_count * std::max(1, occupancy(hk, 256, 0))), 256, 0,
-                     aux>>>(a);
+                launch_chained(hk, (int)std::min<std::size_t>(max_tiles, (std::size_t)ctx.sm_count * std::max(1, occupancy(hk, 256, 0))),
+                               256, 0, aux, a);
             };
             const int rgrid = (int)std::min<std::size_t>(max_large, (std::size_t)ctx.sm_count * 8);
             if (two_steps) {
                 count(&k_seg_large_count<K, TILE, COUNT_FIRST>);
-                k_seg_route<K, TILE, COUNT_FIRST><<<rgrid, 256, 0, aux>>>(a, true);
+                launch_chained(&k_seg_route<K, TILE, COUNT_FIRST>, rgrid, 256, 0, aux, a, true);
                 count(&k_seg_large_count<K, TILE, COUNT_REST>);
-                k_seg_route<K, TILE, COUNT_REST><<<rgrid, 256, 0, aux>>>(a, true);
+                launch_chained(&k_seg_route<K, TILE, COUNT_REST>, rgrid, 256, 0, aux, a, true);
             } else {
                 count(&k_seg_large_count<K, TILE, COUNT_ALL>);
-                k_seg_route<K, TILE, COUNT_ALL><<<rgrid, 256, 0, aux>>>(a, msd);
+                launch_chained(&k_seg_route<K, TILE, COUNT_ALL>, rgrid, 256, 0, aux, a, msd);
             }
             check_cuda(cudaGetLastError(), "segmented sort histogram launch");
         }
@@ -1135,14 +1140,14 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
             auto mk = &k_seg_large_pass<K, HAS_V, LS::THREADS, LS::ITEMS, LS::MINB, LS::LBW, true>;
             const int mgrid = pass_grid(mk);
             kernel_timer kt(ctx, "segsort.msd_pass", aux);
-            mk<<<mgrid, LS::THREADS, psmem, aux>>>(a, 0, true);
+            launch_chained(mk, mgrid, LS::THREADS, psmem, aux, a, 0, true);
             check_cuda(cudaGetLastError(), "segmented sort MSD pass launch");
         }
         auto pk = &k_seg_large_pass<K, HAS_V, LS::THREADS, LS::ITEMS, LS::MINB, LS::LBW, false>;
         const int pgrid = pass_grid(pk);
         for (int s = 0; s < P; ++s) {
             kernel_timer kt(ctx, "segsort.large_pass", aux);
-            pk<<<pgrid, LS::THREADS, psmem, aux>>>(a, s, msd);
+            launch_chained(pk, pgrid, LS::THREADS, psmem, aux, a, s, msd);
             check_cuda(cudaGetLastError(), "segmented sort pass launch");
         }
         if (msd) {
@@ -1152,7 +1157,7 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
             auto wk = &k_seg_small_warp<K, HAS_V, true>;
             const int grid = (int)std::min<std::size_t>((max_sub + SMALL_WARPS - 1) / SMALL_WARPS,
                                                         (std::size_t)ctx.sm_count * std::max(1, occupancy(wk, SMALL_THREADS, smem)));
-            wk<<<grid, SMALL_THREADS, smem, aux>>>(a);
+            launch_chained(wk, grid, SMALL_THREADS, smem, aux, a);
             launch_cta_sorts<K, HAS_V>(ctx, a, true, msd_cap, n, opt.cta_threads, aux);
         }
     }

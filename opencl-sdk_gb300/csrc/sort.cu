@@ -87,6 +87,7 @@ template <typename K> struct SortArgs {
 template <typename K, int THREADS, int NSUB>
 __global__ void __launch_bounds__(THREADS) k_upfront(SortArgs<K> a)
 {
+    dev::chain();
     constexpr int P = Traits<K>::PASSES;
     constexpr int PER_VEC = 16 / sizeof(K);
     extern __shared__ __align__(16) uint32_t sh_hist[];  // NSUB x P x 256
@@ -178,6 +179,7 @@ __global__ void __launch_bounds__(THREADS) k_upfront(SortArgs<K> a)
 // number of active passes, which then start from the scratch buffer).
 template <typename K> __global__ void k_precopy(SortArgs<K> a)
 {
+    dev::chain();
     const uint32_t act = a.ctl->plan.num_active;
     const K* s;
     K* d;
@@ -417,11 +419,13 @@ __device__ __forceinline__ void pass_body(const SortArgs<K>& a, int slot)
 template <typename K, bool HAS_V, int THREADS, int ITEMS, bool MATCH>
 __global__ void __launch_bounds__(THREADS) k_pass(SortArgs<K> a, int slot)
 {
+    dev::chain();
     pass_body<K, HAS_V, THREADS, ITEMS, MATCH>(a, slot);
 }
 template <typename K, bool HAS_V, int THREADS, int ITEMS, bool MATCH, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) k_pass_mb(SortArgs<K> a, int slot)
 {
+    dev::chain();
     pass_body<K, HAS_V, THREADS, ITEMS, MATCH>(a, slot);
 }
 
@@ -979,6 +983,7 @@ template <typename K, bool HAS_V, int THREADS, int ITEMS, bool IDENT, int MINB, 
           bool HALF, int PAD, bool PACK = false, bool TOFF = false>
 __global__ void __launch_bounds__(THREADS, MINB) k_pass2(SortArgs<K> a, int slot)
 {
+    dev::chain();
     pass2_body<K, HAS_V, THREADS, ITEMS, IDENT, LBW, STAGED, PF, BR, HALF, PAD, PACK, TOFF>(a, slot);
 }
 
@@ -1254,7 +1259,7 @@ static void run_passes(device_context& ctx, SortArgs<K> a, const PassVariant<K>&
     const int cgrid = (int)std::max<std::size_t>(1, std::min<std::size_t>((n + 255) / 256, (std::size_t)ctx.sm_count * 8));
     if (copy) {
         kernel_timer kt(ctx, "sort.precopy");
-        k_precopy<K><<<cgrid, 256, 0, ctx.stream>>>(a);
+        launch_chained(&k_precopy<K>, cgrid, 256, 0, ctx.stream, a);
         check_cuda(cudaGetLastError(), "radix sort copy launch");
     }
 
@@ -1267,7 +1272,7 @@ static void run_passes(device_context& ctx, SortArgs<K> a, const PassVariant<K>&
     if (pv.hist == nullptr) {
         for (int s = 0; s < passes; ++s) {
             kernel_timer kt(ctx, "sort.digit_pass");
-            pk<<<pgrid, pv.threads, psmem, ctx.stream>>>(a, s);
+            launch_chained(pk, pgrid, pv.threads, psmem, ctx.stream, a, s);
             check_cuda(cudaGetLastError(), "radix sort pass launch");
         }
         return;
@@ -1358,20 +1363,21 @@ template <typename K, bool HAS_V> static bool run_partial(device_context& ctx, c
         kernel_timer kt(ctx, "sort.faults");
         const int per_sm = prepare_kernel(&k_faults<K, HAS_V>, 256, 0, g_occupancy, g_occupancy_mutex);
         const int grid = (int)std::min<std::size_t>((n + FT_TILE - 1) / FT_TILE, (std::size_t)ctx.sm_count * per_sm);
-        k_faults<K, HAS_V><<<grid, 256, 0, ctx.stream>>>(p);
+        launch_chained(&k_faults<K, HAS_V>, grid, 256, 0, ctx.stream, p);
         check_cuda(cudaGetLastError(), "radix sort fault search launch");
     }
     {
         kernel_timer kt(ctx, "sort.repair");
-        k_repair<K, HAS_V><<<std::max<int>(1, std::min<int>((int)(max_faults / 256), ctx.sm_count * 2)), 256, 0, ctx.stream>>>(p);
+        launch_chained(&k_repair<K, HAS_V>, std::max<int>(1, std::min<int>((int)(max_faults / 256), ctx.sm_count * 2)), 256, 0,
+                       ctx.stream, p);
         if (segmented) {
             const std::size_t smem = tile::Sorter<uint32_t, true, 1024, MAX_LONG / 1024>::SMEM;
             prepare_kernel(&k_long_runs, 1024, smem, g_occupancy, g_occupancy_mutex);
-            k_long_runs<<<1, 1024, smem, ctx.stream>>>(p.ctl, p.all, p.begin, p.end, p.off, a.n, ctx.d_error);
+            launch_chained(&k_long_runs, 1, 1024, smem, ctx.stream, p.ctl, p.all, p.begin, p.end, p.off, a.n, ctx.d_error);
         } else {
             const std::size_t smem = tile::Sorter<K, HAS_V, 512, 16>::SMEM;
             prepare_kernel(&k_sort_long_runs<K, HAS_V>, 512, smem, g_occupancy, g_occupancy_mutex);
-            k_sort_long_runs<K, HAS_V><<<ctx.sm_count, 512, smem, ctx.stream>>>(p, ctx.d_error);
+            launch_chained(&k_sort_long_runs<K, HAS_V>, ctx.sm_count, 512, smem, ctx.stream, p, ctx.d_error);
         }
         check_cuda(cudaGetLastError(), "radix sort repair launch");
     }

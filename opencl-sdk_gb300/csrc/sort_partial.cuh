@@ -238,6 +238,7 @@ template <typename K> __device__ __noinline__ void note_long_run(const Args<K>& 
 // for 2^29 Zipf keys and 6 ms for uniform ones.)
 template <typename K, bool HAS_V> __global__ void __launch_bounds__(256) k_faults(Args<K> p)
 {
+    dev::chain();
     const uint32_t lo = p.ctl->lowest;
     if (lo == 0) return;
     __shared__ K s_keys[FT_TILE + 2 * FT_HALO];
@@ -300,6 +301,7 @@ template <typename K, bool HAS_V> __global__ void __launch_bounds__(256) k_fault
 // One thread per short run: insertion in place, on the output arrays.
 template <typename K, bool HAS_V> __global__ void __launch_bounds__(256) k_repair(Args<K> p)
 {
+    dev::chain();
     const uint32_t lo = p.ctl->lowest;
     if (lo == 0) return;
     const Output<K> out{p.a.out_keys, p.a.xf, p.a.n, lo};
@@ -332,6 +334,7 @@ template <typename K, bool HAS_V> __global__ void __launch_bounds__(256) k_repai
 __global__ void __launch_bounds__(1024) k_long_runs(Control* ctl, SortControl* all, const uint32_t* begin,
                                                     const uint32_t* end, uint32_t* off, uint32_t n, int* err)
 {
+    dev::chain();
     constexpr int ITEMS = MAX_LONG / 1024;
     using S = tile::Sorter<uint32_t, true, 1024, ITEMS>;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -364,6 +367,7 @@ __global__ void __launch_bounds__(1024) k_long_runs(Control* ctl, SortControl* a
 // each. One that fits no CTA sends the array through all its digits.
 template <typename K, bool HAS_V> __global__ void __launch_bounds__(512, 1) k_sort_long_runs(Args<K> p, int* err)
 {
+    dev::chain();
     using S = tile::Sorter<K, HAS_V, 512, 16>;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ tile::Scratch<512> scratch;
