@@ -959,12 +959,13 @@ def run_extras(ctx, gbc, torch, np, stream, timed, uniform_u32, n, peak, steps, 
                                    torch.from_numpy(lens).cuda())
     ok = ok and bool(torch.equal(sy.to(torch.int64), csum - sx.to(torch.int64) - base))
     graph.release()
-    # bytes the chosen pass counts move: segments up to the one-CTA capacity
-    # are read and written once (24 B per u64 key + u32 value); larger ones
-    # take the batched onesweep: an 8 B histogram read and 8 digit passes of
-    # 24 B (uniform 64-bit keys: no digit position is skipped); the scan 8 B
+    # bytes the chosen route moves: segments up to the one-CTA capacity are
+    # read and written once (24 B per u64 key + u32 value); larger ones are
+    # counted (8 B) and take one pass and the one-CTA sorts of its buckets
+    # (24 B each), or without that route 8 digit passes; the scan 8 B
     large_keys = int(lens[lens > int(seg_cap)].sum())
-    seg_bytes = 24 * (total - large_keys) + (8 + 8 * 24) * large_keys + 8 * total
+    large_bytes = 8 + 24 * (2 if msd_cap != 0 else 8)
+    seg_bytes = 24 * (total - large_keys) + large_bytes * large_keys + 8 * total
     entry("segmented_sort_u64kv_200k_lognormal", total, "Gkeys/s", ms_seg, seg_bytes, ok, prof_s,
           {"segments": int(lens.size), "total_keys": total, "graph": True, "autotuned_cta_capacity": seg_cap,
            "autotuned_msd_capacity": msd_cap, "autotuned_cta_threads": seg_threads,
@@ -978,8 +979,8 @@ def run_extras(ctx, gbc, torch, np, stream, timed, uniform_u32, n, peak, steps, 
            "plain_lsd": "stable plain sort of all pairs by key, stable plain sort of the segment ids in that order, "
                         "gathers of keys and values (sort only: the segmented figure also includes the scan)",
            "hbm_frac_one_pass": 32 * total / (ms_seg * 1e-3) / 1e9 / peak,
-           "note": "bytes: 24 B/pair in segments <= the one-CTA capacity, 200 B/pair above it (8 B histogram "
-                   "+ 8 digit passes x 24 B), 8 B/elem scan; hbm_frac_one_pass counts 32 B/key"})
+           "note": f"bytes: 24 B/pair in segments <= the one-CTA capacity, {large_bytes} B/pair above it (8 B count, "
+                   f"{(large_bytes - 8) // 24} passes x 24 B), 8 B/elem scan; hbm_frac_one_pass counts 32 B/key"})
     del sk, sv, sko, svo, sx, sy, seg_id, order, csum, base
     torch.cuda.empty_cache()
 
@@ -1013,10 +1014,11 @@ def run_extras(ctx, gbc, torch, np, stream, timed, uniform_u32, n, peak, steps, 
     ref_sums = torch.zeros(r, dtype=torch.int64, device="cuda").index_add_(0, seg, zvo.long())
     ok = ok and bool(torch.equal(sums[:r], ref_sums))
     ok = ok and bool(torch.equal(torch.bincount(zk & 0xFFFF, minlength=65536).to(torch.int32), h16))
-    entry("pipeline_sort_rbk_hist_u64_zipf_n2^29", np_, "Gkeys/s", ms_pipe, 212 * np_, ok,
+    entry("pipeline_sort_rbk_hist_u64_zipf_n2^29", np_, "Gkeys/s", ms_pipe, 172 * np_, ok,
           prof_pipe, {"runs": int(r), "key": "splitmix64(Zipf(1.1) rank over 2^24 values)",
                       "values": "u32 uniform [0, 2^16)",
-                      "note": "bytes: 8 B upfront histogram + 8 digit passes x 24 B + 12 B reduce_by_key read = 212 B/key"})
+                      "note": "bytes: 8 B upfront histogram + 6 leading digit passes x 24 B + 8 B check + 12 B reduce_by_key "
+                              "read = 172 B/key; all 8 passes would be 212"})
     # the learned-CDF form of the same pipeline: the key-value learned sort
     # (64-bit keys bucketed through a monotone 32-bit projection, stable
     # partition), then the same reduce_by_key + histogram; identical results
@@ -1035,13 +1037,13 @@ def run_extras(ctx, gbc, torch, np, stream, timed, uniform_u32, n, peak, steps, 
     ok_l = ok_l and bool(torch.equal(sums[:r], ref_sums))
     ok_l = ok_l and bool(torch.equal(torch.bincount(zk & 0xFFFF, minlength=65536).to(torch.int32), h16))
     ls = lstats[-1]
-    entry("pipeline_learned_sort_rbk_hist_u64_zipf_n2^29", np_, "Gkeys/s", ms_learn, 212 * np_, ok_l, prof_learn,
+    entry("pipeline_learned_sort_rbk_hist_u64_zipf_n2^29", np_, "Gkeys/s", ms_learn, 172 * np_, ok_l, prof_learn,
           {"plain_pipeline_ms": ms_pipe, "speedup_vs_plain": ms_pipe / ms_learn,
            "stats": {"buckets": ls.buckets, "nonempty_buckets": ls.nonempty_buckets,
                      "oversized_keys": ls.oversized_keys, "fallback": ls.fallback, "violation": ls.violation,
                      "first_loss": ls.first_loss, "last_loss": ls.last_loss},
            "note": "learned-CDF key-value sort (fit, stable bucket partition, segmented finish) + reduce_by_key + "
-                   "histogram; bytes counted as the plain form's 212 B/key"})
+                   "histogram; bytes counted as the plain form's 172 B/key"})
     # the same pipeline on the raw Zipf ranks as keys (< 2^24: the pass plan
     # runs 3 of the 8 digit passes)
     rk, _ = zipf_splitmix_keys(torch, np_, 1.1, 1 << 24, 6, raw_rank=True)
@@ -1099,8 +1101,8 @@ def run_extras(ctx, gbc, torch, np, stream, timed, uniform_u32, n, peak, steps, 
     entry("bitpack_compress_u32_timestamps_n2^28", nb, "Gelem/s", ms_c, 8 * nb + 4 * w, ok, prof_c,
           {"ratio": 4 * nb / (4 * w), "words": int(w), "delta": True, "chunk": 2048,
            "note": "includes the blocking read of the compressed size"})
-    entry("bitpack_decompress_u32_timestamps_n2^28", nb, "Gelem/s", ms_d, 4 * w + 4 * nb + 8 * nb, ok, prof_d,
-          {"note": "unpack (packed words in, deltas out) + in-place inclusive scan"})
+    entry("bitpack_decompress_u32_timestamps_n2^28", nb, "Gelem/s", ms_d, 4 * w + 4 * nb, ok, prof_d,
+          {"note": "one pass: decode and prefix sum (packed words in, values out)"})
     del ts, packed, back
     torch.cuda.empty_cache()
 
