@@ -20,7 +20,7 @@ struct seg_options {
     // sorts finish the buckets; 0: every large segment takes all digit
     // passes; -1: the default (the tuning table's entry, else off for
     // 32-bit keys up to 2^26 of them and the one-CTA maximum otherwise: the
-    // batch of 200,000 lognormal segments of u64 pairs takes 11.7 ms with its
+    // batch of 200,000 lognormal segments of u64 pairs takes 11.1 ms with its
     // scan, 27.0 with the one-CTA sorts of every digit and the route off)
     int msd_cap = -1;
     // threads of the one-CTA sorts of up to 4,096 keys: 256 (16 keys per

@@ -1076,7 +1076,8 @@ template <bool HV> struct Variants<uint32_t, HV> {
     // stay at 24: 28 and 32 cost 3 to 6 % from 2^22.
     static constexpr int LONG_TILES = 7;
     // 8 a thread, the default to 2^18 elements: the passes are then a chain of
-    // launches that each take a tile's latency, with most SMs idle (2^14 keys
+    // launches that each take a tile's latency, with most SMs idle (before
+    // launches overlapped: 2^14 keys
     // 43 us for 49, pairs 48 for 55; 2^18 56 for 56 and 56 for 64; at 2^19
     // pairs 71 for 65).
     static constexpr int SHORT_TILES = 8;

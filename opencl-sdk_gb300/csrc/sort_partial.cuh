@@ -35,12 +35,14 @@ namespace partial {
 
 using dev::FULL_MASK;
 
-// MIN_KEYS and SEGMENTED_KEYS: where the extra launches (62 us, and 160 with the
-// segmented sort's) stay below 2% of a sort that has no use for them (2^26
-// pairs whose keys are the AND of 4 words: 4.40 -> 4.46 ms; uniform 4.20 ->
-// 2.48). Long runs of any length go to the segmented sort in the largest sorts
-// only; below, one kernel sorts those of up to a CTA's capacity.
-constexpr std::size_t MIN_KEYS = std::size_t(1) << 26, SEGMENTED_KEYS = std::size_t(1) << 27;
+// MIN_KEYS: the extra steps cost a sort that has no use for them 25 to 30 us and
+// save 40% of one that has (pairs, all digits at once / this: 2^23 keys that are
+// the AND of 4 words 628 / 660 us, uniform ones 631 / 420; 2^25 2075 / 2106 and
+// 2159 / 1278; 2^22 356 / 386 and 366 / 271).
+// SEGMENTED_KEYS: long runs of any length go to the segmented sort, which is 50 us
+// more; below, one kernel sorts those of up to a CTA's capacity (sort and
+// reduce_by_key of 1.5 10^8 Zipf keys: 5.91 ms for 6.78).
+constexpr std::size_t MIN_KEYS = std::size_t(1) << 23, SEGMENTED_KEYS = std::size_t(1) << 27;
 constexpr int CANDIDATES = 3;  // digit counts tried: the least possible, and one or two more
 constexpr int FIRST_PASSES = 6;  // digit passes launched before the faults are looked for
 constexpr uint32_t MIN_SAMPLE = 1u << 15, MAX_SAMPLE = 1u << 17;

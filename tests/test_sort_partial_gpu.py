@@ -1,4 +1,4 @@
-"""64-bit sorts that order the leading digits and repair the rest (from 2^26
+"""64-bit sorts that order the leading digits and repair the rest (from 2^23
 keys; from 2^27 long runs go to the segmented sort): distributions that need no
 repair, short and long repairs, all digits, and one that the sample misjudges,
 against torch's stable sort bit for bit."""
@@ -7,6 +7,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
+N_LEAST = 1 << 23
 N = (1 << 26) + 4321
 N_SEGMENTED = (1 << 27) + 4321
 
@@ -64,7 +65,8 @@ def expected(keys, descending=False):
     return keys.view(np.uint64)[order], order.astype(np.uint32)
 
 
-CASES = [(N, k) for k in ("uniform", "few_values", "long_runs", "groups", "low_digits", "seven_digits", "misjudged")] + \
+CASES = [(n, k) for n in (N_LEAST, N) for k in ("uniform", "few_values", "long_runs", "groups", "low_digits",
+                                                "seven_digits", "misjudged")] + \
         [(N_SEGMENTED, "long_runs")]
 
 
