@@ -1014,11 +1014,11 @@ def run_extras(ctx, gbc, torch, np, stream, timed, uniform_u32, n, peak, steps, 
     ref_sums = torch.zeros(r, dtype=torch.int64, device="cuda").index_add_(0, seg, zvo.long())
     ok = ok and bool(torch.equal(sums[:r], ref_sums))
     ok = ok and bool(torch.equal(torch.bincount(zk & 0xFFFF, minlength=65536).to(torch.int32), h16))
-    entry("pipeline_sort_rbk_hist_u64_zipf_n2^29", np_, "Gkeys/s", ms_pipe, 172 * np_, ok,
+    entry("pipeline_sort_rbk_hist_u64_zipf_n2^29", np_, "Gkeys/s", ms_pipe, 124 * np_, ok,
           prof_pipe, {"runs": int(r), "key": "splitmix64(Zipf(1.1) rank over 2^24 values)",
                       "values": "u32 uniform [0, 2^16)",
-                      "note": "bytes: 8 B upfront histogram + 6 leading digit passes x 24 B + 8 B check + 12 B reduce_by_key "
-                              "read = 172 B/key; all 8 passes would be 212"})
+                      "note": "bytes: 8 B upfront histogram + 4 leading digit passes x 24 B + 8 B check + 12 B reduce_by_key "
+                              "read = 124 B/key; all 8 passes would be 212"})
     # the learned-CDF form of the same pipeline: the key-value learned sort
     # (64-bit keys bucketed through a monotone 32-bit projection, stable
     # partition), then the same reduce_by_key + histogram; identical results
@@ -1037,13 +1037,13 @@ def run_extras(ctx, gbc, torch, np, stream, timed, uniform_u32, n, peak, steps, 
     ok_l = ok_l and bool(torch.equal(sums[:r], ref_sums))
     ok_l = ok_l and bool(torch.equal(torch.bincount(zk & 0xFFFF, minlength=65536).to(torch.int32), h16))
     ls = lstats[-1]
-    entry("pipeline_learned_sort_rbk_hist_u64_zipf_n2^29", np_, "Gkeys/s", ms_learn, 172 * np_, ok_l, prof_learn,
+    entry("pipeline_learned_sort_rbk_hist_u64_zipf_n2^29", np_, "Gkeys/s", ms_learn, 124 * np_, ok_l, prof_learn,
           {"plain_pipeline_ms": ms_pipe, "speedup_vs_plain": ms_pipe / ms_learn,
            "stats": {"buckets": ls.buckets, "nonempty_buckets": ls.nonempty_buckets,
                      "oversized_keys": ls.oversized_keys, "fallback": ls.fallback, "violation": ls.violation,
                      "first_loss": ls.first_loss, "last_loss": ls.last_loss},
            "note": "learned-CDF key-value sort (fit, stable bucket partition, segmented finish) + reduce_by_key + "
-                   "histogram; bytes counted as the plain form's 172 B/key"})
+                   "histogram; bytes counted as the plain form's 124 B/key"})
     # the same pipeline on the raw Zipf ranks as keys (< 2^24: the pass plan
     # runs 3 of the 8 digit passes)
     rk, _ = zipf_splitmix_keys(torch, np_, 1.1, 1 << 24, 6, raw_rank=True)
