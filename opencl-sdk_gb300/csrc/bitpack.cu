@@ -32,6 +32,7 @@
 //     reading the 1-5 packed words that hold them; delta mode then runs the
 //     library's scan in place.
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <functional>
 #include <stdexcept>
@@ -512,9 +513,14 @@ void bitpack_decompress(device_context& ctx, const uint32_t* data, std::size_t w
         tiles.seq0 = ctx.reserve_seq(num_tiles);
         tiles.err = ctx.d_error;
         auto kern = delta ? &k_bp_unpack_tiles<true> : &k_bp_unpack_tiles<false>;
-        int per_sm = 1;
-        check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, UT, 0), "cudaOccupancy");
-        const int grid = (int)std::min<std::size_t>(num_tiles, (std::size_t)ctx.sm_count * std::max(per_sm, 1));
+        // asked once (one architecture): the query takes as long as a launch
+        static std::atomic<int> known[2];
+        int per_sm = known[delta].load(std::memory_order_relaxed);
+        if (per_sm == 0) {
+            check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, UT, 0), "cudaOccupancy");
+            known[delta].store(per_sm = std::max(per_sm, 1), std::memory_order_relaxed);
+        }
+        const int grid = (int)std::min<std::size_t>(num_tiles, (std::size_t)ctx.sm_count * per_sm);
         kernel_timer kt(ctx, "bitpack.unpack");
         kern<<<grid, UT, 0, ctx.stream>>>(data, (uint64_t)words, (uint32_t)n, shift, chunks, out, tiles);
         check_cuda(cudaGetLastError(), "bitpack unpack launch");
