@@ -224,12 +224,11 @@ __device__ void copy_role(const Tiles& a, Shared<T>& sh, unsigned char* stages, 
 }
 
 // The prefix warp: prefix[s] = first, combined with the aggregates of all tiles
-// before the stage's. ANY_ORDER: the operator commutes, and the lanes read
-// neighbouring words (a quarter of the sectors: scan of 2^30 int32 1.31 -> 1.26
-// ms); else each lane reads
-// PER consecutive ones, so that they combine in order. (Two prefix warps taking
-// the CTA's tiles in turn read twice as many words and were slower: 2^30 int32
-// 1.31 -> 1.55 ms.)
+// before the stage's. ANY_ORDER: no order changes the operator's result, and the
+// lanes read neighbouring words, a quarter of the sectors (scan of 2^30 int32
+// 1.31 -> 1.26 ms); else each lane reads PER consecutive ones, so that they
+// combine in order. (Two prefix warps taking the CTA's tiles in turn read twice
+// as many words and were slower: 2^30 int32 1.31 -> 1.55 ms.)
 template <bool ANY_ORDER, typename T, typename Op> __device__ void prefix_role(const Tiles& a, Shared<T>& sh, T first, Op op)
 {
     const int lane = threadIdx.x & 31;

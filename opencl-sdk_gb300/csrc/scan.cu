@@ -359,14 +359,46 @@ __global__ void __launch_bounds__(THREADS, MINB) k_scan(ScanArgs<T> a)
 // shape and the reads of pipe.cuh 1.21 ms, the copy rate. 2^28 int64 2.05 ->
 // 0.75 ms.
 // ---------------------------------------------------------------------------
+// Operators for which a thread may combine its rows before its lane's neighbours,
+// and the prefix warp tiles 32 apart: those whose results no order changes.
+// Floating-point ones keep the sequence's order: minimum and maximum return the
+// first of two equal operands (so -0.0 and +0.0 do not commute), and sums and
+// products that overflow in one order need not in another. (2^28 floats: 309
+// us in any order, 324 in sequence.)
+template <typename T, typename Op>
+constexpr bool any_order = std::is_integral<T>::value && !std::is_same<Op, ops::Right>::value;
+
+// op over four rows of one value per lane, in sequence order (row, then lane),
+// to lane 0. The lanes halve the rows among them while they combine, which takes
+// 8 operations where a reduction per row takes 23: what counts for doubles,
+// whose arithmetic bounds their scan (2^28 of them: 4.56 ms with a reduction
+// per row, 3.42 with this, 3.46 in the look-back form).
+template <typename T, typename Op> __device__ __forceinline__ T fold_rows(const T (&acc)[4], Op op)
+{
+    const int lane = threadIdx.x & 31;
+    // `mine` and the value of lane ^ o, the lower lane's first
+    auto with = [&](const T& mine, const T& sent, int o) {
+        const T got = __shfl_xor_sync(FULL_MASK, sent, o);
+        const bool upper = (lane & o) != 0;
+        return op(upper ? got : mine, upper ? mine : got);
+    };
+    const bool b0 = (lane & 1) != 0, b1 = (lane & 2) != 0;
+    const T even = with(b0 ? acc[2] : acc[0], b0 ? acc[0] : acc[2], 1);  // row 0, odd lanes 2
+    const T odd = with(b0 ? acc[3] : acc[1], b0 ? acc[1] : acc[3], 1);   // row 1, odd lanes 3
+    T v = with(b1 ? odd : even, b1 ? even : odd, 2);                     // lanes 0, 2, 1, 3 of each four: rows 0 to 3
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) v = with(v, v, o);
+    v = with(v, v, 2);
+    return with(v, v, 1);
+}
+
 template <typename T, typename Op, bool WIDE_SUM>
 __global__ void __launch_bounds__(pipe::THREADS, 1) k_scan_pipe(ScanArgs<T> a)
 {
     using namespace pipe;
     constexpr int VEC = 16 / sizeof(T);
     constexpr uint32_t TILE = TILE_BYTES / sizeof(T);
-    // Operators for which a thread may combine its rows before its lane's neighbours.
-    constexpr bool ANY_ORDER = !std::is_same<Op, ops::Right>::value;
+    static_assert(ROWS == 4, "fold_rows");
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ Shared<T> sh;
     __shared__ T s_before[STAGES][WRITERS];
@@ -375,7 +407,7 @@ __global__ void __launch_bounds__(pipe::THREADS, 1) k_scan_pipe(ScanArgs<T> a)
     const Op op;
     sh.init();
     if (warp == COPY_WARP) return copy_role(tiles, sh, smem, a.in, (uint64_t)a.n * sizeof(T));
-    if (warp == PREFIX_WARP) return prefix_role<ANY_ORDER>(tiles, sh, a.identity, op);
+    if (warp == PREFIX_WARP) return prefix_role<any_order<T, Op>>(tiles, sh, a.identity, op);
 
     // A row of 512 bytes of the tile: this lane's 16 bytes, from the stage or,
     // for a partial tile, from the input (the identity past its end).
@@ -420,14 +452,12 @@ __global__ void __launch_bounds__(pipe::THREADS, 1) k_scan_pipe(ScanArgs<T> a)
                     }
                 }
                 T total;
-                if (ANY_ORDER) {
+                if (any_order<T, Op>) {
 #pragma unroll
                     for (int r = 1; r < ROWS; ++r) acc[0] = op(acc[0], acc[r]);
                     total = dev::warp_reduce(acc[0], op);
                 } else {
-                    total = dev::warp_reduce(acc[0], op);
-#pragma unroll
-                    for (int r = 1; r < ROWS; ++r) total = op(total, dev::warp_reduce(acc[r], op));
+                    total = fold_rows(acc, op);
                 }
                 if (lane == 0) sh.total[k & 1][f * BLOCKS + b] = total;
             }
@@ -517,9 +547,12 @@ template <typename F> int blocks_per_sm(F* kernel, std::size_t smem = 0, int thr
     return b;
 }
 
-// From this input size the pipelined kernel is the faster one (int32, k_scan
-// against it: 16 MiB 16.0 / 15.2 us, 32 MiB 25.2 / 19.0, 64 MiB 44.8 / 32.6).
-constexpr std::size_t PIPE_MIN_BYTES = std::size_t(1) << 24;
+// From this input size the pipelined kernel is the faster one (k_scan against
+// it, int32: 16 MiB 16.0 / 15.2 us, 32 MiB 25.2 / 19.0, 64 MiB 44.8 / 32.6; with
+// the sequence's order kept, float: 16 MiB 14.6 / 16.7, 24 MiB 20.9 / 19.3, 32
+// MiB 24.0 / 20.7; double: 16 MiB 44.7 / 47.2, 24 MiB 62.1 / 58.3, 32 MiB 76.7 / 68.2).
+template <typename T, typename Op>
+constexpr std::size_t PIPE_MIN_BYTES = std::size_t(1) << (any_order<T, Op> ? 24 : 25);
 
 struct ScanLaunch {
     device_context& ctx;
@@ -549,7 +582,7 @@ struct ScanLaunch {
             default: break;
             }
         }
-        if (n * sizeof(T) >= PIPE_MIN_BYTES && aligned() && ctx.smem_optin >= pipe::SMEM + 4096) run_pipe<T, Op>();
+        if (n * sizeof(T) >= PIPE_MIN_BYTES<T, Op> && aligned() && ctx.smem_optin >= pipe::SMEM + 4096) run_pipe<T, Op>();
         else if constexpr (sizeof(T) == 4) run_shape<T, Op, 16, 2, PREFETCH_GRIDS>();
         else run_shape<T, Op, 8, 2, PREFETCH_GRIDS>();
     }
