@@ -67,6 +67,15 @@ __device__ __forceinline__ void st_relaxed(uint64_t* p, uint64_t v)
 {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
+// Two neighbouring words in one access (16-byte aligned), with no order between them.
+__device__ __forceinline__ void ld_relaxed2(const uint64_t* p, uint64_t& x, uint64_t& y)
+{
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void st_relaxed2(uint64_t* p, uint64_t x, uint64_t y)
+{
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(x), "l"(y) : "memory");
+}
 __device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p)
 {
     uint32_t v;

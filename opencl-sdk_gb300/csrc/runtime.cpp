@@ -215,7 +215,9 @@ bool device_context::capturing() const
 
 uint64_t device_context::reserve_seq(uint64_t count)
 {
-    constexpr uint64_t WRAP = uint64_t(1) << 30;
+    // The segmented scan's tags have 29 bits, the others' 30; with the ring cleared
+    // whenever the shortest starts over, no word can pass for one of a later tile.
+    constexpr uint64_t WRAP = uint64_t(1) << 29;
     if (capturing()) {
         // A graph replays the sequence numbers it was captured with, so the
         // words of the previous replay would carry matching tags: a captured

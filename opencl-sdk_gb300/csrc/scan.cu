@@ -54,9 +54,10 @@ template <typename T> __device__ __forceinline__ T from_bits(uint64_t b)
 }
 
 // Status of one tile. 32-bit elements: one word (flag | tag | value) that is
-// overwritten atomically from AGG to PRE. 64-bit elements: separate words for
-// the aggregate and the inclusive prefix, published with release stores
-// before the flag word, so a reader never pairs a flag with the wrong value.
+// overwritten atomically from AGG to PRE. 64-bit elements: two such words, each
+// with half of the value, for the aggregate and two for the inclusive prefix.
+// Every word of the ring carries its tag: a bare value could read as another
+// tile's status later (a double in [2, 4) has the bits of FLAG_AGG and a tag).
 template <typename T, bool WIDE = (sizeof(T) == 8)> struct Status;
 
 template <typename T> struct Status<T, false> {
@@ -78,20 +79,28 @@ template <typename T> struct Status<T, false> {
 
 template <typename T> struct Status<T, true> {
     static constexpr uint64_t SLOTS = onesweep::RING_BYTES / 32;
+    __device__ static uint64_t head(uint64_t flag, uint64_t seq) { return (flag << 30) | (seq & TAG_MASK); }
     __device__ static void publish(uint64_t* ring, uint64_t seq, uint64_t flag, T v)
     {
-        uint64_t* s = ring + (seq & (SLOTS - 1)) * 4;
-        dev::st_relaxed(&s[flag == FLAG_PRE ? 1 : 0], to_bits(v));
-        dev::st_release(&s[2], (flag << 62) | ((seq & TAG_MASK) << 32));
+        uint64_t* s = ring + (seq & (SLOTS - 1)) * 4 + (flag == FLAG_PRE ? 2 : 0);
+        const uint64_t bits = to_bits(v), h = head(flag, seq) << 32;
+        dev::st_relaxed2(s, h | (uint32_t)bits, h | (bits >> 32));
     }
     __device__ static bool read(const uint64_t* ring, uint64_t seq, uint64_t& flag, T& v)
     {
         const uint64_t* s = ring + (seq & (SLOTS - 1)) * 4;
-        const uint64_t w = dev::ld_acquire(&s[2]);
-        flag = w >> 62;
-        if (flag == 0 || ((w >> 32) & TAG_MASK) != (seq & TAG_MASK)) return false;
-        v = from_bits<T>(dev::ld_relaxed(&s[flag == FLAG_PRE ? 1 : 0]));
-        return true;
+        uint64_t w[4];  // all on their way at once
+        dev::ld_relaxed2(s, w[0], w[1]);
+        dev::ld_relaxed2(s + 2, w[2], w[3]);
+        const uint64_t pre = head(FLAG_PRE, seq), agg = head(FLAG_AGG, seq);
+        if ((w[2] >> 32) == pre && (w[3] >> 32) == pre) {
+            flag = FLAG_PRE;
+            v = from_bits<T>((w[3] << 32) | (uint32_t)w[2]);
+            return true;
+        }
+        flag = FLAG_AGG;
+        v = from_bits<T>((w[1] << 32) | (uint32_t)w[0]);
+        return (w[0] >> 32) == agg && (w[1] >> 32) == agg;
     }
 };
 

@@ -63,23 +63,29 @@ template <typename T> struct SStatus<T, false> {
         return true;
     }
 };
-template <typename T> struct SStatus<T, true> {
+template <typename T> struct SStatus<T, true> {  // halves of the value, as in the scan's status
     static constexpr uint64_t SLOTS = onesweep::RING_BYTES / 32;
+    static constexpr uint64_t HEAD = HEAD_BIT >> 32;
+    __device__ static uint64_t front(uint64_t flag, uint64_t seq) { return (flag << 30) | (seq & TAG_MASK); }
     __device__ static void publish(uint64_t* ring, uint64_t seq, uint64_t flag, bool head, T v)
     {
-        uint64_t* s = ring + (seq & (SLOTS - 1)) * 4;
-        dev::st_relaxed(&s[flag == FLAG_PRE ? 1 : 0], to_bits(v));
-        dev::st_release(&s[2], (flag << 62) | (head ? HEAD_BIT : 0) | ((seq & TAG_MASK) << 32));
+        uint64_t* s = ring + (seq & (SLOTS - 1)) * 4 + (flag == FLAG_PRE ? 2 : 0);
+        const uint64_t bits = to_bits(v), h = (front(flag, seq) | (head ? HEAD : 0)) << 32;
+        dev::st_relaxed2(s, h | (uint32_t)bits, h | (bits >> 32));
     }
     __device__ static bool read(const uint64_t* ring, uint64_t seq, uint64_t& flag, bool& head, T& v)
     {
         const uint64_t* s = ring + (seq & (SLOTS - 1)) * 4;
-        const uint64_t w = dev::ld_acquire(&s[2]);
-        flag = w >> 62;
-        if (flag == 0 || ((w >> 32) & TAG_MASK) != (seq & TAG_MASK)) return false;
-        head = (w & HEAD_BIT) != 0;
-        v = from_bits<T>(dev::ld_relaxed(&s[flag == FLAG_PRE ? 1 : 0]));
-        return true;
+        uint64_t w[4];
+        dev::ld_relaxed2(s, w[0], w[1]);
+        dev::ld_relaxed2(s + 2, w[2], w[3]);
+        const uint64_t pre = front(FLAG_PRE, seq), agg = front(FLAG_AGG, seq);
+        const bool done = ((w[2] >> 32) & ~HEAD) == pre && ((w[3] >> 32) & ~HEAD) == pre;
+        const uint64_t lo = done ? w[2] : w[0], hi = done ? w[3] : w[1];
+        flag = done ? FLAG_PRE : FLAG_AGG;
+        head = (lo & HEAD_BIT) != 0;
+        v = from_bits<T>((hi << 32) | (uint32_t)lo);
+        return done || (((lo >> 32) & ~HEAD) == agg && ((hi >> 32) & ~HEAD) == agg);
     }
 };
 
