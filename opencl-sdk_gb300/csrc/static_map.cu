@@ -51,46 +51,84 @@ __global__ void __launch_bounds__(THREADS) k_map_fill(unsigned long long* slots,
         slots[i] = empty;
 }
 
-// counters[0]: keys newly inserted, counters[1]: keys not placed (table full)
-__global__ void __launch_bounds__(THREADS)
-    k_map_insert(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ values, uint32_t n,
-                 unsigned long long* slots, uint32_t mask, uint32_t empty_key, uint32_t empty_value,
-                 unsigned int* counters, const uint32_t* n_device)
+// Written by one call, read by the host: zero at its start.
+struct Outcome {
+    unsigned int added, failed;  // keys newly inserted; keys not placed (table full)
+    unsigned int met;            // sampled keys that were there already
+};
+
+struct Table {
+    unsigned long long* slots;
+    uint32_t mask, empty_key, empty_value;
+    Outcome* outcome;
+};
+
+enum class Found { nothing, added, present, full };
+
+__device__ __forceinline__ Found insert_pair(const Table& t, uint32_t key, uint32_t value)
 {
-    if (n_device != nullptr) n = *n_device;  // at most n
-    const unsigned long long empty = pack(empty_key, empty_value);
+    if (key == t.empty_key) return Found::nothing;
+    const unsigned long long empty = pack(t.empty_key, t.empty_value), pair = pack(key, value);
+    uint32_t slot = fmix32(key) & t.mask;
+    for (uint32_t probe = 0; probe <= t.mask; ++probe) {
+        unsigned long long seen = t.slots[slot];
+        if ((uint32_t)seen == t.empty_key) seen = atomicCAS(&t.slots[slot], empty, pair);
+        if (seen == empty) return Found::added;
+        if ((uint32_t)seen == key) return Found::present;  // the first value stays
+        slot = (slot + 1) & t.mask;
+    }
+    return Found::full;
+}
+
+// Adds the lanes that found `what` to the counter; every lane of the warp calls it.
+__device__ __forceinline__ void count_found(unsigned int* counter, Found f, Found what)
+{
+    const uint32_t who = __ballot_sync(dev::FULL_MASK, f == what);
+    if (who != 0 && (threadIdx.x & 31) == 0) atomicAdd(counter, (unsigned)__popc(who));
+}
+
+// Whether the insert by regions (below) is the faster one depends on how many of
+// the keys are distinct: the direct insert of a key that is there already is a
+// read of a cached line, while the regions' cost is the table's and the keys' size
+// (2^24 keys into 2^25 slots, directly and by regions: all distinct 1.00 / 0.54 ms,
+// 2^22 values 0.75 / 0.45, 2^20 0.35 / 0.41, 1,000 0.08 / 0.51). So SAMPLE keys are
+// inserted first, and those that are there already counted: `least` distinct and
+// equally frequent values would give SAMPLE^2 / (2 least) of them. That takes up to
+// 15 us where the rest follows directly (2^22 keys into 2^25 slots: 1,000 values 35
+// us with and without it, 65,536 69 / 84, 2^20 191 / 203), and without it one value
+// repeated 2^24 times took 26 ms for 0.25, Zipf keys 9.2 for 0.17.
+constexpr uint32_t SAMPLE = 1u << 15;
+constexpr uint32_t DISTINCT_SHARE = 16;  // the lines cross at about capacity / 16 distinct values
+
+__host__ __device__ inline bool mostly_distinct(unsigned int met, uint32_t least)
+{
+    return (uint64_t)met * 2 * least <= (uint64_t)SAMPLE * SAMPLE;
+}
+
+__global__ void __launch_bounds__(THREADS)
+    k_map_sample(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ values, uint32_t n, Table t)
+{
+    const uint32_t i = blockIdx.x * THREADS + threadIdx.x, step = n / SAMPLE;
+    const uint32_t at = i * step + fmix32(i) % step;  // a varying place, so that no period of the input is followed
+    const Found f = insert_pair(t, keys[at], values[at]);
+    count_found(&t.outcome->added, f, Found::added);
+    count_found(&t.outcome->met, f, Found::present);
+}
+
+// SAMPLED: nothing to do when the sample says that the regions come next.
+template <bool SAMPLED>
+__global__ void __launch_bounds__(THREADS)
+    k_map_insert(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ values, uint32_t n, Table t, uint32_t least)
+{
+    dev::chain();
+    if (SAMPLED && mostly_distinct(*(volatile unsigned int*)&t.outcome->met, least)) return;
     const uint32_t stride = gridDim.x * THREADS;
     const uint32_t rounds = (n + stride - 1) / stride;
-    const int lane = threadIdx.x & 31;
     for (uint32_t r = 0; r < rounds; ++r) {
         const uint32_t i = r * stride + blockIdx.x * THREADS + threadIdx.x;
-        bool added = false, failed = false;
-        if (i < n) {
-            const uint32_t key = keys[i];
-            if (key != empty_key) {
-                const unsigned long long mine = pack(key, values[i]);
-                uint32_t slot = fmix32(key) & mask;
-                failed = true;
-                for (uint32_t probe = 0; probe <= mask; ++probe) {
-                    unsigned long long seen = slots[slot];
-                    if ((uint32_t)seen == empty_key) seen = atomicCAS(&slots[slot], empty, mine);
-                    if (seen == empty) {
-                        added = true, failed = false;
-                        break;
-                    }
-                    if ((uint32_t)seen == key) {  // present: the first value stays
-                        failed = false;
-                        break;
-                    }
-                    slot = (slot + 1) & mask;
-                }
-            }
-        }
-        const uint32_t a = __ballot_sync(dev::FULL_MASK, added), f = __ballot_sync(dev::FULL_MASK, failed);
-        if (lane == 0) {
-            if (a) atomicAdd(&counters[0], (unsigned)__popc(a));
-            if (f) atomicAdd(&counters[1], (unsigned)__popc(f));
-        }
+        const Found f = i < n ? insert_pair(t, keys[i], values[i]) : Found::nothing;
+        count_found(&t.outcome->added, f, Found::added);
+        count_found(&t.outcome->failed, f, Found::full);
     }
 }
 
@@ -112,8 +150,8 @@ __global__ void __launch_bounds__(THREADS)
 constexpr uint32_t REGION_BITS = 13, REGION = 1u << REGION_BITS;
 constexpr int REGION_THREADS = 512;
 constexpr uint32_t PROBES = 64;
-// A region given more pairs than this is not worth one CTA's time (a few keys
-// repeated very often): they are inserted directly.
+// A region given more pairs than this (keys repeated very often) would keep one
+// CTA busy long after the others: its pairs are inserted directly, by all of them.
 constexpr uint32_t REGION_PAIRS = 4 * REGION;
 
 __device__ __forceinline__ uint32_t undo_fmix32(uint32_t k)
@@ -182,33 +220,40 @@ __global__ void __launch_bounds__(THREADS)
     }
 }
 
-// counters: as k_map_insert; rest: pairs left over for it, rest_count of them.
+// What the region kernel leaves to direct inserts.
+struct Rest {
+    uint32_t *keys, *values;  // pairs
+    uint32_t* count;          // how many, and how many regions
+    uint32_t* regions;        // those with more than REGION_PAIRS
+};
+
 __global__ void __launch_bounds__(REGION_THREADS, 3)
     k_map_fill_regions(const uint32_t* __restrict__ hashed, const uint32_t* __restrict__ values, int rotate,
-                       const uint32_t* __restrict__ first, uint32_t regions, unsigned long long* slots, uint32_t empty_key,
-                       uint32_t empty_value, unsigned int* counters, uint32_t* rest_keys, uint32_t* rest_values,
-                       uint32_t* rest_count)
+                       const uint32_t* __restrict__ first, uint32_t regions, Table t, Rest rest)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     volatile unsigned long long* region = reinterpret_cast<volatile unsigned long long*>(smem);
-    const unsigned long long empty = pack(empty_key, empty_value);
+    const unsigned long long empty = pack(t.empty_key, t.empty_value);
     const int tid = threadIdx.x, lane = tid & 31;
     uint32_t added = 0;
     auto leave = [&](bool mine, uint32_t key, uint32_t value) {  // every lane of the warp
         const uint32_t who = __ballot_sync(dev::FULL_MASK, mine);
         if (who == 0) return;
         uint32_t at = 0;
-        if (lane == 0) at = atomicAdd(rest_count, (uint32_t)__popc(who));
+        if (lane == 0) at = atomicAdd(&rest.count[0], (uint32_t)__popc(who));
         at = __shfl_sync(dev::FULL_MASK, at, 0) + __popc(who & dev::lanemask_lt());
         if (mine) {
-            rest_keys[at] = key;
-            rest_values[at] = value;
+            rest.keys[at] = key;
+            rest.values[at] = value;
         }
     };
     for (uint32_t r = blockIdx.x; r < regions; r += gridDim.x) {
         const uint32_t b = first[r], e = first[r + 1];
         if (b == e) continue;
-        const bool direct = e - b > REGION_PAIRS;
+        if (e - b > REGION_PAIRS) {
+            if (tid == 0) rest.regions[atomicAdd(&rest.count[1], 1u)] = r;
+            continue;
+        }
         // the first pairs are on their way while the region is read
         constexpr int AHEAD = 2;
         uint32_t x[AHEAD], v[AHEAD];
@@ -221,13 +266,11 @@ __global__ void __launch_bounds__(REGION_THREADS, 3)
             }
         };
         fetch(b);
-        uint4* mem = reinterpret_cast<uint4*>(slots + (size_t)r * REGION);
+        uint4* mem = reinterpret_cast<uint4*>(t.slots + (size_t)r * REGION);
         uint4* copy = reinterpret_cast<uint4*>(smem);
-        if (!direct) {
 #pragma unroll
-            for (uint32_t i = 0; i < REGION / 2 / REGION_THREADS; ++i)
-                copy[i * REGION_THREADS + tid] = dev::ld_stream(mem + i * REGION_THREADS + tid);
-        }
+        for (uint32_t i = 0; i < REGION / 2 / REGION_THREADS; ++i)
+            copy[i * REGION_THREADS + tid] = dev::ld_stream(mem + i * REGION_THREADS + tid);
         __syncthreads();
         for (uint32_t i0 = b; i0 < e; i0 += AHEAD * REGION_THREADS) {
             if (i0 != b) fetch(i0);
@@ -236,13 +279,13 @@ __global__ void __launch_bounds__(REGION_THREADS, 3)
             for (int q = 0; q < AHEAD; ++q) {
                 const uint32_t h = __funnelshift_r(x[q], x[q], rotate);
                 const uint32_t key = undo_fmix32(h);
-                if (i0 + q * REGION_THREADS + tid >= e || key == empty_key) continue;
+                if (i0 + q * REGION_THREADS + tid >= e || key == t.empty_key) continue;
                 const unsigned long long mine = pack(key, v[q]);
                 uint32_t slot = h & (REGION - 1);
                 bool placed = false;
-                for (uint32_t p = 0; !direct && p < PROBES && slot < REGION; ++p, ++slot) {
+                for (uint32_t p = 0; p < PROBES && slot < REGION; ++p, ++slot) {
                     unsigned long long seen = region[slot];
-                    if ((uint32_t)seen == empty_key)
+                    if ((uint32_t)seen == t.empty_key)
                         seen = atomicCAS(const_cast<unsigned long long*>(&region[slot]), empty, mine);
                     if (seen == empty) ++added;
                     if (seen == empty || (uint32_t)seen == key) {  // placed, or present: the first value stays
@@ -259,15 +302,37 @@ __global__ void __launch_bounds__(REGION_THREADS, 3)
             }
         }
         __syncthreads();
-        if (!direct) {
 #pragma unroll
-            for (uint32_t i = 0; i < REGION / 2 / REGION_THREADS; ++i)
-                mem[i * REGION_THREADS + tid] = copy[i * REGION_THREADS + tid];
-        }
+        for (uint32_t i = 0; i < REGION / 2 / REGION_THREADS; ++i)
+            mem[i * REGION_THREADS + tid] = copy[i * REGION_THREADS + tid];
         __syncthreads();
     }
     added = __reduce_add_sync(dev::FULL_MASK, added);
-    if (lane == 0 && added != 0) atomicAdd(&counters[0], added);
+    if (lane == 0 && added != 0) atomicAdd(&t.outcome->added, added);
+}
+
+// The direct inserts: the pairs that left their region, then the regions left whole.
+__global__ void __launch_bounds__(THREADS)
+    k_map_insert_rest(const uint32_t* __restrict__ hashed, const uint32_t* __restrict__ values, int rotate,
+                      const uint32_t* __restrict__ first, Table t, Rest rest)
+{
+    const uint32_t stride = gridDim.x * THREADS;
+    const uint32_t n = rest.count[0], whole = rest.count[1];
+    for (uint32_t i0 = blockIdx.x * THREADS; i0 < n; i0 += stride) {
+        const uint32_t i = i0 + threadIdx.x;
+        const Found f = i < n ? insert_pair(t, rest.keys[i], rest.values[i]) : Found::nothing;
+        count_found(&t.outcome->added, f, Found::added);
+        count_found(&t.outcome->failed, f, Found::full);
+    }
+    for (uint32_t w = 0; w < whole; ++w) {
+        const uint32_t r = rest.regions[w], e = first[r + 1];
+        for (uint32_t i0 = first[r] + (blockIdx.x + w) % gridDim.x * THREADS; i0 < e; i0 += stride) {
+            const uint32_t i = i0 + threadIdx.x, x = i < e ? hashed[i] : 0u;
+            const Found f = i < e ? insert_pair(t, undo_fmix32(__funnelshift_r(x, x, rotate)), values[i]) : Found::nothing;
+            count_found(&t.outcome->added, f, Found::added);
+            count_found(&t.outcome->failed, f, Found::full);
+        }
+    }
 }
 
 // The slot holding key, or mask + 1 when absent (the walk ends at an empty slot).
@@ -329,27 +394,28 @@ int grid(device_context& ctx, uint64_t work)
 constexpr std::size_t REGION_MIN_SLOTS = std::size_t(1) << 25, REGION_MAX_SLOTS = std::size_t(REGION) << 16;
 
 // Enqueues the insert by regions; false when there is no memory for its scratch.
-bool insert_by_regions(device_context& ctx, unsigned long long* slots, std::size_t capacity, uint32_t empty_key,
-                       uint32_t empty_value, const uint32_t* keys, const uint32_t* values, uint32_t n,
-                       unsigned int* counters)
+bool insert_by_regions(device_context& ctx, const Table& t, std::size_t capacity, const uint32_t* keys, const uint32_t* values,
+                       uint32_t n)
 {
     int bits = 0;
     while ((std::size_t(1) << bits) < capacity) ++bits;
     const int rotate = 32 - bits, shift = 32 - (bits - (int)REGION_BITS);
     const uint32_t regions = (uint32_t)(capacity / REGION);
     const std::size_t words = ((std::size_t)n + 63) / 64 * 64;
+    const std::size_t whole = (n / REGION_PAIRS + 63) / 64 * 64;
     std::unique_ptr<temp_buffer> scratch;
     try {
-        scratch = std::make_unique<temp_buffer>(ctx.resource, (4 * words + regions + 64) * 4 + sizeof(onesweep::SortControl));
+        scratch = std::make_unique<temp_buffer>(ctx.resource,
+                                                (4 * words + regions + 64 + whole) * 4 + sizeof(onesweep::SortControl));
     } catch (const out_of_memory&) {
         return false;
     }
     uint32_t* hashed = scratch->as<uint32_t>();
     uint32_t *alt_hashed = hashed + words, *ordered = hashed + 2 * words, *alt_values = hashed + 3 * words;
-    uint32_t* first = hashed + 4 * words;  // regions + 1, then the rest's count
-    uint32_t* rest_count = first + regions + 1;
-    auto* ctl = reinterpret_cast<onesweep::SortControl*>(first + regions + 64);
-    check_cuda(cudaMemsetAsync(rest_count, 0, 4, ctx.stream), "cudaMemsetAsync");
+    uint32_t* first = hashed + 4 * words;  // regions + 1, then the rest's two counts
+    Rest rest{alt_hashed, alt_values, first + regions + 1, first + regions + 64};
+    auto* ctl = reinterpret_cast<onesweep::SortControl*>(rest.regions + whole);
+    check_cuda(cudaMemsetAsync(rest.count, 0, 8, ctx.stream), "cudaMemsetAsync");
     check_cuda(cudaMemsetAsync(ctl, 0, sizeof(onesweep::SortControl), ctx.stream), "cudaMemsetAsync");
     {
         kernel_timer kt(ctx, "static_map.hash");
@@ -365,15 +431,13 @@ bool insert_by_regions(device_context& ctx, unsigned long long* slots, std::size
             check_cuda(cudaFuncSetAttribute(&k_map_fill_regions, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                        "cudaFuncSetAttribute");
         // the ordered pairs are read, so the passes' other buffers take the rest
-        k_map_fill_regions<<<ctx.sm_count * 3, REGION_THREADS, smem, ctx.stream>>>(
-            hashed, ordered, rotate, first, regions, slots, empty_key, empty_value, counters, alt_hashed, alt_values,
-            rest_count);
+        k_map_fill_regions<<<ctx.sm_count * 3, REGION_THREADS, smem, ctx.stream>>>(hashed, ordered, rotate, first, regions, t,
+                                                                                   rest);
         check_cuda(cudaGetLastError(), "static_map region launch");
     }
     {
         kernel_timer kt(ctx, "static_map.insert");
-        k_map_insert<<<grid(ctx, n), THREADS, 0, ctx.stream>>>(alt_hashed, alt_values, n, slots, (uint32_t)(capacity - 1),
-                                                             empty_key, empty_value, counters, rest_count);
+        k_map_insert_rest<<<grid(ctx, n), THREADS, 0, ctx.stream>>>(hashed, ordered, rotate, first, t, rest);
         check_cuda(cudaGetLastError(), "static_map insert launch");
     }
     return true;
@@ -410,29 +474,44 @@ std::size_t static_map_insert(device_context& ctx, void* slots, std::size_t capa
     check_size(n);
     if (keys == nullptr || values == nullptr) throw std::invalid_argument("static_map::insert: null keys or values");
     ctx.activate();
-    unsigned int* counters = reinterpret_cast<unsigned int*>(ctx.d_small);
-    check_cuda(cudaMemsetAsync(counters, 0, 8, ctx.stream), "cudaMemsetAsync");
+    auto* o = reinterpret_cast<Outcome*>(ctx.d_small);
+    check_cuda(cudaMemsetAsync(o, 0, sizeof(Outcome), ctx.stream), "cudaMemsetAsync");
+    const Table t{static_cast<unsigned long long*>(slots), (uint32_t)(capacity - 1), empty_key, empty_value, o};
     // By regions where the table is larger than L2 and the keys are dense in
     // it (a region is read and written whole for its share of the keys):
     // into 2^26 slots, directly and by regions, capacity / 16 keys 0.29 / 0.31
-    // ms, / 8 0.57 / 0.36, / 2 2.43 / 0.96.
-    bool done = false;
-    if (capacity >= REGION_MIN_SLOTS && capacity <= REGION_MAX_SLOTS && n >= capacity / 8)
-        done = insert_by_regions(ctx, static_cast<unsigned long long*>(slots), capacity, empty_key, empty_value, keys, values,
-                                 (uint32_t)n, counters);
-    if (!done) {
+    // ms, / 8 0.57 / 0.36, / 2 2.43 / 0.96; and where enough of them are distinct,
+    // which the host learns with the direct insert's counts.
+    const bool dense = capacity >= REGION_MIN_SLOTS && capacity <= REGION_MAX_SLOTS && n >= capacity / 8;
+    const uint32_t least = (uint32_t)(capacity / DISTINCT_SHARE);
+    auto* h = static_cast<Outcome*>(ctx.pinned);
+    auto read = [&] {
+        check_cuda(cudaMemcpyAsync(h, o, sizeof(Outcome), cudaMemcpyDeviceToHost, ctx.stream), "cudaMemcpyAsync");
+        check_cuda(cudaStreamSynchronize(ctx.stream), "cudaStreamSynchronize");
+    };
+    auto direct = [&](auto kernel) {
         kernel_timer kt(ctx, "static_map.insert");
-        k_map_insert<<<grid(ctx, n), THREADS, 0, ctx.stream>>>(keys, values, (uint32_t)n,
-                                                             static_cast<unsigned long long*>(slots),
-                                                             (uint32_t)(capacity - 1), empty_key, empty_value,
-                                                             counters, nullptr);
+        launch_chained(kernel, grid(ctx, n), THREADS, 0, ctx.stream, keys, values, (uint32_t)n, t, least);
         check_cuda(cudaGetLastError(), "static_map insert launch");
+    };
+    if (dense) {
+        {
+            kernel_timer kt(ctx, "static_map.sample");
+            k_map_sample<<<SAMPLE / THREADS, THREADS, 0, ctx.stream>>>(keys, values, (uint32_t)n, t);
+            check_cuda(cudaGetLastError(), "static_map sample launch");
+        }
+        direct(&k_map_insert<true>);
+        read();
+        if (mostly_distinct(h->met, least)) {
+            if (!insert_by_regions(ctx, t, capacity, keys, values, (uint32_t)n)) direct(&k_map_insert<false>);
+            read();
+        }
+    } else {
+        direct(&k_map_insert<false>);
+        read();
     }
-    unsigned int* h = static_cast<unsigned int*>(ctx.pinned);
-    check_cuda(cudaMemcpyAsync(h, counters, 8, cudaMemcpyDeviceToHost, ctx.stream), "cudaMemcpyAsync");
-    check_cuda(cudaStreamSynchronize(ctx.stream), "cudaStreamSynchronize");
-    not_placed = h[1];
-    return h[0];
+    not_placed = h->failed;
+    return h->added;
 }
 
 void static_map_find(device_context& ctx, const void* slots, std::size_t capacity, uint32_t empty_key,
