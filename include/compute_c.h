@@ -408,7 +408,9 @@ GBC_EXPORT clc_status clc_bitpack_deserialize(clc_context ctx, const void* blob,
  *
  * clc_map_insert blocks and reports how many keys were new; a full table
  * returns CLC_ERROR_OUT_OF_MEMORY ("table is full", as the reference throws
- * std::overflow_error) after inserting what fits. find/contains run
+ * std::overflow_error) after inserting what fits; inserts into one map from
+ * several threads, each with a context of its own, run one after another.
+ * find/contains run
  * asynchronously on the context's stream and see every earlier insert;
  * found[i] is a byte, 1 when keys[i] is present. clc_map_slots copies the
  * table into separate slot-key and slot-value arrays (either may be NULL),

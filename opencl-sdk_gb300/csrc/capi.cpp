@@ -55,6 +55,10 @@ struct clc_map_s {
     std::size_t capacity;
     uint32_t empty_key, empty_value;
     std::size_t size;
+    // An insert by regions writes whole regions back, so what another insert puts
+    // there meanwhile would be lost: inserts into one map, which block anyway,
+    // exclude each other, whichever contexts they run on.
+    std::mutex m;
 };
 
 struct clc_graph_s {
@@ -1302,7 +1306,7 @@ clc_status clc_map_create(clc_context ctx, size_t capacity, uint32_t empty_key, 
         const std::size_t slots = gbc::static_map_slots(std::max<std::size_t>(capacity, 2));
         ctx->ctx->activate();
         std::unique_ptr<clc_map_s> m(
-            new clc_map_s{ctx->ctx->resource, ctx->ctx->holder, nullptr, slots, empty_key, empty_value, 0});
+            new clc_map_s{ctx->ctx->resource, ctx->ctx->holder, nullptr, slots, empty_key, empty_value, 0, {}});
         m->slots = m->resource->allocate(slots * 8);
         try {
             gbc::static_map_clear(*ctx->ctx, m->slots, slots, empty_key, empty_value);
@@ -1325,7 +1329,10 @@ void clc_map_release(clc_map map)
 clc_status clc_map_info(clc_map map, size_t* size, size_t* capacity, uint32_t* empty_key, uint32_t* empty_value)
 {
     if (map == nullptr) return fail(CLC_ERROR_INVALID_ARGUMENT, "clc: null map");
-    if (size != nullptr) *size = map->size;
+    if (size != nullptr) {
+        std::lock_guard<std::mutex> lock(map->m);
+        *size = map->size;
+    }
     if (capacity != nullptr) *capacity = map->capacity;
     if (empty_key != nullptr) *empty_key = map->empty_key;
     if (empty_value != nullptr) *empty_value = map->empty_value;
@@ -1337,6 +1344,7 @@ clc_status clc_map_clear(clc_context ctx, clc_map map)
     return guarded([&] {
         require(ctx != nullptr && map != nullptr, "clc: null argument");
         require(map->holder->device == ctx->ctx->device, "clc: map belongs to another device");
+        std::lock_guard<std::mutex> lock(map->m);
         gbc::static_map_clear(*ctx->ctx, map->slots, map->capacity, map->empty_key, map->empty_value);
         map->size = 0;
     });
@@ -1350,6 +1358,7 @@ clc_status clc_map_insert_raw(clc_context ctx, clc_map map, const uint32_t* keys
         require(ctx != nullptr && map != nullptr, "clc: null argument");
         require(map->holder->device == ctx->ctx->device, "clc: map belongs to another device");
         std::size_t not_placed = 0;
+        std::lock_guard<std::mutex> lock(map->m);
         const std::size_t added = gbc::static_map_insert(*ctx->ctx, map->slots, map->capacity, map->empty_key,
                                                          map->empty_value, keys, values, n, not_placed);
         map->size += added;
