@@ -192,7 +192,11 @@ template <typename K, int TILE> __device__ __forceinline__ void seg_classify(con
     }
 }
 
-template <typename K, int TILE> __global__ void k_seg_classify(SegArgs<K> a) { seg_classify<K, TILE>(a); }
+template <typename K, int TILE> __global__ void k_seg_classify(SegArgs<K> a)
+{
+    dev::chain();
+    seg_classify<K, TILE>(a);
+}
 
 // The tile -> segment map (a warp of the first `ctas` CTAs per large segment),
 // and zeros in the histogram rows of the large segments present.
@@ -1094,9 +1098,11 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
         check_cuda(cudaGetLastError(), "segmented sort classify launch");
     }
     // Fork: the large-segment path runs on the auxiliary stream.
-    cudaStream_t aux = ctx.aux_stream();
-    check_cuda(cudaEventRecord(ctx.fork_event, ctx.stream), "cudaEventRecord");
-    check_cuda(cudaStreamWaitEvent(aux, ctx.fork_event, 0), "cudaStreamWaitEvent");
+    cudaStream_t aux = opt.sparse ? ctx.stream : ctx.aux_stream();
+    if (!opt.sparse) {
+        check_cuda(cudaEventRecord(ctx.fork_event, ctx.stream), "cudaEventRecord");
+        check_cuda(cudaStreamWaitEvent(aux, ctx.fork_event, 0), "cudaStreamWaitEvent");
+    }
 
     {
         kernel_timer kt(ctx, "segsort.small_warp");
@@ -1109,7 +1115,7 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
     }
     {
         kernel_timer kt(ctx, "segsort.small_cta");
-        launch_cta_sorts<K, HAS_V>(ctx, a, false, cta_cap, n, opt.cta_threads, ctx.stream);
+        launch_cta_sorts<K, HAS_V>(ctx, a, false, cta_cap, opt.sparse ? VERY_FEW_KEYS : n, opt.cta_threads, ctx.stream);
     }
     if (maybe_large) {
         {
@@ -1145,7 +1151,9 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
         }
         auto pk = &k_seg_large_pass<K, HAS_V, LS::THREADS, LS::ITEMS, LS::MINB, LS::LBW, false>;
         const int pgrid = pass_grid(pk);
-        for (int s = 0; s < P; ++s) {
+        // an even number of passes left out, so that the last one writes the output
+        const int passes = opt.low_digits > 0 ? std::min(P, (opt.low_digits + 1) / 2 * 2) : P;
+        for (int s = 0; s < passes; ++s) {
             kernel_timer kt(ctx, "segsort.large_pass", aux);
             launch_chained(pk, pgrid, LS::THREADS, psmem, aux, a, s, msd);
             check_cuda(cudaGetLastError(), "segmented sort pass launch");
@@ -1161,9 +1169,10 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
             launch_cta_sorts<K, HAS_V>(ctx, a, true, msd_cap, n, opt.cta_threads, aux);
         }
     }
-    // Join.
-    check_cuda(cudaEventRecord(ctx.join_event, aux), "cudaEventRecord");
-    check_cuda(cudaStreamWaitEvent(ctx.stream, ctx.join_event, 0), "cudaStreamWaitEvent");
+    if (!opt.sparse) {  // join
+        check_cuda(cudaEventRecord(ctx.join_event, aux), "cudaEventRecord");
+        check_cuda(cudaStreamWaitEvent(ctx.stream, ctx.join_event, 0), "cudaStreamWaitEvent");
+    }
 }
 
 }  // namespace seg

@@ -29,6 +29,12 @@ struct seg_options {
     // "segsort:cta_threads" entry, else 256. The longer classes have 512 or
     // 1,024 threads.
     int cta_threads = 0;
+    // the keys of a segment differ in this many of their lowest 8-bit digits at
+    // most (0: in any); the passes over the others are not launched
+    int low_digits = 0;
+    // few launches, all on the context's stream: for calls that mostly have
+    // little to do or nothing
+    bool sparse = false;
     // scratch of the call's n keys (and values), or null: from the context's arena
     void* alt_keys = nullptr;
     uint32_t* alt_vals = nullptr;

@@ -1241,12 +1241,11 @@ static void run_sort(device_context& ctx, const K* in_k, K* out_k, const uint32_
     a.chunks = 0;
     a.tiles_per_chunk = 0;
 
-    run_upfront<K>(ctx, a);
-
     // The leading digits only, where that is enough (sort_partial.cuh).
     if constexpr (sizeof(K) == 8) {
         if (n >= partial::MIN_KEYS && run_partial<K, HAS_V>(ctx, a, pv)) return;
     }
+    run_upfront<K>(ctx, a);
     run_passes<K, HAS_V>(ctx, a, pv, P, true);
 }
 
@@ -1311,9 +1310,9 @@ static void run_passes(device_context& ctx, SortArgs<K> a, const PassVariant<K>&
     }
 }
 
-// After the upfront histogram: the fewest leading digits that leave little out
-// of order, their passes, and the repair of what they leave.
-// False, with nothing enqueued, when there is no memory for its tables.
+// The digit counts, the fewest leading digits that leave little out of order,
+// their passes, and the repair of what they leave. False, with nothing enqueued,
+// when there is no memory for its tables.
 template <typename K, bool HAS_V> static bool run_partial(device_context& ctx, const SortArgs<K>& a, const PassVariant<K>& pv)
 {
     using namespace partial;
@@ -1322,28 +1321,25 @@ template <typename K, bool HAS_V> static bool run_partial(device_context& ctx, c
     const bool segmented = n >= SEGMENTED_KEYS;
     int bits = 0;
     while ((std::size_t(1) << bits) < n) ++bits;
-    // one block: the control words and the plan of all digits (zeroed), then
-    // the tables and the set (all ones), then the lists
-    const std::size_t zeroed = 256 + sizeof(SortControl);
+    // the control words, the plan of all digits, the tables and the set (all zeroed); the lists
     const uint32_t sample = sample_size(n);
-    const std::size_t ones = (std::size_t)CANDIDATES * 2 * sample * 8 + LONG_SET * 4;
+    const std::size_t zeroed = 256 + sizeof(SortControl) + (std::size_t)CANDIDATES * 2 * sample * 8 + LONG_SET * 4;
+    static_assert(sizeof(Control) <= 256 && sizeof(SortControl) % 8 == 0, "the tables are 8-byte aligned");
     const std::size_t max_faults = (n + FT_TILE - 1) / FT_TILE + 1;
-    std::unique_ptr<temp_buffer> head_b, sets_b, lists_b;
+    std::unique_ptr<temp_buffer> zeroed_b, lists_b;
     try {
-        head_b = std::make_unique<temp_buffer>(ctx.resource, zeroed);
-        sets_b = std::make_unique<temp_buffer>(ctx.resource, ones);
-        lists_b = std::make_unique<temp_buffer>(ctx.resource, (4 * (std::size_t)MAX_LONG + max_faults) * sizeof(uint32_t) + SEGMENTS);
+        zeroed_b = std::make_unique<temp_buffer>(ctx.resource, zeroed);
+        lists_b = std::make_unique<temp_buffer>(ctx.resource, (4 * (std::size_t)MAX_LONG + max_faults) * sizeof(uint32_t) + 2 * MAX_LONG);
     } catch (const out_of_memory&) {
         return false;
     }
-    temp_buffer &head = *head_b, &sets = *sets_b, &lists = *lists_b;
+    temp_buffer &head = *zeroed_b, &lists = *lists_b;
     check_cuda(cudaMemsetAsync(head.get(), 0, zeroed, ctx.stream), "cudaMemsetAsync");
-    check_cuda(cudaMemsetAsync(sets.get(), 0xFF, ones, ctx.stream), "cudaMemsetAsync");
     Args<K> p;
     p.a = a;
     p.ctl = head.as<Control>();
     p.all = reinterpret_cast<SortControl*>(head.as<unsigned char>() + 256);
-    p.tables = sets.as<unsigned long long>();
+    p.tables = reinterpret_cast<unsigned long long*>(p.all + 1);
     p.sample = sample;
     p.segmented = segmented;
     p.set = reinterpret_cast<uint32_t*>(p.tables + (std::size_t)CANDIDATES * 2 * sample);
@@ -1352,11 +1348,11 @@ template <typename K, bool HAS_V> static bool run_partial(device_context& ctx, c
     p.end = p.begin + MAX_LONG;
     p.off = p.end + MAX_LONG;
     p.fault = p.off + 2 * MAX_LONG;
-    uint8_t* skip = reinterpret_cast<uint8_t*>(p.fault + max_faults);
+    uint32_t* skip = p.fault + max_faults;
+    run_upfront<K>(ctx, a);
     {
         kernel_timer kt(ctx, "sort.sample");
-        k_sample<K><<<sample / 256, 256, 0, ctx.stream>>>(p);
-        if (segmented) k_odd_segments<<<(SEGMENTS + 255) / 256, 256, 0, ctx.stream>>>(skip, SEGMENTS);
+        launch_chained(&k_sample<K>, (int)(sample / 256), 256, 0, ctx.stream, p);
         check_cuda(cudaGetLastError(), "radix sort sample launch");
     }
     run_passes<K, HAS_V>(ctx, a, pv, FIRST_PASSES, true);
@@ -1369,12 +1365,12 @@ template <typename K, bool HAS_V> static bool run_partial(device_context& ctx, c
     }
     {
         kernel_timer kt(ctx, "sort.repair");
-        launch_chained(&k_repair<K, HAS_V>, std::max<int>(1, std::min<int>((int)(max_faults / 256), ctx.sm_count * 2)), 256, 0,
-                       ctx.stream, p);
         if (segmented) {
+            launch_chained(&k_repair<K, HAS_V>, std::min<int>((int)(max_faults / 8), ctx.sm_count * 4), 256, 0, ctx.stream, p);
             const std::size_t smem = tile::Sorter<uint32_t, true, 1024, MAX_LONG / 1024>::SMEM;
             prepare_kernel(&k_long_runs, 1024, smem, g_occupancy, g_occupancy_mutex);
-            launch_chained(&k_long_runs, 1, 1024, smem, ctx.stream, p.ctl, p.all, p.begin, p.end, p.off, a.n, ctx.d_error);
+            launch_chained(&k_long_runs, 1, 1024, smem, ctx.stream, p.ctl, p.all, p.begin, p.end, p.off, skip, a.n,
+                           ctx.d_error);
         } else {
             const std::size_t smem = tile::Sorter<K, HAS_V, 512, 16>::SMEM;
             prepare_kernel(&k_sort_long_runs<K, HAS_V>, 512, smem, g_occupancy, g_occupancy_mutex);
@@ -1391,9 +1387,12 @@ template <typename K, bool HAS_V> static bool run_partial(device_context& ctx, c
     bool copy = false;  // that plan has all passes, an even number, or none
     if (segmented) {
         seg_options so;
-        so.skip = skip;
+        so.skip = reinterpret_cast<const uint8_t*>(skip);
+        so.sparse = true;
         so.cta_threads = 256;
-        so.msd_cap = (int)segsort_cta_cap(sizeof(K), HAS_V);
+        so.msd_cap = 0;
+        // a run's keys agree in `least` digits or more, and so differ in the others' positions only
+        so.low_digits = Traits<K>::PASSES - p.least;
         so.alt_keys = a.alt_keys;
         so.alt_vals = a.alt_vals;
         try {
