@@ -484,6 +484,9 @@ GBC_EXPORT clc_status clc_selftest_noalloc_timeout(int32_t* buf, size_t n, void*
  * call reports: CLC_ERROR_OPENCL with a "timed out" message. The context
  * stays usable. */
 GBC_EXPORT clc_status clc_selftest_lookback_timeout(clc_context ctx);
+/* The same for a pass of the batched sort given places outside its segment:
+ * it writes nothing there, and CLC_ERROR_OPENCL is returned. */
+GBC_EXPORT clc_status clc_selftest_misplaced(clc_context ctx);
 
 /* Profiling: when enabled, every kernel launch is bracketed by CUDA events on
  * the context's stream and its time accumulated per kernel family

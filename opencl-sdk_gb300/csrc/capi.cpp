@@ -1014,6 +1014,15 @@ clc_status clc_selftest_lookback_timeout(clc_context ctx)
     });
 }
 
+clc_status clc_selftest_misplaced(clc_context ctx)
+{
+    if (ctx == nullptr) return fail(CLC_ERROR_INVALID_ARGUMENT, "clc: null context");
+    return guarded([&] {
+        gbc::selftest_misplaced(*ctx->ctx);
+        ctx->ctx->finish();
+    });
+}
+
 // ---- profiling ------------------------------------------------------------
 
 clc_status clc_profile_enable(clc_context ctx, int enable)

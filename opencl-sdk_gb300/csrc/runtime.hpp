@@ -295,6 +295,7 @@ void static_map_unzip(device_context& ctx, const void* slots, std::size_t capaci
 //! Launches one scan tile whose predecessor never publishes (the failure
 //! path of the bounded look-back wait); the next finish() reports it.
 void selftest_lookback_timeout(device_context& ctx);
+void selftest_misplaced(device_context& ctx);
 
 //! Records a clc_status and message as the calling thread's last error (for
 //! C entry points defined outside capi.cpp); returns the status.

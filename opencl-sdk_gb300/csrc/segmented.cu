@@ -29,6 +29,7 @@
 #include <mutex>
 #include <string>
 #include <tuple>
+#include <vector>
 
 #include "device_common.cuh"
 #include "runtime.hpp"
@@ -884,6 +885,7 @@ __device__ __forceinline__ void seg_large_pass(const SegArgs<K>& a, int slot, bo
         }
         __syncthreads();
         const uint32_t limit = s_abort ? 0u : valid;
+        bool outside = false;  // a place outside the segment: nothing is written there, and the call fails
         if (limit == (uint32_t)TILE) {
             uint32_t o[ITEMS];
 #pragma unroll
@@ -899,6 +901,8 @@ __device__ __forceinline__ void seg_large_pass(const SegArgs<K>& a, int slot, bo
                 if (o[i] >= segb && o[i] < sege) {
                     dst_k[o[i]] = key[i];
                     if (HAS_V) dst_v[o[i]] = val[i];
+                } else {
+                    outside = true;
                 }
             }
         } else {
@@ -908,9 +912,12 @@ __device__ __forceinline__ void seg_large_pass(const SegArgs<K>& a, int slot, bo
                 if (o >= segb && o < sege) {
                     dst_k[o] = kk;
                     if (HAS_V) dst_v[o] = s_vals[q];
+                } else {
+                    outside = true;
                 }
             }
         }
+        if (outside) dev::raise_error(a.err, dev::ERR_MISPLACED);
         __syncthreads();
     }
 }
@@ -1176,6 +1183,47 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
 }
 
 }  // namespace seg
+
+void selftest_misplaced(device_context& ctx)
+{
+    // One segment of equal keys, whose bin starts lie just past its end: the
+    // large pass must write none of them and record the error.
+    using namespace seg;
+    using LS = LargeShape<uint32_t, false>;
+    constexpr uint32_t N = 1000, P = Traits<uint32_t>::PASSES;
+    constexpr std::size_t smem =
+        (std::size_t)(LS::THREADS / 32) * (RADIX + LARGE_PAD) * 8 + (std::size_t)LS::THREADS * LS::ITEMS * sizeof(uint32_t);
+    ctx.activate();
+    // the keys and the two other arrays; the segment's offsets; its index, first tile and tile; the bin starts
+    std::vector<uint32_t> host(3 * N, 0u);
+    host.insert(host.end(), {0u, N, 0u, 0u, 0u});
+    host.resize(host.size() + P * RADIX, N);
+    SegControl control{};
+    control.n_large = control.large_tiles = 1;
+    temp_buffer words(ctx.resource, host.size() * 4), ctl(ctx.resource, sizeof(SegControl));
+    check_cuda(cudaMemcpyAsync(words.get(), host.data(), host.size() * 4, cudaMemcpyHostToDevice, ctx.stream), "cudaMemcpyAsync");
+    check_cuda(cudaMemcpyAsync(ctl.get(), &control, sizeof(control), cudaMemcpyHostToDevice, ctx.stream), "cudaMemcpyAsync");
+    SegArgs<uint32_t> a{};
+    uint32_t* w = words.as<uint32_t>();
+    a.in_k = w;
+    a.out_k = w + N;
+    a.alt_k = w + 2 * N;
+    a.off = w + 3 * N;
+    a.large_list = w + 3 * N + 2;
+    a.tile_begin = a.lsd_begin = w + 3 * N + 3;
+    a.tile_seg = a.lsd_seg = w + 3 * N + 4;
+    a.seg_hist = w + 3 * N + 5;
+    a.nseg = a.max_large = a.max_tiles = 1;
+    a.ctl = ctl.as<SegControl>();
+    a.ring = ctx.lookback_ring;
+    a.seq0 = ctx.reserve_seq(P + 1);
+    a.err = ctx.d_error;
+    auto kernel = &k_seg_large_pass<uint32_t, false, LS::THREADS, LS::ITEMS, LS::MINB, LS::LBW, false>;
+    occupancy(kernel, LS::THREADS, smem);  // opts in to the shared memory
+    kernel<<<1, LS::THREADS, smem, ctx.stream>>>(a, 0, false);
+    check_cuda(cudaGetLastError(), "segmented sort pass launch");
+    check_cuda(cudaStreamSynchronize(ctx.stream), "cudaStreamSynchronize");  // the host's copies are read
+}
 
 uint32_t segsort_cta_cap(int key_bytes, bool has_values)
 {

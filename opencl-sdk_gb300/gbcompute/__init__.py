@@ -223,6 +223,7 @@ _PROTOS = {
     "clc_scan_i32_noalloc_status": (_i, [_vp]),
     "clc_selftest_noalloc_timeout": (_i, [_vp, _sz, _vp]),
     "clc_selftest_lookback_timeout": (_i, [_vp]),
+    "clc_selftest_misplaced": (_i, [_vp]),
     "clc_profile_enable": (_i, [_vp, _i]),
     "clc_profile_reset": (_i, [_vp]),
     "clc_profile_count": (_i, [_vp, C.POINTER(_sz)]),
