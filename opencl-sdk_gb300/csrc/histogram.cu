@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(THREADS)
                 ACC lower, ACC upper, int offset)
 {
     constexpr int VEC = 16 / sizeof(T);
-    extern __shared__ uint32_t sh[];
+    extern __shared__ __align__(16) uint32_t sh[];
     const uint32_t copies = MODE == 0 ? WARPS : 1;
     if (MODE != 2) {
         for (uint32_t i = threadIdx.x; i < bins * copies; i += THREADS) sh[i] = 0;
@@ -133,7 +133,7 @@ constexpr std::size_t PAIR_MIN = std::size_t(1) << 28;
 template <typename T> __global__ void __launch_bounds__(PAIR_THREADS, 1)
     k_histogram_pairs(const T* __restrict__ in, uint32_t n, uint32_t* __restrict__ hist, uint32_t bins, float lower, float upper)
 {
-    extern __shared__ uint32_t sh[];  // pair (a, b): half b / 128 of word (b % 128) * 256 + a
+    extern __shared__ __align__(16) uint32_t sh[];  // pair (a, b): half b / 128 of word (b % 128) * 256 + a
     __shared__ uint32_t s_value[256], s_sum, s_most;
     const int tid = threadIdx.x, warp = tid >> 5;
     const uint4* vin = reinterpret_cast<const uint4*>(in);

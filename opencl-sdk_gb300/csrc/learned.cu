@@ -188,7 +188,7 @@ struct TrainArgs {
 
 __global__ void __launch_bounds__(TRAIN_THREADS, 1) k_train(TrainArgs a)
 {
-    extern __shared__ float sm[];
+    extern __shared__ __align__(16) float sm[];
     float* p = sm;              // this CTA's copy of the raw parameters
     float* am = p + NPARAM;     // Adam first moment
     float* as = am + NPARAM;    // Adam second moment
@@ -633,7 +633,7 @@ __device__ __forceinline__ Bucketer load_bucketer(const PartArgs& a, uint32_t* s
 
 __global__ void __launch_bounds__(PART_THREADS, 1) k_count(PartArgs a)
 {
-    extern __shared__ uint32_t sh[];
+    extern __shared__ __align__(16) uint32_t sh[];
     uint32_t* hist = sh;  // buckets
     for (uint32_t i = threadIdx.x; i < a.buckets; i += PART_THREADS) hist[i] = 0;
     const Bucketer bk = load_bucketer(a, sh);
@@ -723,7 +723,7 @@ __global__ void __launch_bounds__(T, 1024 / T) k_partition_buckets(PartArgs a, c
                                                                 uint32_t* __restrict__ dst,
                                                                 uint32_t* __restrict__ cursor)
 {
-    extern __shared__ uint32_t sh[];
+    extern __shared__ __align__(16) uint32_t sh[];
     constexpr uint32_t PER = PART_ITEMS * T;
     constexpr uint32_t NONE = 0xFFFFFFFFu;
     constexpr uint32_t PART_RANGE = 2 * T;  // two range entries per thread
@@ -834,7 +834,7 @@ __global__ void __launch_bounds__(T, 1024 / T) k_partition_groups(PartArgs a, ui
                                                                uint16_t* __restrict__ dst_ids,
                                                                uint32_t* __restrict__ cursor)
 {
-    extern __shared__ uint32_t sh[];
+    extern __shared__ __align__(16) uint32_t sh[];
     constexpr uint32_t PER = PART_ITEMS * T;
     constexpr uint32_t NONE = 0xFFFFFFFFu;
     uint32_t* hist = sh;                                       // [groups]: counts, then chunk offsets
@@ -1031,7 +1031,7 @@ __global__ void __launch_bounds__(PART_THREADS) k_bucket_ids(const K* __restrict
                                                              const uint16_t* __restrict__ glut, uint32_t buckets,
                                                              uint32_t* __restrict__ ids, uint32_t* __restrict__ idx)
 {
-    extern __shared__ uint32_t sh[];
+    extern __shared__ __align__(16) uint32_t sh[];
     uint32_t* sp = sh;
     uint16_t* lut = reinterpret_cast<uint16_t*>(sp + (buckets - 1));
     for (uint32_t i = threadIdx.x; i + 1 < buckets; i += PART_THREADS) sp[i] = gsp[i];
