@@ -1047,6 +1047,7 @@ template <typename K> struct PassVariant {
     void (*hist_ident)(SortArgs<K>, int) = nullptr;
 };
 
+// Saved tuning tables name a shape by its index here (see tuning_table::load).
 template <typename K, bool HAS_V> struct Variants;
 
 // sort_default_variant picks the shape when the tuning table has no entry:
