@@ -1313,7 +1313,7 @@ static void run_passes(device_context& ctx, SortArgs<K> a, const PassVariant<K>&
 
 // The digit counts, the fewest leading digits that leave little out of order,
 // their passes, and the repair of what they leave. False, with nothing enqueued,
-// when there is no memory for its tables.
+// when there is no memory for its tables (or, under capture, none in the pool).
 template <typename K, bool HAS_V> static bool run_partial(device_context& ctx, const SortArgs<K>& a, const PassVariant<K>& pv)
 {
     using namespace partial;
@@ -1332,6 +1332,8 @@ template <typename K, bool HAS_V> static bool run_partial(device_context& ctx, c
         zeroed_b = std::make_unique<temp_buffer>(ctx.resource, zeroed);
         lists_b = std::make_unique<temp_buffer>(ctx.resource, (4 * (std::size_t)MAX_LONG + max_faults) * sizeof(uint32_t) + 2 * MAX_LONG);
     } catch (const out_of_memory&) {
+        return false;
+    } catch (const unsupported_error&) {
         return false;
     }
     temp_buffer &head = *zeroed_b, &lists = *lists_b;
@@ -1396,10 +1398,14 @@ template <typename K, bool HAS_V> static bool run_partial(device_context& ctx, c
         so.low_digits = Traits<K>::PASSES - p.least;
         so.alt_keys = a.alt_keys;
         so.alt_vals = a.alt_vals;
+        bool done = false;  // it takes its memory before it enqueues anything
         try {
             segmented_sort_xf(ctx, a.out_keys, a.out_vals, a.xf.a, a.xf.b, n, p.off, SEGMENTS, so);
+            done = true;
         } catch (const out_of_memory&) {
-            // it takes its memory before it enqueues anything: every digit, then
+        } catch (const unsupported_error&) {
+        }
+        if (!done) {  // every digit, then
             check_cuda(cudaMemsetAsync(p.all, 0, sizeof(SortControl), ctx.stream), "cudaMemsetAsync");
             run_upfront<K>(ctx, all);
             copy = true;
