@@ -111,36 +111,57 @@ __global__ void __launch_bounds__(THREADS)
 // A counter may wrap, and carry into its neighbour: either loses 65,535 or
 // 65,536 from the sum of all counters and nothing adds to it, so a batch whose
 // counters do not add up to its pairs is counted again, by bytes, into per-warp
-// 32-bit histograms, and so is the rest of the CTA's share. A first batch too
-// small to wrap tells whether one pair is so frequent that this is to be
-// expected (or that its atomics meet on one address).
+// 32-bit histograms, and so is the rest of the CTA's share.
+//
+// Pairs pay where a warp's words differ. Lanes with equal bytes add 1 to a counter
+// together; their pairs' additions (1 or 2^16) meet on one address one after
+// another, and so do all that meet in a bank, which the first byte chooses. So
+// the warps look at one byte per lane (all of them before the first batch, some
+// before the others), and the bytes are counted one by one from where the
+// busiest bank makes the pairs the slower way (2^30 bytes, counted singly by k_histogram / always in pairs / now: runs of 256
+// equal bytes 279 / 934 / 189 us, 16 values 279 / 336 / 189, normal with a
+// deviation of 10 279 / 279 / 244, one value 279 / 204 / 188, uniform 385 / 270 / 267).
 //
 // 2^30 uniform bytes: 384 -> 269 us (one read at the copy rate 158; loading
 // alone takes 150, the pairs' atomics 234, and with the counters' old values
 // returned, to see them wrap, 293).
 // ---------------------------------------------------------------------------
 constexpr int PAIR_THREADS = 1024, PAIR_WARPS = PAIR_THREADS / 32;
-constexpr int PAIR_FIRST = 4;    // 16-byte loads per thread in the first batch: 32,768 pairs
-constexpr int PAIR_BATCH = 64;   // and in the others: 524,288 pairs
-constexpr uint32_t PAIR_COMMON = 32768 / 10;  // a pair's count in the first batch that rules pairs out
+constexpr int PAIR_BATCH = 64;   // 16-byte loads per thread in a batch: 524,288 pairs
 constexpr std::size_t PAIR_SMEM = 32768 * 4;
 // Below, the CTAs' 128 KiB to clear and add up cost too much where the pairs are
 // given up (uniform / one value in nine places of ten / constant bytes, by
-// bytes and by pairs: 2^26 29.7 / 24.3 / 22.7 and 27.6 / 36.9 / 36.5 us; 2^28
-// 101.6 / 74.8 / 74.7 and 76.0 / 73.5 / 70.6).
+// k_histogram and here: 2^26, with a first batch in pairs always, 29.7 / 24.3 / 22.7
+// and 27.6 / 36.9 / 36.5 us; 2^28 102.6 / 75.6 / 75.9 and 74.0 / 57.8 / 53.6).
 constexpr std::size_t PAIR_MIN = std::size_t(1) << 28;
+
+// What counting the warp's lanes' bytes in pairs costs, less what it costs byte by
+// byte, in halves of an addition: those that the busiest bank takes, all of a
+// counter's pairs or (by 1, as lanes with the same counter add together) one per
+// counter, twice. An addition of 1 is about half the work of a pair's, and each
+// has about one more around it (from the times above).
+__device__ __forceinline__ int pairs_over_bytes(uint32_t byte)
+{
+    const uint32_t bank = __match_any_sync(dev::FULL_MASK, byte & 31u), same = __match_any_sync(dev::FULL_MASK, byte);
+    const uint32_t once = __ballot_sync(dev::FULL_MASK, (int)(threadIdx.x & 31) == __ffs(same) - 1);
+    const int pairs = (int)__reduce_max_sync(dev::FULL_MASK, (uint32_t)__popc(bank));
+    const int bytes = (int)__reduce_max_sync(dev::FULL_MASK, (uint32_t)__popc(bank & once));
+    return 2 * pairs - 2 * bytes - 2;
+}
 
 template <typename T> __global__ void __launch_bounds__(PAIR_THREADS, 1)
     k_histogram_pairs(const T* __restrict__ in, uint32_t n, uint32_t* __restrict__ hist, uint32_t bins, float lower, float upper)
 {
     extern __shared__ __align__(16) uint32_t sh[];  // pair (a, b): half b / 128 of word (b % 128) * 256 + a
-    __shared__ uint32_t s_value[256], s_sum, s_most;
+    __shared__ uint32_t s_value[256], s_sum;
+    __shared__ int s_cost;  // the sum of pairs_over_bytes so far
     const int tid = threadIdx.x, warp = tid >> 5;
     const uint4* vin = reinterpret_cast<const uint4*>(in);
     const uint32_t nv = n / 16;
     const uint32_t first = (uint32_t)((uint64_t)nv * blockIdx.x / gridDim.x);
     const uint32_t last = (uint32_t)((uint64_t)nv * (blockIdx.x + 1) / gridDim.x);
     if (tid < 256) s_value[tid] = 0;
+    if (tid == 0) s_cost = 0;
     auto clear = [&] {
         __syncthreads();
         for (int i = tid; i < (int)(PAIR_SMEM / 16); i += PAIR_THREADS) reinterpret_cast<uint4*>(sh)[i] = make_uint4(0, 0, 0, 0);
@@ -164,28 +185,31 @@ template <typename T> __global__ void __launch_bounds__(PAIR_THREADS, 1)
     auto pair = [&](uint32_t x) { atomicAdd(&sh[x & 0x7FFFu], x & 0x8000u ? 0x10000u : 1u); };
 
     uint32_t b = first;  // what is left of the share
-    clear();
-    for (uint32_t size = PAIR_FIRST * PAIR_THREADS; b < last; size = PAIR_BATCH * PAIR_THREADS) {
-        const uint32_t e = min(last, b + size);
+    auto look = [&](uint32_t v) { return v < last ? vin[v].x : 0u; };
+    uint32_t seen = look(b + tid);  // of the next batch, one word per thread
+    __syncthreads();
+    for (int k = 0; b < last; ++k) {
+        if ((k == 0 || warp < 8) && b + (tid | 31) < last) {  // every lane of the warp has a word
+            const int cost = pairs_over_bytes(seen & 0xFFu);
+            if ((tid & 31) == 0) atomicAdd(&s_cost, cost);
+        }
+        clear();
+        if (s_cost >= 0) break;
+        const uint32_t e = min(last, b + PAIR_BATCH * PAIR_THREADS);
+        seen = look(e + tid);
         words(b, e, [&](uint32_t w) { pair(w & 0xFFFFu), pair(w >> 16); });
-        if (tid == 0) s_sum = s_most = 0;
+        if (tid == 0) s_sum = 0;
         __syncthreads();
         // by first value: a value and a quarter of the rows per thread
-        uint32_t sum = 0, most = 0;
+        uint32_t sum = 0;
         for (int r = 0; r < 32; ++r) {
             const uint32_t w = sh[((tid >> 8) * 32 + r) * 256 + (tid & 255)];
             sum += (w & 0xFFFFu) + (w >> 16);
-            most = max(most, max(w & 0xFFFFu, w >> 16));
         }
         const uint32_t warp_sum = __reduce_add_sync(dev::FULL_MASK, sum);
-        most = __reduce_max_sync(dev::FULL_MASK, most);
-        if ((tid & 31) == 0) {
-            atomicAdd(&s_sum, warp_sum);
-            atomicMax(&s_most, most);
-        }
+        if ((tid & 31) == 0) atomicAdd(&s_sum, warp_sum);
         __syncthreads();
         if (s_sum != (e - b) * 8) break;  // a counter has wrapped: this batch again
-        const bool common = b == first && s_most > PAIR_COMMON;
         if (sum != 0) atomicAdd(&s_value[tid & 255], sum);
         // by second value: eight threads per row, 32 words each, every lane of
         // a warp in a bank of its own
@@ -206,8 +230,6 @@ template <typename T> __global__ void __launch_bounds__(PAIR_THREADS, 1)
             if (high != 0) atomicAdd(&s_value[row + 128], high);
         }
         b = e;
-        clear();
-        if (common) break;
     }
     if (b < last) {  // the rest by bytes
         clear();
