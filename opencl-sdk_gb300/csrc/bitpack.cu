@@ -19,8 +19,8 @@
 //     word counts are turned into offsets by the library's single-pass scan
 //     (the reference's scan client at Compression.cpp:178), which also
 //     yields the total size;
-//   * pack: one warp per chunk, in rounds of 1,024 elements, which fill whole
-//     words: the encoded elements go to shared memory, and each lane puts
+//   * pack: one warp per chunk or part of it, in rounds of 1,024 elements, which
+//     fill whole words: the encoded elements go to shared memory, and each lane puts
 //     together every 32nd word of the round from the elements in it (the
 //     reference ORs every element into global memory with atomics);
 //   * unpack, delta mode with a mean width of at most 26 bits: one pass. A
@@ -119,23 +119,28 @@ __global__ void __launch_bounds__(THREADS) k_bp_analyze(const uint32_t* __restri
     }
 }
 
-// One warp per chunk: the header triple and the chunk's packed words. Bound by
-// DRAM where the loads are (8 x 16 bytes per lane in flight); lane-private runs
-// of 64 elements, read 256 bytes apart, took 389 us for 2 10^8 timestamps, this
-// 223 (0.64 of the copy rate).
+// One warp per `span` elements (a chunk or a part of it, whole rounds): their packed
+// words, and with a chunk's first part its header triple. Bound by DRAM where the
+// loads are (8 x 16 bytes per lane in flight); lane-private runs of 64 elements,
+// read 256 bytes apart, took 389 us for 2 10^8 timestamps, this 223 (0.64 of the copy
+// rate).
 template <bool DELTA>
 __global__ void __launch_bounds__(THREADS) k_bp_pack(const uint32_t* __restrict__ in, uint32_t n, uint32_t chunk,
                                                      uint32_t chunks, const uint32_t* __restrict__ hdr,
-                                                     const uint32_t* __restrict__ offsets, uint32_t* __restrict__ out)
+                                                     const uint32_t* __restrict__ offsets, uint32_t* __restrict__ out,
+                                                     uint32_t span)
 {
     __shared__ __align__(16) uint32_t stage[WARPS][ROUND];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t* my = stage[warp];
     const bool vec = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
-    for (uint32_t c = blockIdx.x * WARPS + warp; c < chunks; c += gridDim.x * WARPS) {
-        const uint32_t start = c * chunk, count = min(chunk, n - start);
+    const uint32_t per_chunk = chunk / span, parts = chunks * per_chunk;  // powers of two; the last chunk's may be empty
+    for (uint32_t u = blockIdx.x * WARPS + warp; u < parts; u += gridDim.x * WARPS) {
+        const uint32_t c = u / per_chunk, part = u % per_chunk * span;  // the part's first element within the chunk
+        const uint32_t start = c * chunk, count = min(min(chunk, n - start), part + span);
+        if (part >= count) continue;
         const uint32_t base = hdr[2 * c], width = hdr[2 * c + 1], off = offsets[c];
-        if (lane == 0) {
+        if (lane == 0 && part == 0) {
             out[3 * c] = base;
             out[3 * c + 1] = width;
             out[3 * c + 2] = off;
@@ -144,8 +149,8 @@ __global__ void __launch_bounds__(THREADS) k_bp_pack(const uint32_t* __restrict_
         uint32_t* packed = out + 3 * (size_t)chunks + off;
         // x / width for x <= 32 * ROUND = 2^15: the quotient's error term stays below 1 / width
         const uint32_t inverse = (uint32_t)(((1ull << 32) + width - 1) / width);
-        uint32_t before = DELTA && start > 0 ? in[start - 1] : 0u;  // the element before the round
-        for (uint32_t r0 = 0; r0 < count; r0 += ROUND) {
+        uint32_t before = DELTA && start + part > 0 ? in[start + part - 1] : 0u;  // the element before the round
+        for (uint32_t r0 = part; r0 < count; r0 += ROUND) {
             const uint32_t rcount = min(ROUND, count - r0), i0 = start + r0 + 4 * lane;
             uint4 w[PACK_ROWS];
 #pragma unroll
@@ -295,19 +300,6 @@ __device__ __forceinline__ void decode_dispatch(uint32_t width, const uint32_t* 
     }
 }
 
-// The sum of one value per thread over the CTA, to every thread.
-__device__ __forceinline__ uint32_t cta_sum(uint32_t x, uint32_t* scratch)
-{
-    x = __reduce_add_sync(FULL_MASK, x);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = x;
-    __syncthreads();
-    uint32_t all = 0;
-#pragma unroll
-    for (int w = 0; w < UT / 32; ++w) all += scratch[w];
-    return all;
-}
-
 template <bool DELTA>
 __global__ void __launch_bounds__(UT)
     k_bp_unpack_tiles(const uint32_t* __restrict__ data, uint64_t words, uint32_t n, uint32_t chunk_shift,
@@ -315,7 +307,7 @@ __global__ void __launch_bounds__(UT)
 {
     using Sum = pipe::Aggregate<uint32_t>;
     __shared__ uint32_t s_out[UT * (UE + 1)];
-    __shared__ uint32_t s_warp[UT / 32];
+    __shared__ uint32_t s_warp[UT / 32], s_part[UT / 32];
     __shared__ uint32_t s_tile;
     uint32_t share = 0, done = 0;  // of the sums of the tiles before `done`
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -353,8 +345,24 @@ __global__ void __launch_bounds__(UT)
             for (int e = 1; e < UE; ++e) v[e] += v[e - 1];
         }
         bool abort = false;
+        uint32_t add = 0;  // to the thread's sums
         if (DELTA) {
-            const uint32_t sum = cta_sum(v[UE - 1], s_warp);
+            uint32_t inc = v[UE - 1];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(FULL_MASK, inc, o);
+                if (lane >= o) inc += y;
+            }
+            if (lane == 31) s_warp[warp] = inc;
+            __syncthreads();
+            uint32_t sum = 0;
+            add = inc - v[UE - 1];
+#pragma unroll
+            for (int w = 0; w < UT / 32; ++w) {
+                const uint32_t x = s_warp[w];
+                if (w < warp) add += x;
+                sum += x;
+            }
             if (tid == 0) Sum::publish(tiles.ring, tiles.seq0 + t, sum);
             for (uint32_t k = done + tid; k < t; k += UT) {
                 uint32_t x;
@@ -373,25 +381,17 @@ __global__ void __launch_bounds__(UT)
                 share += x;
             }
             done = t;
-            const uint32_t before = cta_sum(share, s_warp);
-            uint32_t inc = v[UE - 1];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(FULL_MASK, inc, o);
-                if (lane >= o) inc += y;
-            }
-            __syncthreads();
-            if (lane == 31) s_warp[warp] = inc;
-            __syncthreads();
-            uint32_t add = before + inc - v[UE - 1];
-#pragma unroll
-            for (int w = 0; w < UT / 32; ++w)
-                if (w < warp) add += s_warp[w];
-#pragma unroll
-            for (int e = 0; e < UE; ++e) v[e] += add;
+            const uint32_t part = __reduce_add_sync(FULL_MASK, share);
+            if (lane == 0) s_part[warp] = part;
         }
         // after a timed-out wait the prefix is unknown: nothing is written any more
         if (__syncthreads_or(abort)) break;
+        if (DELTA) {
+#pragma unroll
+            for (int w = 0; w < UT / 32; ++w) add += s_part[w];
+#pragma unroll
+            for (int e = 0; e < UE; ++e) v[e] += add;
+        }
         {
             // stage at stride UE + 1 (conflict-free both ways) and write coalesced
 #pragma unroll
@@ -467,14 +467,21 @@ std::size_t bitpack_compress(device_context& ctx, const uint32_t* in, std::size_
     check_cuda(cudaStreamSynchronize(ctx.stream), "cudaStreamSynchronize");
     const std::size_t out_words = 3 * (std::size_t)chunks + packed;
     uint32_t* out = make_output(out_words);
+    // Parts of a chunk where the chunks are too few to keep the SMs' warps busy several
+    // times over (10^7 elements in chunks of 65,536: 474 -> 300 us for the call, 5,000 in
+    // chunks of 2,048 45 -> 38); a whole chunk else, whose header is read once (10^8
+    // elements in chunks of 2,048: 283 us, in rounds 294).
+    std::size_t span = chunk;
+    while (span > ROUND && n / span < (std::size_t(1) << 15)) span /= 2;
     {
         kernel_timer kt(ctx, "bitpack.pack");
+        const int grid = grid_for(ctx, (n + span - 1) / span, WARPS);
         if (delta)
             k_bp_pack<true><<<grid, THREADS, 0, ctx.stream>>>(in, (uint32_t)n, (uint32_t)chunk, chunks,
-                                                              hdr.as<uint32_t>(), offs.as<uint32_t>(), out);
+                                                              hdr.as<uint32_t>(), offs.as<uint32_t>(), out, (uint32_t)span);
         else
             k_bp_pack<false><<<grid, THREADS, 0, ctx.stream>>>(in, (uint32_t)n, (uint32_t)chunk, chunks,
-                                                               hdr.as<uint32_t>(), offs.as<uint32_t>(), out);
+                                                               hdr.as<uint32_t>(), offs.as<uint32_t>(), out, (uint32_t)span);
         check_cuda(cudaGetLastError(), "bitpack pack launch");
     }
     return out_words;
