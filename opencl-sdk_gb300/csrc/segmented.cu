@@ -21,8 +21,8 @@
 //     the MSD route: one pass on that digit, then one-CTA sorts of ranges of
 //     buckets. The others take a batched onesweep over every digit, whose
 //     decoupled look-back stops at the first tile of its segment.
-// The small/medium path and the large path are independent and run on two
-// streams that fork from and join back to the context's stream.
+// The small/medium path and the large path are independent; where both have much to
+// do they run on two streams that fork from and join back to the context's stream.
 #include <algorithm>
 #include <cstring>
 #include <map>
@@ -253,9 +253,9 @@ template <typename K> __device__ __forceinline__ void seg_guess(const SegArgs<K>
             uint32_t m = 0;
             for (int d = lane; d < RADIX; d += 32) m = max(m, count[d]);
             m = __reduce_max_sync(FULL_MASK, m);
-            // three deviations below the estimate
+            // three deviations below the estimate; and evenly filled bins
             const float least = ((float)m - 3.0f * sqrtf((float)m)) * (1.0f / (32 * ROWS)) * (float)len;
-            if (least > (float)a.sub_cap) top = -1;
+            if (least > (float)min(a.sub_cap, len / 2) || len / RADIX + SUB_WINDOW > a.sub_cap) top = -1;
             __syncwarp();
         }
         if (lane == 0) {
@@ -577,7 +577,10 @@ template <typename K, int TILE, int STEP> __global__ void __launch_bounds__(256)
 // that varies inside the segment (its bins are not all in one) and, when every
 // bin there leaves room for a window in sub_cap, the MSD route: one
 // pass on that digit partitions the segment into its bins (stable), and
-// ranges of neighbouring bins become sub-buckets for the warp and CTA sorts;
+// ranges of neighbouring bins become sub-buckets for the warp and CTA sorts.
+// A bin with more than half of the segment is as long a sort as all of it
+// (segments of 12,000 u64 keys that are the AND of four words: 894 us by that
+// route, 819 by the passes; 100 of 10,000: 395 and 261);
 // else the full LSD passes, over tiles appended to their own sequence.
 // COUNT_FIRST: a segment of which one digit was counted takes the MSD route
 // with it or is put off to COUNT_REST, with its counts cleared.
@@ -633,7 +636,8 @@ __device__ __forceinline__ void seg_route(const SegArgs<K>& a, bool with_msd, ui
 #pragma unroll
         for (int w = 0; w < 8; ++w) biggest = max(biggest, s_max[w]);
         // room for a window's keys and its last bucket
-        const bool msd = top >= 0 && (one < 0 || top == one) && biggest + SUB_WINDOW <= a.sub_cap;
+        const bool msd =
+            top >= 0 && (one < 0 || top == one) && biggest + SUB_WINDOW <= a.sub_cap && biggest <= len / 2;
         if (threadIdx.x == 0) a.route[j] = msd ? (uint8_t)top : (uint8_t)(one < 0 ? NO_ROUTE : REST);
         if (msd) {
             const uint32_t* row = a.seg_hist + ((size_t)j * P + top) * RADIX;
@@ -952,6 +956,14 @@ constexpr std::size_t FEW_KEYS = std::size_t(1) << 22;
 constexpr std::size_t VERY_FEW_KEYS = std::size_t(1) << 18;
 constexpr std::size_t ROUTE_32BIT_KEYS = std::size_t(1) << 26;
 constexpr std::size_t TWO_STEP_KEYS = std::size_t(1) << 24;
+// The large path runs beside the small one, on the second stream, where both have
+// much to do. Where most keys are in large segments (a mean of twice the one-CTA
+// capacity, or of ONE_STREAM_SHARE of it in small batches), the small path's CTAs
+// only keep the large path's from their SMs, and the other way round (us beside /
+// after each other: 100 segments of 10,000 u64 keys 198 / 130, u32 pairs 127 / 106;
+// of 100,000 u64 pairs 448 / 405, u32 keys 282 / 255). Others gain from running beside
+// (1,000 of 200 u64 keys 78 / 104, of 12,000 floats with values 381 / 421).
+constexpr float ONE_STREAM_SHARE = 0.7f;
 
 template <typename K, bool HAS_V> struct LargeShape;
 template <bool HV> struct LargeShape<uint32_t, HV> {
@@ -1104,9 +1116,11 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
         k_seg_classify<K, TILE><<<grid, 256, 0, ctx.stream>>>(a);
         check_cuda(cudaGetLastError(), "segmented sort classify launch");
     }
-    // Fork: the large-segment path runs on the auxiliary stream.
-    cudaStream_t aux = opt.sparse ? ctx.stream : ctx.aux_stream();
-    if (!opt.sparse) {
+    // Fork: the large-segment path runs on the auxiliary stream (ONE_STREAM_SHARE).
+    const float mean = (float)n / (float)nseg / (float)cta_cap;  // segment, in capacities
+    const bool fork = !opt.sparse && maybe_large && mean < (n <= FEW_KEYS ? ONE_STREAM_SHARE : 2.0f);
+    cudaStream_t aux = fork ? ctx.aux_stream() : ctx.stream;
+    if (fork) {
         check_cuda(cudaEventRecord(ctx.fork_event, ctx.stream), "cudaEventRecord");
         check_cuda(cudaStreamWaitEvent(aux, ctx.fork_event, 0), "cudaStreamWaitEvent");
     }
@@ -1176,7 +1190,7 @@ void run(device_context& ctx, const K* in_k, K* out_k, const uint32_t* in_v, uin
             launch_cta_sorts<K, HAS_V>(ctx, a, true, msd_cap, n, opt.cta_threads, aux);
         }
     }
-    if (!opt.sparse) {  // join
+    if (fork) {  // join
         check_cuda(cudaEventRecord(ctx.join_event, aux), "cudaEventRecord");
         check_cuda(cudaStreamWaitEvent(ctx.stream, ctx.join_event, 0), "cudaStreamWaitEvent");
     }
