@@ -255,7 +255,7 @@ template <typename K> __device__ __forceinline__ void seg_guess(const SegArgs<K>
             m = __reduce_max_sync(FULL_MASK, m);
             // three deviations below the estimate; and evenly filled bins
             const float least = ((float)m - 3.0f * sqrtf((float)m)) * (1.0f / (32 * ROWS)) * (float)len;
-            if (least > (float)min(a.sub_cap, len / 2) || len / RADIX + SUB_WINDOW > a.sub_cap) top = -1;
+            if (least > (float)min(a.sub_cap, sizeof(K) == 4 ? a.sub_cap : len / 2) || len / RADIX + SUB_WINDOW > a.sub_cap) top = -1;
             __syncwarp();
         }
         if (lane == 0) {
@@ -578,9 +578,11 @@ template <typename K, int TILE, int STEP> __global__ void __launch_bounds__(256)
 // bin there leaves room for a window in sub_cap, the MSD route: one
 // pass on that digit partitions the segment into its bins (stable), and
 // ranges of neighbouring bins become sub-buckets for the warp and CTA sorts.
-// A bin with more than half of the segment is as long a sort as all of it
-// (segments of 12,000 u64 keys that are the AND of four words: 894 us by that
-// route, 819 by the passes; 100 of 10,000: 395 and 261);
+// For 64-bit keys a bin with more than half of the segment is as long a sort as
+// all of it (segments of 12,000 u64 keys that are the AND of four words: 894 us by
+// that route, 819 by the passes; 100 of 10,000: 395 and 261). 32-bit keys take the
+// route all the same (the learned sort's oversized buckets, 2^28 floats: 6.23 ms for
+// 6.37);
 // else the full LSD passes, over tiles appended to their own sequence.
 // COUNT_FIRST: a segment of which one digit was counted takes the MSD route
 // with it or is put off to COUNT_REST, with its counts cleared.
@@ -637,7 +639,7 @@ __device__ __forceinline__ void seg_route(const SegArgs<K>& a, bool with_msd, ui
         for (int w = 0; w < 8; ++w) biggest = max(biggest, s_max[w]);
         // room for a window's keys and its last bucket
         const bool msd =
-            top >= 0 && (one < 0 || top == one) && biggest + SUB_WINDOW <= a.sub_cap && biggest <= len / 2;
+            top >= 0 && (one < 0 || top == one) && biggest + SUB_WINDOW <= a.sub_cap && (sizeof(K) == 4 || biggest <= len / 2);
         if (threadIdx.x == 0) a.route[j] = msd ? (uint8_t)top : (uint8_t)(one < 0 ? NO_ROUTE : REST);
         if (msd) {
             const uint32_t* row = a.seg_hist + ((size_t)j * P + top) * RADIX;
