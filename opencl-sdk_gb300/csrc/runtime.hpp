@@ -204,9 +204,9 @@ struct device_context {
     device_context& operator=(const device_context&) = delete;
 
     void activate() const;  // cudaSetDevice(device)
-    //! Reserves `count` consecutive look-back sequence numbers. Tags are 30
-    //! bits wide: before they would wrap, the ring is cleared (stream-ordered)
-    //! so that no stale word can carry a matching tag.
+    //! Reserves `count` consecutive look-back sequence numbers. The shortest
+    //! tags are 29 bits wide: before they would wrap, the ring is cleared
+    //! (stream-ordered) so that no stale word can carry a matching tag.
     uint64_t reserve_seq(uint64_t count);
     //! True while the context's stream is being captured into a CUDA graph.
     bool capturing() const;
